@@ -193,6 +193,23 @@ __device__ __noinline__ bool ring_intersects_segment(const GeomsView& G, uint32_
       ring_pip<kFast>(G, r, q.b, q.b32, aoe, esc).hit)
     return true;
   if (aoe) return ring_seg_hits<kFast>(G, r, q.a, q.b, q.a32, q.b32, esc) >= 2;
+  if (kFast) {
+    // The band index first: with no segment left open by the FP32 tier the
+    // visit order does not matter (proper crossings only count), and most
+    // queries meet no segment at all.
+    int cross = 0;
+    bool open = false;
+    any_segment_near<kFast>(
+        G, r, fmin0f(q.a32.x, q.b32.x), fmin0f(q.a32.y, q.b32.y), fmax0f(q.a32.x, q.b32.x),
+        fmax0f(q.a32.y, q.b32.y), [&](int i) {
+          const uint32_t v = G.ring_vtx[r] + (uint32_t)i;
+          const int c = seg_x32(q.a32, q.b32, G.xy32[v], G.xy32[v + 1]);
+          cross += c == 1;
+          open = c < 0;
+          return open;
+        });
+    if (!open) return cross >= 2;
+  }
   const uint32_t V = G.ring_vtx[r];
   const int ns = G.ring_nsegs[r];
   int count = 0;
@@ -284,6 +301,11 @@ __device__ __noinline__ bool ring_intersects_ring_aoe(const GeomsView& GA, uint3
     rr = rb;
     ro = ra;
   }
+  // no edge of the larger ring near the smaller one's box: inside, the first
+  // segment's end is in the ring (on no edge, so allow_on_edge is moot);
+  // outside, no end is in and no segment meets an edge
+  const int iso = ring_isolation<kFast>(*Gr, rr, *Go, ro, esc);
+  if (iso >= 0) return iso == 1;
   const int nso = Go->ring_nsegs[ro];
   for (int i = 0; i < nso; i++)
     if (ring_intersects_segment<kFast>(*Gr, rr, ring_segment(*Go, ro, i), false, esc)) return true;

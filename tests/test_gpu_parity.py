@@ -763,3 +763,38 @@ def test_dwithin_distance_column(capi, oracle_mod):
     assert pairs(b, p) == pairs(ob, op)
     with pytest.raises(capi.GpuSpatialError, match="distance column"):
         j1.probe(inp1.probe.slice(0, 100), "dwithin", distance=0.0)
+
+
+@pytest.mark.parametrize("pred", ["contains", "covers", "intersects", "touches"])
+def test_holed_zones_and_small_polygons(capi, oracle_mod, pred):
+    """Zones with a star hole (band-indexed rings) against small polygons inside
+    the hole, across its edges, beside it, and sharing vertices and edges with
+    it: the isolation exit and the indexed segment test of the hole."""
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(5)
+    build, probe = [], []
+    for z in range(6):
+        n = int(rng.integers(16, 80))
+        ang = np.sort(rng.uniform(0, 2 * np.pi, n))
+        rad = 100.0 * rng.uniform(0.6, 1.0, n)
+        c = np.array([z * 150.0, 0.0])
+        ring = np.round(c + np.stack([rad * np.cos(ang), rad * np.sin(ang)], 1), 1)
+        hole = np.round(c + (ring[::-1] - c) / 3.0, 1)
+        build.append(wkb.wkb_polygon([np.vstack([ring, ring[:1]]), np.vstack([hole, hole[:1]])]))
+        for _ in range(120):
+            m = int(rng.integers(3, 9))
+            a = np.linspace(0, 2 * np.pi, m, endpoint=False) + rng.uniform(0, 6)
+            r = rng.uniform(0.5, 12.0)
+            at = c + rng.normal(0, 30.0, 2)
+            p = np.round(at + r * np.stack([np.cos(a), np.sin(a)], 1), 1)
+            if rng.random() < 0.3:  # shares one or two vertices with the hole
+                i = int(rng.integers(0, n))
+                p[0] = hole[i]
+                if rng.random() < 0.5:
+                    p[1] = hole[(i + 1) % n]
+            probe.append(wkb.wkb_polygon([np.vstack([p, p[:1]])]))
+    bcol, pcol = wkb.column_from_values(build), wkb.column_from_values(probe)
+    j = capi.SpatialJoin()
+    j.build(bcol)
+    b, p = j.probe(pcol, pred)
+    assert pairs(b, p) == oracle_pairs(oracle_mod, bcol, pcol, pred)
