@@ -798,3 +798,42 @@ def test_holed_zones_and_small_polygons(capi, oracle_mod, pred):
     j.build(bcol)
     b, p = j.probe(pcol, pred)
     assert pairs(b, p) == oracle_pairs(oracle_mod, bcol, pcol, pred)
+
+
+@pytest.mark.parametrize("k", [1, 3, 8, 9, 16])
+@pytest.mark.parametrize("n_build,n_probe", [(1, 2), (9, 31), (300, 300), (300, 1025), (2000, 3001)])
+def test_knn_packet_and_queue(capi, oracle_mod, n_build, n_probe, k):
+    """At least as many probes as build points: warps of neighbouring probes
+    share a traversal.  Some probes are NaN or past the split range, some sit
+    on a heap of equal points (ties at rank k, the queued exact kernel) and
+    some far outside (warps whose probes lie apart)."""
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(n_build * 100 + n_probe + k)
+    bx, by = rng.normal(0, 10.0, n_build), rng.normal(0, 10.0, n_build)
+    heap = rng.random(n_build) < 0.3
+    bx[heap], by[heap] = 3.0, -2.0
+    px, py = rng.normal(0, 12.0, n_probe), rng.normal(0, 12.0, n_probe)
+    far = rng.random(n_probe) < 0.1
+    px[far] *= 1e4
+    on = rng.random(n_probe) < 0.1
+    px[on], py[on] = 3.0, -2.0
+    if n_probe > 31:
+        px[7] = np.nan
+        px[11], py[12] = 2e18, -3e18
+    kj = capi.KnnJoin(refine_form=1)
+    kj.build(bx, by)
+    idx, dist = kj.query(px, py, k)
+    nan = np.isnan(px)
+    assert (idx[nan] == 0xFFFFFFFF).all() and np.isinf(dist[nan]).all()
+    # 1e18 away every build point is at one rounded distance, which is what the
+    # oracle ranks by; those probes take the plain form's kernel
+    off = (np.abs(px) > 1e18) | (np.abs(py) > 1e18)
+    plain = capi.KnnJoin(refine_form=0)
+    plain.build(bx, by)
+    pi, pd = plain.query(px, py, k)
+    assert np.array_equal(idx[off], pi[off]) and np.array_equal(dist[off], pd[off])
+    ok = ~nan & ~off
+    oi, od = oracle_mod.knn(oracle_mod.Geoms(wkb.points_column(bx, by)),
+                            oracle_mod.Geoms(wkb.points_column(px[ok], py[ok])), k, nthreads=4)
+    assert np.array_equal(idx[ok], oi)
+    np.testing.assert_allclose(dist[ok], od, rtol=1e-12, atol=0)
