@@ -1,16 +1,24 @@
 // cellgrid.cu — per-ring cell grids for the FP32 refine.
 //
 // A ring with at least kGridMinSegs segments gets a G x G grid over its
-// outward f32 rect.  A cell is clean when no edge of the ring touches the
-// closed cell, proven on f32 values: the edge's RN32 bbox strictly separated
-// from the cell (a strict comparison of RN values proves the exact one), or
-// all four cell corners strictly on one side of the edge (decided orient32,
-// whose static bound covers the rounding of the edge's coordinates).  Edges
-// whose y-range misses the cell's are strictly separated in y and are not
-// listed in the bands the cell spans, so only those bands are scanned.
-// Every point of a clean cell has the same tg answer (the isolation-exit
-// argument in predicates.cuh); the cell stores it, evaluated at the cell
-// centre with the regular point-in-ring code.
+// outward f32 rect.  An edge touches a cell unless it provably does not, on
+// f32 values: its RN32 bbox strictly separated from the closed cell (a strict
+// comparison of RN values proves the exact one), or all four cell corners
+// strictly on one side of it (box_side32, whose static bound covers the
+// rounding of the edge's coordinates).  A cell that no edge touches is clean:
+// every point of it has the same tg answer (the isolation-exit argument in
+// predicates.cuh).  The other cells list the edges that touch them.  Each cell
+// stores the answer at its centre, from the regular point-in-ring code, and
+// each listed edge runs so that the centre is strictly left of it (a cell
+// with an edge whose side of the centre is not decided is not answered).
+//
+// Every edge visits the cells of its bbox (6 or 7 for the zones' rings of 145
+// vertices and 26 x 26 cells), twice: to count and to fill.  (When each cell
+// scanned the bands it spans instead, some 50 edges a cell, 50k zones took
+// 4.47 ms; counting takes 0.46 and filling 3.36, most of it the centres' point
+// tests.)  A point in a mixed cell reads the 2 or 3 edges of its cell where the
+// y-band scan reads some 10, and a box those of the cells it lies in where that
+// reads 20.
 #include "geoms.cuh"
 #include "predicates.cuh"
 #include "prims.cuh"
@@ -47,62 +55,146 @@ __device__ __forceinline__ bool grid_axis(double a, double b, int n, float& o, f
   return grid_edge(o, step, n) >= hi;
 }
 
-// One block per ring (grid-stride over rings), threads over the cells.
-__global__ void __launch_bounds__(256)
-    k_grid_fill(GeomsView G, const uint64_t* __restrict__ cell_off, uint2* __restrict__ meta,
-                float4* __restrict__ rect, uint8_t* __restrict__ status) {
-  __shared__ float4 s_rect;
-  __shared__ int s_ok;
+constexpr int kMaxCells = 1024;  // grid_dim <= 32
+constexpr int kCellThreads = 128;
+
+// The ring's grid (false: none).  meta: the grid's (first cell, G, 0, 0).
+__device__ __forceinline__ bool ring_grid(const GeomsView& G, uint32_t r, int& g, float4& q) {
+  g = (int)grid_dim(G.ring_nsegs[r]);
+  q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const Rect64 R = G.ring_rect[r];
+  return g > 0 && G.ring_bands != nullptr && G.band_param[r].y >= 0.0f &&
+         grid_axis(R.x, R.z, g, q.x, q.z) && grid_axis(R.y, R.w, g, q.y, q.w);
+}
+
+// Calls f(cell) for the cells that edge (a, b) touches.
+template <class F>
+__device__ __forceinline__ void edge_cells(float4 q, int g, float2 a, float2 b, F&& f) {
+  const float xmin = fmin0f(a.x, b.x), xmax = fmax0f(a.x, b.x);
+  const float ymin = fmin0f(a.y, b.y), ymax = fmax0f(a.y, b.y);
+  // closed cells that the bbox is not strictly separated from
+  auto lo = [g](float o, float step, float v) {
+    int i = (int)fminf(fmaxf(__fdividef(v - o, step), 0.0f), (float)(g - 1));
+    while (i < g - 1 && grid_edge(o, step, i + 1) < v) i++;
+    while (i > 0 && !(grid_edge(o, step, i) < v)) i--;
+    return i;
+  };
+  auto hi = [g](float o, float step, float v) {
+    int i = (int)fminf(fmaxf(__fdividef(v - o, step), 0.0f), (float)(g - 1));
+    while (i > 0 && v < grid_edge(o, step, i)) i--;
+    while (i < g - 1 && !(v < grid_edge(o, step, i + 1))) i++;
+    return i;
+  };
+  const int i0 = lo(q.x, q.z, xmin), i1 = hi(q.x, q.z, xmax);
+  const int j0 = lo(q.y, q.w, ymin), j1 = hi(q.y, q.w, ymax);
+  for (int j = j0; j <= j1; j++) {
+    const float y0 = grid_edge(q.y, q.w, j), y1 = grid_edge(q.y, q.w, j + 1);
+    for (int i = i0; i <= i1; i++) {
+      const float x0 = grid_edge(q.x, q.z, i), x1 = grid_edge(q.x, q.z, i + 1);
+      if (xmax < x0 || xmin > x1 || ymax < y0 || ymin > y1) continue;
+      if (box_side32(a, b, make_float4(x0, y0, x1, y1)) == 0) f(j * g + i);
+    }
+  }
+}
+
+// One block per ring (grid-stride over rings), threads over the edges:
+// cell[] receives each cell's edge count, entries[r] their sum.
+__global__ void __launch_bounds__(kCellThreads)
+    k_cell_count(GeomsView G, const uint64_t* __restrict__ cell_off, uint4* __restrict__ meta,
+                 float4* __restrict__ rect, uint32_t* __restrict__ cell,
+                 uint32_t* __restrict__ entries) {
+  __shared__ uint32_t cnt[kMaxCells];
+  __shared__ uint32_t total;
   for (uint32_t r = blockIdx.x; r < G.nrings; r += gridDim.x) {
-    const uint32_t g = grid_dim(G.ring_nsegs[r]);
+    int g;
+    float4 q;
+    const bool ok = ring_grid(G, r, g, q);
     if (threadIdx.x == 0) {
-      float ox = 0, oy = 0, sx = 0, sy = 0;
-      const Rect64 R = G.ring_rect[r];
-      const bool ok = g > 0 && G.ring_bands != nullptr && G.band_param[r].y >= 0.0f &&
-                      grid_axis(R.x, R.z, (int)g, ox, sx) && grid_axis(R.y, R.w, (int)g, oy, sy);
-      s_ok = ok ? 1 : 0;
-      s_rect = make_float4(ox, oy, sx, sy);
-      meta[r] = make_uint2((uint32_t)cell_off[r], ok ? g : 0u);
-      rect[r] = s_rect;
+      meta[r] = make_uint4((uint32_t)cell_off[r], ok ? (uint32_t)g : 0u, 0u, 0u);
+      rect[r] = q;
+      total = 0;
+    }
+    for (int c = threadIdx.x; c < g * g; c += blockDim.x) cnt[c] = 0;
+    __syncthreads();
+    uint32_t mine = 0;
+    if (ok) {
+      const uint32_t V = G.ring_vtx[r];
+      const int ns = G.ring_nsegs[r];
+      for (int e = threadIdx.x; e < ns; e += blockDim.x)
+        edge_cells(q, g, G.xy32[V + e], G.xy32[V + e + 1], [&](int c) {
+          atomicAdd(&cnt[c], 1u);
+          mine++;
+        });
+    }
+    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&total, mine);
+    __syncthreads();
+    for (int c = threadIdx.x; c < g * g; c += blockDim.x) cell[cell_off[r] + c] = cnt[c];
+    if (threadIdx.x == 0) entries[r] = total;
+    __syncthreads();
+  }
+}
+
+// The cells' words from their counts, and their edges: first = the ring's
+// first entry.
+__global__ void __launch_bounds__(kCellThreads)
+    k_cell_fill(GeomsView G, const uint64_t* __restrict__ first, uint4* __restrict__ meta,
+                const float4* __restrict__ rect, uint32_t* __restrict__ cell,
+                float4* __restrict__ seg, uint16_t* __restrict__ edge_id) {
+  __shared__ uint32_t start[kMaxCells], at[kMaxCells];
+  __shared__ uint8_t bad[kMaxCells];
+  __shared__ uint32_t warp_sum[kCellThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint32_t r = blockIdx.x; r < G.nrings; r += gridDim.x) {
+    const uint4 m = meta[r];
+    const int g = (int)m.y, cells = g * g;
+    if (g == 0) continue;
+    const float4 q = rect[r];
+    const uint64_t base = first[r];
+    uint32_t* word = cell + m.x;
+    // exclusive scan of the counts, each thread a run of cells
+    const int per = (cells + kCellThreads - 1) / kCellThreads;
+    const int c0 = min((int)threadIdx.x * per, cells), c1 = min(c0 + per, cells);
+    uint32_t sum = 0;
+    for (int c = c0; c < c1; c++) sum += word[c];
+    uint32_t inc = warp_inclusive_scan(sum);
+    if (lane == 31) warp_sum[warp] = inc;
+    __syncthreads();
+    uint32_t run = inc - sum;
+    for (int w = 0; w < warp; w++) run += warp_sum[w];
+    for (int c = c0; c < c1; c++) {
+      start[c] = at[c] = run;
+      bad[c] = 0;
+      run += word[c];
     }
     __syncthreads();
-    if (s_ok) {
-      const float4 q = s_rect;
-      const uint32_t B = G.ring_bands[r];
-      const int nb = (int)(G.ring_bands[r + 1] - B) - 1;
-      const float2 prm = G.band_param[r];
-      for (uint32_t c = threadIdx.x; c < g * g; c += blockDim.x) {
-        const int i = (int)(c % g), j = (int)(c / g);
-        const float x0 = grid_edge(q.x, q.z, i), x1 = grid_edge(q.x, q.z, i + 1);
-        const float y0 = grid_edge(q.y, q.w, j), y1 = grid_edge(q.y, q.w, j + 1);
-        const int b0 = band_of(y0, prm.x, prm.y, nb), b1 = band_of(y1, prm.x, prm.y, nb);
-        bool clean = true;
-        for (uint32_t k = G.band_off[B + b0]; k < G.band_off[B + b1 + 1] && clean; k++) {
-          const float4 sg = G.band_seg[k];
-          const float2 a = make_float2(sg.x, sg.y), b = make_float2(sg.z, sg.w);
-          if (fmax0f(a.x, b.x) < x0 || fmin0f(a.x, b.x) > x1 || fmax0f(a.y, b.y) < y0 ||
-              fmin0f(a.y, b.y) > y1)
-            continue;
-          const int s0 = orient32(a, b, make_float2(x0, y0));
-          if (s0 != 0 && orient32(a, b, make_float2(x1, y0)) == s0 &&
-              orient32(a, b, make_float2(x1, y1)) == s0 && orient32(a, b, make_float2(x0, y1)) == s0)
-            continue;
-          clean = false;
-        }
-        uint8_t st = 0;
-        if (clean) {
-          // the centre, an f32 point strictly inside the cell
-          const float cx = __fmul_rn(0.5f, __fadd_rn(x0, x1));
-          const float cy = __fmul_rn(0.5f, __fadd_rn(y0, y1));
-          uint32_t esc = 0;
-          const bool in = ring_pip_fast(G, r, make_double2((double)cx, (double)cy),
-                                        make_float2(cx, cy), true, esc)
-                              .hit;
-          st = in ? 1 : 2;
-        }
-        status[cell_off[r] + c] = st;
-      }
+    const uint32_t V = G.ring_vtx[r];
+    const int ns = G.ring_nsegs[r];
+    for (int e = threadIdx.x; e < ns; e += blockDim.x) {
+      const float2 a = G.xy32[V + e], b = G.xy32[V + e + 1];
+      edge_cells(q, g, a, b, [&](int c) {
+        const int o = orient32(a, b, grid_centre(q, c % g, c / g));
+        if (o == 0) bad[c] = 1;
+        const uint32_t k = atomicAdd(&at[c], 1u);
+        edge_id[base + k] = (uint16_t)e;
+        seg[base + k] = o < 0 ? make_float4(b.x, b.y, a.x, a.y) : make_float4(a.x, a.y, b.x, b.y);
+      });
     }
+    __syncthreads();
+    for (int c = threadIdx.x; c < cells; c += blockDim.x) {
+      const uint32_t n = at[c] - start[c];
+      uint32_t w = kCellUnknown;
+      if (!bad[c] && n <= 255u && start[c] < (1u << 21)) {
+        const float2 p = grid_centre(q, c % g, c / g);
+        uint32_t esc = 0;
+        const bool in =
+            ring_pip_fast(G, r, make_double2((double)p.x, (double)p.y), p, true, esc).hit;
+        w = (n ? (in ? kCellMixedIn : kCellMixedOut) : (in ? kCellIn : kCellOut)) | n << 3 |
+            start[c] << 11;
+      }
+      word[c] = w;
+    }
+    if (threadIdx.x == 0) meta[r].z = (uint32_t)base;
     __syncthreads();
   }
 }
@@ -113,7 +205,7 @@ void build_cell_grid(DeviceGeoms& g, DecodeScratch& sc, cudaStream_t s) {
   const uint32_t nr = g.nrings;
   g.has_grid = false;
   if (nr == 0 || !g.has_bands) return;
-  g.grid_meta.reserve(((size_t)nr + 1) * sizeof(uint2), s);
+  g.grid_meta.reserve(((size_t)nr + 1) * sizeof(uint4), s);
   g.grid_rect.reserve(((size_t)nr + 1) * sizeof(float4), s);
   sc.counts.reserve(((size_t)nr + 1) * 4, s);
   sc.scans.reserve(((size_t)nr + 1) * 8, s);
@@ -124,12 +216,25 @@ void build_cell_grid(DeviceGeoms& g, DecodeScratch& sc, cudaStream_t s) {
   SPJ_CUDA(cudaMemcpyAsync(&total, sc.scans.as<uint64_t>() + nr, 8, cudaMemcpyDeviceToHost, s));
   SPJ_CUDA(cudaStreamSynchronize(s));
   SPJ_CHECK(total < 0xFFFFFFFFull, "cell grid too large");
-  g.grid_status.reserve(total + 16, s);
+  g.grid_cell.reserve((total + 1) * 4, s);
   // the grid is built with the point-in-ring code of a view without a grid
-  GeomsView v = g.view();
-  k_grid_fill<<<grid_for(nr, 1, kNumSMs * 8), 256, 0, s>>>(
-      v, sc.scans.as<uint64_t>(), g.grid_meta.as<uint2>(), g.grid_rect.as<float4>(),
-      g.grid_status.as<uint8_t>());
+  const GeomsView v = g.view();
+  const int blocks = grid_for(nr, 1, kNumSMs * 16);
+  k_cell_count<<<blocks, kCellThreads, 0, s>>>(v, sc.scans.as<uint64_t>(), g.grid_meta.as<uint4>(),
+                                               g.grid_rect.as<float4>(),
+                                               g.grid_cell.as<uint32_t>(),
+                                               sc.counts.as<uint32_t>());
+  scan_u32_u64(sc.counts.as<uint32_t>(), sc.scans.as<uint64_t>(), nr, sc.tmp, s);
+  SPJ_CUDA(cudaMemcpyAsync(&total, sc.scans.as<uint64_t>() + nr, 8, cudaMemcpyDeviceToHost, s));
+  SPJ_CUDA(cudaStreamSynchronize(s));
+  if (total >= 0xFFFFFFFFull) return;  // (more entries than 32 bits count: no grid)
+  g.grid_seg.reserve((total + 1) * sizeof(float4), s);
+  g.grid_edge_id.reserve((total + 1) * sizeof(uint16_t), s);
+  k_cell_fill<<<blocks, kCellThreads, 0, s>>>(v, sc.scans.as<uint64_t>(), g.grid_meta.as<uint4>(),
+                                              g.grid_rect.as<float4>(),
+                                              g.grid_cell.as<uint32_t>(),
+                                              g.grid_seg.as<float4>(),
+                                              g.grid_edge_id.as<uint16_t>());
   SPJ_CUDA(cudaGetLastError());
   SPJ_CUDA(cudaStreamSynchronize(s));
   g.has_grid = true;

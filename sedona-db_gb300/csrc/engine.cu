@@ -35,6 +35,7 @@ Workspace::~Workspace() {
   arena.release();
   rqueue.release();
   status.release();
+  packet.release();
   wkb_data.release();
   wkb_offsets.release();
   wkb_validity.release();
@@ -92,6 +93,71 @@ static inline float ev_ms(cudaEvent_t a, cudaEvent_t b) {
   float ms = 0;
   cudaEventElapsedTime(&ms, a, b);
   return ms;
+}
+
+// Relation predicates over a build side with rings, in the FP32 form and with
+// the automatic candidate order and refine: the packet kernels, where they
+// take the probe rows (which have to be in Morton order).
+bool JoinEngine::packet_path(int predicate, bool points) const {
+  const EngineConfig auto_cfg;
+  return predicate != kPredDWithin && cfg_.refine_form == kFastF32 && !bg_.all_points &&
+         bg_.nrings > 0 && bvh_.nprims > 0 && cfg_.candidate_order == auto_cfg.candidate_order &&
+         cfg_.order_tiles == auto_cfg.order_tiles && cfg_.refine_split == auto_cfg.refine_split &&
+         cfg_.refine_min_blocks == auto_cfg.refine_min_blocks && !cfg_.grid_rings &&
+         packet_takes(predicate, points);
+}
+
+uint64_t JoinEngine::packet_probe(Workspace& ws, int predicate, uint32_t probe_base,
+                                  const uint32_t* order, DeviceStatus& hst, uint64_t& launches) {
+  struct Readback {
+    DeviceStatus st;
+    uint64_t total, ctrl[4];
+    unsigned fault[2];
+  };
+  cudaStream_t s = ws.stream;
+  const uint32_t n = ws.probe.n;
+  const bool points = ws.probe.all_points;
+  const LbvhView tv = bvh_.view();
+  const GeomsView bv = bg_.view(), pv = ws.probe.view();
+  ws.host.reserve(sizeof(Readback));
+  Readback* rb = ws.host.as<Readback>();
+  ws.psc.counts.reserve(((size_t)n + 1) * 4, s);
+  ws.psc.offsets.reserve(((size_t)n + 1) * 8, s);
+  // first guesses (2M buildings x 50k zones: 2.4 records and 6 open pairs per
+  // probe row); a column that needs more tells how much and runs again
+  uint64_t chunks = n / 8 + 1024, queued = points ? 0 : (uint64_t)n * 8 + 1024;
+  for (int attempt = 0;; attempt++) {
+    ws.packet.reserve(n, chunks, queued, s);
+    const PacketStore a = ws.packet.store(n);
+    reset_status(ws.status, s);
+    packet_join(tv, bv, pv, points, order, predicate, ws.psc.counts.as<uint32_t>(), a,
+                ws.status.as<DeviceStatus>(), s);
+    scan_u32_u64(ws.psc.counts.as<uint32_t>(), ws.psc.offsets.as<uint64_t>(), n, ws.psc.tmp, s);
+    SPJ_CUDA(cudaMemcpyAsync(&rb->st, ws.status.get(), sizeof rb->st, cudaMemcpyDeviceToHost, s));
+    SPJ_CUDA(cudaMemcpyAsync(&rb->total, ws.psc.offsets.as<uint64_t>() + n, 8,
+                             cudaMemcpyDeviceToHost, s));
+    SPJ_CUDA(cudaMemcpyAsync(rb->ctrl, a.ctrl, sizeof rb->ctrl, cudaMemcpyDeviceToHost, s));
+    SPJ_CUDA(cudaMemcpyAsync(rb->fault, tv.fault, 8, cudaMemcpyDeviceToHost, s));
+    SPJ_CUDA(cudaStreamSynchronize(s));
+    launches += points ? 5 : 6;
+    check_traversal_word(rb->fault);
+    if (rb->ctrl[0] <= a.chunks && rb->ctrl[1] <= a.queue_cap) break;
+    SPJ_CHECK(attempt < 2, "packet refine: record capacities did not settle");
+    chunks = rb->ctrl[0] + rb->ctrl[0] / 8;
+    queued = rb->ctrl[1] + rb->ctrl[1] / 8;
+  }
+  hst = rb->st;
+  const uint64_t total = rb->total;
+  SPJ_CHECK(hst.counters[1] < (1ull << 34), "candidate pair count too large");
+  if (hst.first_bad != ~0ull)
+    throw Error(std::string("refine: ") + status_message((uint32_t)(hst.first_bad >> 40)));
+  if (cfg_.profile) SPJ_CUDA(cudaEventRecord(ws.ev[3], s));
+  ws.out_build.reserve((total + 1) * 4, s);
+  ws.out_probe.reserve((total + 1) * 4, s);
+  packet_scatter(pv, order, ws.psc.offsets.as<uint64_t>(), probe_base, ws.packet.store(n),
+                 ws.out_build.as<uint32_t>(), ws.out_probe.as<uint32_t>(), total, s);
+  launches++;
+  return total;
 }
 
 uint64_t JoinEngine::probe(Workspace& ws, const WkbDeviceColumn& col, int predicate,
@@ -181,6 +247,34 @@ uint64_t JoinEngine::probe(Workspace& ws, const WkbDeviceColumn& col, int predic
       SPJ_CUDA(cudaEventRecord(ws.ev[3], s));
       SPJ_CUDA(cudaEventRecord(ws.ev[4], s));
     }
+    SPJ_CUDA(cudaStreamSynchronize(s));
+    {
+      std::lock_guard<std::mutex> lk(stats_mu_);
+      stats_.calls++;
+      stats_.probe_rows += n;
+      stats_.candidates += hst.counters[1];
+      stats_.results += total;
+      stats_.escalations += hst.counters[0];
+      stats_.pairs_evaluated += hst.counters[1];
+      stats_.kernel_launches += launches;
+      stats_.probe_bytes +=
+          (uint64_t)col.data_len + (uint64_t)(col.n + 1) * (col.offsets64 ? 8 : 4);
+      if (prof) {
+        stats_.ms_decode += ev_ms(ws.ev[0], ws.ev[1]);
+        stats_.ms_filter += ev_ms(ws.ev[1], ws.ev[2]);
+        stats_.ms_refine += ev_ms(ws.ev[2], ws.ev[3]);
+        stats_.ms_compact += ev_ms(ws.ev[3], ws.ev[4]);
+      }
+    }
+    *d_build = ws.out_build.as<uint32_t>();
+    *d_probe = ws.out_probe.as<uint32_t>();
+    return total;
+  }
+  if (order && packet_path(predicate, ws.probe.all_points)) {
+    if (prof) SPJ_CUDA(cudaEventRecord(ws.ev[2], s));
+    DeviceStatus hst;
+    const uint64_t total = packet_probe(ws, predicate, probe_base, order, hst, launches);
+    if (prof) SPJ_CUDA(cudaEventRecord(ws.ev[4], s));
     SPJ_CUDA(cudaStreamSynchronize(s));
     {
       std::lock_guard<std::mutex> lk(stats_mu_);

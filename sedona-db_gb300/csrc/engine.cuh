@@ -13,6 +13,7 @@
 #include "geoms.cuh"
 #include "dwithin.cuh"
 #include "lbvh.cuh"
+#include "packet.cuh"
 #include "refine.cuh"
 
 namespace spj {
@@ -125,6 +126,8 @@ struct Workspace {
   DevBuf arena;   // fused ST_DWithin overflow arena: cursor, heads, chunks
   DevBuf rqueue;  // pairs left open by the refine's cheap pass, then its count
   DevBuf wkb_data, wkb_offsets, wkb_validity;  // H2D staging of host columns
+  PacketBufs packet;  // records and open pairs of the packet refine
+  PinnedBuf host;     // counts and status read back by a probe
   cudaEvent_t ev[6] = {};
   bool last_probe_points = true;
   Workspace();
@@ -169,6 +172,9 @@ class JoinEngine {
 
  private:
   void split_points();
+  bool packet_path(int predicate, bool points) const;
+  uint64_t packet_probe(Workspace& ws, int predicate, uint32_t probe_base, const uint32_t* order,
+                        DeviceStatus& hst, uint64_t& launches);
   int device_;
   EngineConfig cfg_;
   DeviceGeoms bg_;

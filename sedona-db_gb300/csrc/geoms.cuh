@@ -39,6 +39,18 @@ namespace spj {
 
 enum GeomKind : uint8_t { kEmpty = 0, kPoint = 1, kPolygon = 3, kMultiPolygon = 6 };
 
+// A grid cell's word: its state, the number of its edges and the first of
+// them among its ring's entries.
+constexpr uint32_t kCellUnknown = 0;  // not answered by the grid
+constexpr uint32_t kCellIn = 1;       // clean, inside
+constexpr uint32_t kCellOut = 2;      // clean, outside
+constexpr uint32_t kCellMixedIn = 5;  // edges touch it; its centre is inside ...
+constexpr uint32_t kCellMixedOut = 6;  // ... outside
+constexpr uint32_t kCellMixed = 4;
+__host__ __device__ inline uint32_t cell_state(uint32_t w) { return w & 7u; }
+__host__ __device__ inline uint32_t cell_count(uint32_t w) { return (w >> 3) & 255u; }
+__host__ __device__ inline uint32_t cell_first(uint32_t w) { return w >> 11; }
+
 struct GeomsView {
   uint32_t n = 0;
   uint32_t nparts = 0, nrings = 0, nverts = 0;
@@ -63,13 +75,16 @@ struct GeomsView {
   // one 16-byte word per entry instead of an index and then two vertices
   const float4* band_seg = nullptr;
   const float2* band_param = nullptr;    // per ring: (y origin, bands per unit y)
-  // cell grid (nullptr when not built): per ring (status offset, G; G = 0 for
-  // no grid), (x0, y0, w, h) with cell (i, j) = [x0 + i w, x0 + (i+1) w] x
-  // [y0 + j h, y0 + (j+1) h] in f32 arithmetic, and one status byte per cell
-  // (0 mixed, 1 inside, 2 outside)
-  const uint2* grid_meta = nullptr;
+  // cell grid (nullptr when not built): per ring (first cell, G, first edge
+  // entry, 0; G = 0 for no grid), (x0, y0, w, h) with cell (i, j) = [x0 + i w,
+  // x0 + (i+1) w] x [y0 + j h, y0 + (j+1) h] in f32 arithmetic, one word per cell
+  // (kCell*) and the f32 segments of the edges that touch each cell, directed
+  // so that the cell's centre lies strictly on their left
+  const uint4* grid_meta = nullptr;
   const float4* grid_rect = nullptr;
-  const uint8_t* grid_status = nullptr;
+  const uint32_t* grid_cell = nullptr;
+  const float4* grid_seg = nullptr;
+  const uint16_t* grid_edge_id = nullptr;  // each entry's edge index within the ring
   // ring-ring and ring-in-ring tests may answer from the cells that hold the
   // other ring's box (when they are all clean and alike)
   bool grid_rings = false;
@@ -86,7 +101,7 @@ struct DeviceGeoms {
   bool has_row_flags = false, has_ring_flags = false;
   DevBuf ring_bands, band_off, band_edges, band_seg, band_param;
   bool has_bands = false;
-  DevBuf grid_meta, grid_rect, grid_status;
+  DevBuf grid_meta, grid_rect, grid_cell, grid_seg, grid_edge_id;
   bool has_grid = false;
   bool grid_rings = false;
 
@@ -117,9 +132,11 @@ struct DeviceGeoms {
       v.band_param = band_param.as<float2>();
     }
     if (has_grid) {
-      v.grid_meta = grid_meta.as<uint2>();
+      v.grid_meta = grid_meta.as<uint4>();
       v.grid_rect = grid_rect.as<float4>();
-      v.grid_status = grid_status.as<uint8_t>();
+      v.grid_cell = grid_cell.as<uint32_t>();
+      v.grid_seg = grid_seg.as<float4>();
+      v.grid_edge_id = grid_edge_id.as<uint16_t>();
       v.grid_rings = grid_rings;
     }
     return v;
@@ -130,7 +147,8 @@ struct DeviceGeoms {
            xy.size() + xy32.size() + row_flags.size() + ring_flags.size() +
            ring_bands.size() + band_off.size() + band_edges.size() + band_seg.size() +
            band_param.size() +
-           grid_meta.size() + grid_rect.size() + grid_status.size();
+           grid_meta.size() + grid_rect.size() + grid_cell.size() + grid_seg.size() +
+           grid_edge_id.size();
   }
 };
 

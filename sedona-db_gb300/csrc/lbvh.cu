@@ -4,6 +4,8 @@
 #include "prims.cuh"
 
 #include <algorithm>
+#include <cmath>
+#include <cstring>
 
 namespace spj {
 namespace {
@@ -46,9 +48,12 @@ __global__ void k_compact_ids(const uint8_t* __restrict__ flag, const uint64_t* 
     if (flag[i]) ids[pos[i]] = (uint32_t)i;
 }
 
+// ext[0..3]: extent of the box centres (order-preserving integers); sums[0..1]:
+// total box width and height
 __global__ void k_bounds(const float4* __restrict__ boxes, const uint32_t* __restrict__ ids,
-                         uint32_t m, uint32_t* __restrict__ ext) {
+                         uint32_t m, uint32_t* __restrict__ ext, float* __restrict__ sums) {
   float mnx = INFINITY, mny = INFINITY, mxx = -INFINITY, mxy = -INFINITY;
+  float w = 0.0f, h = 0.0f;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m;
        i += (int64_t)gridDim.x * blockDim.x) {
     float4 b = boxes[ids[i]];
@@ -57,18 +62,24 @@ __global__ void k_bounds(const float4* __restrict__ boxes, const uint32_t* __res
     mny = fminf(mny, cy);
     mxx = fmaxf(mxx, cx);
     mxy = fmaxf(mxy, cy);
+    w += b.z - b.x;
+    h += b.w - b.y;
   }
   for (int o = 16; o > 0; o >>= 1) {
     mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
     mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
     mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
     mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
+    w += __shfl_xor_sync(0xffffffffu, w, o);
+    h += __shfl_xor_sync(0xffffffffu, h, o);
   }
   if ((threadIdx.x & 31) == 0) {
     atomicMin(&ext[0], f2o(mnx));
     atomicMin(&ext[1], f2o(mny));
     atomicMax(&ext[2], f2o(mxx));
     atomicMax(&ext[3], f2o(mxy));
+    if (w != 0.0f) atomicAdd(&sums[0], w);
+    if (h != 0.0f) atomicAdd(&sums[1], h);
   }
 }
 
@@ -649,14 +660,15 @@ void build_lbvh(const float4* boxes, uint32_t n, uint32_t leaf_size, Lbvh& out, 
   out.leaf_box.reserve((size_t)(L > 0 ? L : 1) * sizeof(float4), s);
   out.fault.reserve(8, s);
   SPJ_CUDA(cudaMemsetAsync(out.fault.get(), 0, 8, s));
+  out.mean_w = out.mean_h = out.extent_area = 0.0f;
   if (m == 0) return;
   uint32_t* ids = out.sorted_id.as<uint32_t>();
   k_compact_ids<<<g, 256, 0, s>>>(flag.as<uint8_t>(), pos.as<uint64_t>(), n, ids);
-  DevBuf ext(16, s);
-  uint32_t init[4] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u};
-  SPJ_CUDA(cudaMemcpyAsync(ext.get(), init, 16, cudaMemcpyHostToDevice, s));
+  DevBuf ext(24, s);
+  uint32_t init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u};
+  SPJ_CUDA(cudaMemcpyAsync(ext.get(), init, 24, cudaMemcpyHostToDevice, s));
   const int gm = grid_for(m, 256);
-  k_bounds<<<gm, 256, 0, s>>>(boxes, ids, m, ext.as<uint32_t>());
+  k_bounds<<<gm, 256, 0, s>>>(boxes, ids, m, ext.as<uint32_t>(), ext.as<float>() + 4);
   DevBuf keys((size_t)m * 4, s), akeys((size_t)m * 4, s), avals((size_t)m * 4, s);
   k_morton<<<gm, 256, 0, s>>>(boxes, ids, m, ext.as<uint32_t>(), keys.as<uint32_t>());
   radix_sort_pairs(keys.as<uint32_t>(), ids, akeys.as<uint32_t>(), avals.as<uint32_t>(), m, 32,
@@ -675,7 +687,16 @@ void build_lbvh(const float4* boxes, uint32_t n, uint32_t leaf_size, Lbvh& out, 
                                              out.node_box.as<float4>(), visits.as<unsigned>());
   }
   SPJ_CUDA(cudaGetLastError());
+  uint32_t e[6];
+  SPJ_CUDA(cudaMemcpyAsync(e, ext.get(), 24, cudaMemcpyDeviceToHost, s));
   SPJ_CUDA(cudaStreamSynchronize(s));
+  float sums[2];
+  memcpy(sums, e + 4, 8);
+  const float area = (o2f(e[2]) - o2f(e[0])) * (o2f(e[3]) - o2f(e[1]));
+  const bool ok = std::isfinite(sums[0]) && std::isfinite(sums[1]) && std::isfinite(area);
+  out.mean_w = ok ? sums[0] / (float)m : 0.0f;
+  out.mean_h = ok ? sums[1] / (float)m : 0.0f;
+  out.extent_area = ok ? area : 0.0f;
 }
 
 void check_traversal(const LbvhView& t, cudaStream_t s) {
@@ -683,6 +704,10 @@ void check_traversal(const LbvhView& t, cudaStream_t s) {
   unsigned f[2] = {0, 0};
   SPJ_CUDA(cudaMemcpyAsync(f, t.fault, 8, cudaMemcpyDeviceToHost, s));
   SPJ_CUDA(cudaStreamSynchronize(s));
+  check_traversal_word(f);
+}
+
+void check_traversal_word(const unsigned* f) {
   static const char* what[] = {"", "an out-of-range leaf index", "an out-of-range node index",
                                "an out-of-range probe row", "more steps than the tree has nodes",
                                "a path deeper than its stack"};

@@ -29,10 +29,14 @@ struct LbvhView {
   const float4* leaf_box = nullptr;  // [L] union of each leaf's primitive boxes
   // [code, value]: the first out-of-range index a traversal met (code 0 = none)
   unsigned* fault = nullptr;
+  // mean primitive box and the area of the boxes' centres' extent (estimates
+  // of how many primitives a box meets; 0 when not finite)
+  float mean_w = 0.0f, mean_h = 0.0f, extent_area = 0.0f;
 };
 
 struct Lbvh {
   uint32_t nprims = 0, nleaves = 0, leaf_size = 4;
+  float mean_w = 0.0f, mean_h = 0.0f, extent_area = 0.0f;
   DevBuf sorted_box, sorted_id, node_box, node_child, leaf_box, fault;
   LbvhView view() const {
     LbvhView v;
@@ -45,6 +49,9 @@ struct Lbvh {
     v.node_child = node_child.as<int2>();
     v.leaf_box = leaf_box.as<float4>();
     v.fault = fault.as<unsigned>();
+    v.mean_w = mean_w;
+    v.mean_h = mean_h;
+    v.extent_area = extent_area;
     return v;
   }
   size_t device_bytes() const {
@@ -133,6 +140,8 @@ struct ProbeScratch {
 };
 // Throws if a traversal over t recorded an out-of-range index (syncs s).
 void check_traversal(const LbvhView& t, cudaStream_t s);
+// The same for a copy of the tree's fault word.
+void check_traversal_word(const unsigned* fault);
 // returns the number of candidate pairs (syncs the stream once)
 uint64_t probe_count(const LbvhView& t, const float4* probe_box, uint32_t nprobe,
                      ProbeScratch& sc, cudaStream_t s, const uint32_t* order = nullptr);

@@ -1,0 +1,55 @@
+// packet.cuh — filter and refine of relation predicates in one traversal per
+// warp (a packet) of 32 probe rows that are neighbours in Morton order.
+#pragma once
+#include "geoms.cuh"
+#include "lbvh.cuh"
+#include "refine.cuh"
+
+namespace spj {
+
+// The hits of a packet: one record per build row that some of its 32 probes
+// may meet (build row, lane mask of the probes that do), in traversal order,
+// kept in chunks of 32 records linked per packet.  Pairs that the packet
+// leaves open wait in a queue, with the place of their bit.
+struct PacketStore {
+  uint2* rec = nullptr;        // chunks * 32 records
+  uint32_t* next = nullptr;    // chunks: the packet's next chunk
+  uint32_t chunks = 0;
+  uint2* packets = nullptr;    // per packet: first place in the probe order, rows
+  uint32_t* head = nullptr;    // per packet: first chunk
+  uint32_t* nrec = nullptr;    // per packet: records
+  uint4* queue = nullptr;      // (build row, probe row, record, lane | flags)
+  uint32_t queue_cap = 0;
+  // [0] chunks taken, [1] pairs queued, [2] packets started, [3] packets; past
+  // a capacity the counts go on (the caller makes room and runs again)
+  unsigned long long* ctrl = nullptr;
+};
+constexpr size_t kPacketCtrlBytes = 4 * sizeof(unsigned long long);
+
+struct PacketBufs {
+  DevBuf rec, next, heads, queue, ctrl;
+  uint64_t chunk_cap = 0, queue_cap = 0;
+  // reserves room for n probe rows and at least the given chunks / pairs
+  void reserve(uint32_t n, uint64_t chunks, uint64_t queued, cudaStream_t s);
+  PacketStore store(uint32_t n) const;
+  void release();
+};
+
+// Whether the packet kernels answer this predicate for probe rows that are
+// all points (else any rows): the others take the candidate pairs' path.
+bool packet_takes(int predicate, bool points);
+
+// counts[row] = pairs of each probe row and the packets' records in `a`;
+// order: the probe rows in Morton order (n entries).  st: counters[0] += FP64
+// escalations, [1] += candidate pairs (overlapping boxes).
+void packet_join(const LbvhView& t, const GeomsView& build, const GeomsView& probe, bool points,
+                 const uint32_t* order, int predicate, uint32_t* counts, const PacketStore& a,
+                 DeviceStatus* st, cudaStream_t s);
+
+// The pairs, grouped by probe row in ascending order (offs: exclusive scan of
+// counts), writes bounded by cap.
+void packet_scatter(const GeomsView& probe, const uint32_t* order, const uint64_t* offs,
+                    uint32_t probe_base, const PacketStore& a, uint32_t* out_build,
+                    uint32_t* out_probe, uint64_t cap, cudaStream_t s);
+
+}  // namespace spj

@@ -167,40 +167,93 @@ __device__ __forceinline__ void pip_seg_f64(double2 a, double2 b, double2 p, int
   }
 }
 
+// Bound E on the error of an orientation t1 - t2, t1 = dx ey, t2 = dy ex,
+// evaluated in f32 on RN32 copies of FP64 points, from bounds of its parts:
+// the rounded differences |dx|, |dy|, |ex|, |ey|, the sums of the magnitudes
+// of the coordinates they were formed of, and the products.  Per coordinate
+// |c - RN32(c)| <= 2^-24 (1 + 2^-20) |RN32(c)| (kRound) plus 2^-150 in the subnormal
+// range; then the rounding of the two differences, the two products and the
+// final difference.  The result is E (1 + 2^-4) with slack, so that a value
+// beyond it leaves |exact| >= E / 16, some 2^24 times the FP64 rounding of
+// tg's own orientation / slope / intersection arithmetic on the same points:
+// tg's FP64 decisions follow the exact sign.  (With twice the coordinate
+// rounding and 2 E, as this bound once was, four times as many vertices near
+// an edge went undecided.)
+constexpr float kUlp = 5.9604645e-08f;    // 2^-24
+constexpr float kRound = 5.9604702e-08f;  // 2^-24 (1 + 2^-20), rounded up
+constexpr float kTiny = 1.4012985e-45f;
+__device__ __forceinline__ float orient_bound(float dx, float dy, float ex, float ey, float sdx,
+                                              float sdy, float sex, float sey, float t1, float t2,
+                                              float o) {
+  const float Edx = __fadd_ru(__fmul_ru(kRound, sdx), __fadd_ru(__fmul_ru(kUlp, dx), kTiny));
+  const float Edy = __fadd_ru(__fmul_ru(kRound, sdy), __fadd_ru(__fmul_ru(kUlp, dy), kTiny));
+  const float Eex = __fadd_ru(__fmul_ru(kRound, sex), __fadd_ru(__fmul_ru(kUlp, ex), kTiny));
+  const float Eey = __fadd_ru(__fmul_ru(kRound, sey), __fadd_ru(__fmul_ru(kUlp, ey), kTiny));
+  const float E1 = __fadd_ru(__fadd_ru(__fmul_ru(dx, Eey), __fmul_ru(ey, Edx)),
+                             __fadd_ru(__fmul_ru(Edx, Eey), __fmul_ru(kUlp, t1)));
+  const float E2 = __fadd_ru(__fadd_ru(__fmul_ru(dy, Eex), __fmul_ru(ex, Edy)),
+                             __fadd_ru(__fmul_ru(Edy, Eex), __fmul_ru(kUlp, t2)));
+  return __fmul_ru(__fadd_ru(__fadd_ru(E1, E2), __fadd_ru(__fmul_ru(kUlp, o), kTiny)), 1.0625010f);
+}
+
 // Sign of the exact orientation (b - a) x (p - a) of three FP64 points known
 // through their round-to-nearest f32 copies a, b, p: +1 / -1 when the f32
-// evaluation clears twice a static bound E on its error, else 0.
-// E covers the coordinate rounding (|c - RN32(c)| <= 2^-24 |RN32(c)|, doubled,
-// plus 2^-150 absolute for the subnormal range), the rounding of the two
-// differences, the two products and the final difference.  A decided sign
-// therefore leaves |exact| >= E, some 2^28 times the FP64 rounding of tg's
-// own orientation / slope / intersection arithmetic on the same points, so
-// tg's FP64 decisions follow the exact sign.
+// evaluation clears its error bound, else 0 (also for NaN / inf).
 __device__ __forceinline__ int orient32(float2 a, float2 b, float2 p) {
   const float dx = __fsub_rn(b.x, a.x), dy = __fsub_rn(b.y, a.y);
   const float ex = __fsub_rn(p.x, a.x), ey = __fsub_rn(p.y, a.y);
   const float t1 = __fmul_rn(dx, ey), t2 = __fmul_rn(dy, ex);
   const float o = __fsub_rn(t1, t2);
-  const float u = 5.9604645e-08f;   // 2^-24
-  const float c2 = 1.1920929e-07f;  // 2^-23
-  const float tiny = 1.4012985e-45f;
-  const float Edx = __fadd_ru(__fmul_ru(c2, __fadd_ru(fabsf(b.x), fabsf(a.x))),
-                              __fadd_ru(__fmul_ru(u, fabsf(dx)), tiny));
-  const float Edy = __fadd_ru(__fmul_ru(c2, __fadd_ru(fabsf(b.y), fabsf(a.y))),
-                              __fadd_ru(__fmul_ru(u, fabsf(dy)), tiny));
-  const float Eex = __fadd_ru(__fmul_ru(c2, __fadd_ru(fabsf(p.x), fabsf(a.x))),
-                              __fadd_ru(__fmul_ru(u, fabsf(ex)), tiny));
-  const float Eey = __fadd_ru(__fmul_ru(c2, __fadd_ru(fabsf(p.y), fabsf(a.y))),
-                              __fadd_ru(__fmul_ru(u, fabsf(ey)), tiny));
-  const float E1 = __fadd_ru(__fadd_ru(__fmul_ru(fabsf(dx), Eey), __fmul_ru(fabsf(ey), Edx)),
-                             __fadd_ru(__fmul_ru(Edx, Eey), __fmul_ru(u, fabsf(t1))));
-  const float E2 = __fadd_ru(__fadd_ru(__fmul_ru(fabsf(dy), Eex), __fmul_ru(fabsf(ex), Edy)),
-                             __fadd_ru(__fmul_ru(Edy, Eex), __fmul_ru(u, fabsf(t2))));
-  const float E = __fmul_ru(__fadd_ru(__fadd_ru(E1, E2), __fadd_ru(__fmul_ru(u, fabsf(o)), tiny)),
-                            2.0000019f);  // x2 margin, x(1 + 2^-20) slack
+  const float E = orient_bound(
+      fabsf(dx), fabsf(dy), fabsf(ex), fabsf(ey), __fadd_ru(fabsf(b.x), fabsf(a.x)),
+      __fadd_ru(fabsf(b.y), fabsf(a.y)), __fadd_ru(fabsf(p.x), fabsf(a.x)),
+      __fadd_ru(fabsf(p.y), fabsf(a.y)), fabsf(t1), fabsf(t2), fabsf(o));
   if (o > E) return 1;
   if (o < -E) return -1;
-  return 0;  // undecided (also for NaN / inf)
+  return 0;
+}
+
+// orient32's bound for every point of a box q (x0, y0, x1, y1).
+__device__ __forceinline__ float box_orient_bound(float2 a, float2 b, float4 q) {
+  const float dx = fabsf(__fsub_rn(b.x, a.x)), dy = fabsf(__fsub_rn(b.y, a.y));
+  const float ex = fmaxf(fabsf(__fsub_rn(q.x, a.x)), fabsf(__fsub_rn(q.z, a.x)));
+  const float ey = fmaxf(fabsf(__fsub_rn(q.y, a.y)), fabsf(__fsub_rn(q.w, a.y)));
+  const float px = fmaxf(fabsf(q.x), fabsf(q.z)), py = fmaxf(fabsf(q.y), fabsf(q.w));
+  const float t1 = __fmul_ru(dx, ey), t2 = __fmul_ru(dy, ex);
+  return orient_bound(dx, dy, ex, ey, __fadd_ru(fabsf(b.x), fabsf(a.x)),
+                      __fadd_ru(fabsf(b.y), fabsf(a.y)), __fadd_ru(px, fabsf(a.x)),
+                      __fadd_ru(py, fabsf(a.y)), t1, t2, __fadd_ru(t1, t2));
+}
+
+// The extremes of the f32 orientation (b - a) x (p - a) over the corners of a
+// box: the first product depends on the corner's y alone and the second on
+// its x, and the rounded difference is monotone in both.
+__device__ __forceinline__ float2 box_orient(float2 a, float2 b, float4 q) {
+  const float dx = __fsub_rn(b.x, a.x), dy = __fsub_rn(b.y, a.y);
+  const float t0 = __fmul_rn(dx, __fsub_rn(q.y, a.y)), t1 = __fmul_rn(dx, __fsub_rn(q.w, a.y));
+  const float u0 = __fmul_rn(dy, __fsub_rn(q.x, a.x)), u1 = __fmul_rn(dy, __fsub_rn(q.z, a.x));
+  return make_float2(__fsub_rn(fminf(t0, t1), fmaxf(u0, u1)),
+                     __fsub_rn(fmaxf(t0, t1), fminf(u0, u1)));
+}
+
+// +1 / -1 when orient32 decides that side of the line ab for all of a box,
+// else 0 (undecided, or on both sides; also for NaN / inf).
+__device__ __forceinline__ int box_side32(float2 a, float2 b, float4 q) {
+  const float2 o = box_orient(a, b, q);
+  const float E = box_orient_bound(a, b, q);
+  if (o.x > E) return 1;
+  if (o.y < -E) return -1;
+  return 0;
+}
+
+// The same sign in FP64, decided when it clears 2^-40 of the two products
+// (their rounding and that of tg's divisions is 2^-51 of them).
+__device__ __forceinline__ int orient64(double2 a, double2 b, double2 p) {
+  const double t1 = __dmul_rn(__dsub_rn(b.x, a.x), __dsub_rn(p.y, a.y));
+  const double t2 = __dmul_rn(__dsub_rn(b.y, a.y), __dsub_rn(p.x, a.x));
+  const double o = __dsub_rn(t1, t2);
+  const double E = __dadd_rn(__dmul_rn(__dadd_rn(fabs(t1), fabs(t2)), 9.094947017729282e-13), 1e-280);
+  return o > E ? 1 : (o < -E ? -1 : 0);
 }
 
 // FP32 classification of one segment: returns kOut / kIn when it provably
@@ -264,7 +317,7 @@ __device__ __forceinline__ bool p_inside_open(float v32, float a, float b) {
 // against the exact boundary values.
 __device__ __forceinline__ int grid_index(float o, float step, int n, double v) {
   if (!(v >= (double)grid_edge(o, step, 0)) || !(v <= (double)grid_edge(o, step, n))) return -1;
-  int i = (int)floorf(__fdiv_rn(__fsub_rn(__double2float_rn(v), o), step));
+  int i = (int)__fdividef(__fsub_rn(__double2float_rn(v), o), step);
   i = i < 0 ? 0 : (i > n - 1 ? n - 1 : i);
   while (i > 0 && v < (double)grid_edge(o, step, i)) i--;
   while (i < n - 1 && v > (double)grid_edge(o, step, i + 1)) i++;
@@ -280,7 +333,7 @@ __device__ __forceinline__ int grid_index(float o, float step, int n, double v) 
 __device__ __forceinline__ int grid_index32(float o, float step, int n, float v32, double v) {
   const float e0 = grid_edge(o, step, 0), en = grid_edge(o, step, n);
   if (p_inside_open(v32, e0, en)) {
-    int i = (int)floorf(__fdiv_rn(__fsub_rn(v32, o), step));
+    int i = (int)__fdividef(__fsub_rn(v32, o), step);
     i = i < 0 ? 0 : (i > n - 1 ? n - 1 : i);
     while (i > 0 && v32 < grid_edge(o, step, i)) i--;
     while (i < n - 1 && v32 > grid_edge(o, step, i + 1)) i++;
@@ -291,21 +344,31 @@ __device__ __forceinline__ int grid_index32(float o, float step, int n, float v3
   return grid_index(o, step, n, v);
 }
 
-// Status of the grid cell holding p (0 mixed / no grid, 1 inside, 2 outside).
+// Centre of cell (i, j) of a grid: an f32 point of the cell.
+__device__ __forceinline__ float2 grid_centre(float4 q, int i, int j) {
+  return make_float2(
+      __fmul_rn(0.5f, __fadd_rn(grid_edge(q.x, q.z, i), grid_edge(q.x, q.z, i + 1))),
+      __fmul_rn(0.5f, __fadd_rn(grid_edge(q.y, q.w, j), grid_edge(q.y, q.w, j + 1))));
+}
+
+// Status of the grid cell holding p (1 inside, 2 outside, 0 mixed / no grid).
 // A clean cell is touched by no edge, so every point of it has the ring's
 // status there, on tg's arithmetic as well (the argument of the isolation
-// exit in ring_intersects_ring).  p32 is p rounded to nearest.
+// exit in ring_intersects_ring).  p32 is p rounded to nearest.  (One thread
+// alone does not walk a mixed cell's edges: the lanes of a warp then drift
+// apart, and the band scan was faster; packet.cu walks them warp by warp.)
 __device__ __forceinline__ int grid_point_status(const GeomsView& G, uint32_t r, double2 p,
                                                  float2 p32) {
   if (G.grid_meta == nullptr) return 0;
-  const uint2 m = G.grid_meta[r];
+  const uint4 m = G.grid_meta[r];
   if (m.y == 0) return 0;
   const float4 q = G.grid_rect[r];
   const int i = grid_index32(q.x, q.z, (int)m.y, p32.x, p.x);
   if (i < 0) return 0;
   const int j = grid_index32(q.y, q.w, (int)m.y, p32.y, p.y);
   if (j < 0) return 0;
-  return G.grid_status[m.x + (uint32_t)j * m.y + (uint32_t)i];
+  const uint32_t s = cell_state(G.grid_cell[m.x + (uint32_t)j * m.y + (uint32_t)i]);
+  return s < kCellMixed ? (int)s : 0;
 }
 
 // Status shared by every grid cell that holds the closed box of another ring
@@ -319,7 +382,7 @@ __device__ __forceinline__ int grid_point_status(const GeomsView& G, uint32_t r,
 __device__ __forceinline__ int grid_rect_status(const GeomsView& G, uint32_t r, Rect64 R,
                                                 float4 q) {
   if (!G.grid_rings || G.grid_meta == nullptr) return 0;
-  const uint2 m = G.grid_meta[r];
+  const uint4 m = G.grid_meta[r];
   if (m.y == 0) return 0;
   const float4 g = G.grid_rect[r];
   const int i0 = grid_index32(g.x, g.z, (int)m.y, q.x, R.x);
@@ -328,13 +391,52 @@ __device__ __forceinline__ int grid_rect_status(const GeomsView& G, uint32_t r, 
   const int j0 = grid_index32(g.y, g.w, (int)m.y, q.y, R.y);
   const int j1 = grid_index32(g.y, g.w, (int)m.y, q.w, R.w);
   if (j0 < 0 || j1 < 0 || j1 - j0 > 1) return 0;
-  const uint8_t* st = G.grid_status + m.x;
-  const int s = st[(uint32_t)j0 * m.y + (uint32_t)i0];
-  if (s == 0) return 0;
+  const uint32_t* cell = G.grid_cell + m.x;
+  const uint32_t s = cell_state(cell[(uint32_t)j0 * m.y + (uint32_t)i0]);
+  if (s == kCellUnknown || s >= kCellMixed) return 0;
   for (int j = j0; j <= j1; j++)
     for (int i = i0; i <= i1; i++)
-      if (st[(uint32_t)j * m.y + (uint32_t)i] != s) return 0;
-  return s;
+      if (cell_state(cell[(uint32_t)j * m.y + (uint32_t)i]) != s) return 0;
+  return (int)s;
+}
+
+// The cells of a grid that hold the box b (RN32 bounds of points or exact
+// boxes): borders are compared strictly, so what rounds into b lies in them,
+// and each of them meets the box; what reaches past the grid, which covers
+// the ring's rect, is outside the ring.
+struct CellRange {
+  int i0, i1, j0, j1;
+  bool past;  // the box reaches the grid's border
+};
+// 1: c holds the cells; 0: b lies strictly past the grid (outside the ring);
+// -1: not found (steps so small that an estimate is off by more than one).
+__device__ __forceinline__ int grid_cells(float4 q, int n, float4 b, CellRange& c) {
+  const float ex = grid_edge(q.x, q.z, n), ey = grid_edge(q.y, q.w, n);
+  if (b.z < q.x || b.x > ex || b.w < q.y || b.y > ey) return 0;
+  const float ix = __fdividef(1.0f, q.z), iy = __fdividef(1.0f, q.w);
+  bool ok = true;
+  auto first = [n, &ok](float o, float step, float inv, float v) {
+    int i = (int)fminf(fmaxf(v - o, 0.0f) * inv, (float)(n - 1));
+    if (i < n - 1 && grid_edge(o, step, i + 1) < v) i++;
+    if (i > 0 && !(grid_edge(o, step, i) < v)) i--;
+    ok = ok && (i == 0 || grid_edge(o, step, i) < v) &&
+         (i == n - 1 || !(grid_edge(o, step, i + 1) < v));
+    return i;
+  };
+  auto last = [n, &ok](float o, float step, float inv, float v) {
+    int i = (int)fminf(fmaxf(v - o, 0.0f) * inv, (float)(n - 1));
+    if (i > 0 && v < grid_edge(o, step, i)) i--;
+    if (i < n - 1 && !(v < grid_edge(o, step, i + 1))) i++;
+    ok = ok && (i == 0 || !(v < grid_edge(o, step, i))) &&
+         (i == n - 1 || v < grid_edge(o, step, i + 1));
+    return i;
+  };
+  c.i0 = first(q.x, q.z, ix, b.x);
+  c.i1 = last(q.x, q.z, ix, b.z);
+  c.j0 = first(q.y, q.w, iy, b.y);
+  c.j1 = last(q.y, q.w, iy, b.w);
+  c.past = b.x <= q.x || b.z >= ex || b.y <= q.y || b.w >= ey;
+  return ok ? 1 : -1;
 }
 
 // Plain FP64 form: tg's FP64 sequence for every segment it visits, with the
@@ -634,6 +736,7 @@ __device__ __forceinline__ bool ring_rects_intersect(const GeomsView& GA, uint32
 // which every point of ro shares), kIsoNear when a segment of rr comes near
 // the box, kIsoNoIndex when rr has no band index (or ro no segments).
 constexpr int kIsoNear = -4, kIsoNoIndex = -5;
+
 template <bool kFast>
 __device__ __forceinline__ int ring_isolation(const GeomsView& Gr, uint32_t rr,
                                               const GeomsView& Go, uint32_t ro, uint32_t& esc) {
@@ -701,9 +804,12 @@ __device__ __forceinline__ int ring_isolation(const GeomsView& Gr, uint32_t rr,
 // isolation exit does not decide, and whose first vertex is not in the larger
 // ring, returns kDeferred instead of running the vertex and segment loops.
 // Returns 1 / 0 (or kDeferred).
+//
+// kNear: the caller knows that an edge of ring ra comes near ring rb's box
+// (the isolation test is left out).
 constexpr int kDeferred = -2;
 
-template <bool kFast, bool kCheap = false>
+template <bool kFast, bool kCheap = false, bool kNear = false>
 __device__ __forceinline__ int ring_intersects_ring(const GeomsView& GA, uint32_t ra,
                                                     const GeomsView& GB, uint32_t rb,
                                                     uint32_t& esc) {
@@ -720,13 +826,13 @@ __device__ __forceinline__ int ring_intersects_ring(const GeomsView& GA, uint32_
   }
   const uint32_t Vo = Go->ring_vtx[ro];
   const int nso = Go->ring_nsegs[ro];
-  if (kFast && nso > 0) {
+  if (kFast && !kNear && nso > 0) {
     // the smaller ring's box inside clean cells of the larger ring: no edge
     // of the larger ring comes near, so the answer is the cells' status
     const int st = grid_rect_status(*Gr, rr, Go->ring_rect[ro], Go->ring_rect32[ro]);
     if (st != 0) return st == 1 ? 1 : 0;
   }
-  {
+  if (!kNear) {
     const int iso = ring_isolation<kFast>(*Gr, rr, *Go, ro, esc);
     if (iso >= 0) return iso;
     if (kCheap && iso == kIsoNear) {

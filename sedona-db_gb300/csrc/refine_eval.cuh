@@ -208,8 +208,8 @@ __global__ void __launch_bounds__(256, kMinBlocks)
   // with m_dev the pair count lives on the device (graph replays) and m is
   // the buffer capacity: flags past the count are cleared
   const uint64_t mm = m_dev ? min(*m_dev, m) : m;
-  // every lane runs the same number of loop trips so the warp-wide flush
-  // below sees all 32 lanes
+  // every lane runs the same number of loop trips so the warp-wide ballots
+  // and the flush below see all 32 lanes
   // chunk_trips > 0: each block takes chunk_trips consecutive runs of
   // blockDim.x slots (kRefineChunkTrips); 0: the grid strides over all slots
   // (the stream graph, whose pair count lives on the device)
@@ -219,37 +219,47 @@ __global__ void __launch_bounds__(256, kMinBlocks)
   const uint64_t step = chunk_trips ? (uint64_t)blockDim.x : stride;
   const uint64_t trips = chunk_trips ? chunk_trips : (m + stride - 1) / stride;
   const uint64_t nq = kPhase == 2 ? min((uint64_t)*qn, m) : 0;
+  // (all lanes make every trip together: a lane without a pair idles, and the
+  // queue is appended to by a ballot of the whole warp)
   for (uint64_t t = 0; t < trips; t++) {
     const uint64_t u = start + t * step;
-    if (u >= m) continue;
-    if (kPhase == 2 && u >= nq) continue;
     // a permutation with a device-side count covers slots [0, mm) only (the
     // caller clears the flags past mm)
-    if (kPhase != 2 && perm != nullptr && m_dev != nullptr && u >= mm) continue;
-    uint64_t k = perm ? (uint64_t)perm[u] : u;
-    if (kPhase == 2 && slot_perm != nullptr) k = k < m ? (uint64_t)slot_perm[k] : ~0ull;
-    if (k >= mm) {
-      if (kPhase != 2 && k < m) flags[k] = 0;
-      continue;
+    bool on = u < m && !(kPhase == 2 && u >= nq) &&
+              !(kPhase != 2 && perm != nullptr && m_dev != nullptr && u >= mm);
+    uint64_t k = ~0ull;
+    if (on) {
+      k = perm ? (uint64_t)perm[u] : u;
+      if (kPhase == 2 && slot_perm != nullptr) k = k < m ? (uint64_t)slot_perm[k] : ~0ull;
+      if (k >= mm) {
+        if (kPhase != 2 && k < m) flags[k] = 0;
+        on = false;
+      }
     }
-    const uint32_t b = cb[k], p = cp[k] - probe_base;
-    int r = eval<kFast, kPhase == 1>(B, b, P, p, predicate, esc);
-    if (kPhase == 1 && r == kDeferred) {
-      // one atomic per group of lanes that reach this point together
-      const unsigned act = __activemask();
-      const int lane = threadIdx.x & 31, leader = __ffs(act) - 1;
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(qn, (uint32_t)__popc(act));
-      base = __shfl_sync(act, base, leader);
-      queue[base + __popc(act & ((1u << lane) - 1u))] = slot_perm ? (uint32_t)u : (uint32_t)k;
-      continue;
+    int r = 0;
+    if (on) r = eval<kFast, kPhase == 1>(B, cb[k], P, cp[k] - probe_base, predicate, esc);
+    __syncwarp();
+    if (kPhase == 1) {
+      const bool defer = on && r == kDeferred;
+      const unsigned group = __ballot_sync(0xffffffffu, defer);
+      if (group) {
+        const int lane = threadIdx.x & 31;
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(qn, (uint32_t)__popc(group));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (defer)
+          queue[base + __popc(group & ((1u << lane) - 1u))] = slot_perm ? (uint32_t)u : (uint32_t)k;
+      }
+      if (defer) on = false;
     }
-    pairs++;
-    if (r < 0) {
-      status_fail(st, kUnsupported, k);
-      r = 0;
+    if (on) {
+      pairs++;
+      if (r < 0) {
+        status_fail(st, kUnsupported, k);
+        r = 0;
+      }
+      flags[k] = (uint8_t)r;
     }
-    flags[k] = (uint8_t)r;
   }
   flush_counters(st, esc, pairs);
 }

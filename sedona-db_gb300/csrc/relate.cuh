@@ -245,15 +245,16 @@ __device__ __noinline__ bool ring_intersects_segment(const GeomsView& G, uint32_
   return count >= 2;
 }
 
-// tg.c:3120-3156 tg_ring_contains_ring
-template <bool kFast>
+// tg.c:3120-3156 tg_ring_contains_ring.  kNear: the caller knows that an edge
+// of ring ra comes near ring rb's box (the isolation test is left out).
+template <bool kFast, bool kNear = false>
 __device__ __noinline__ bool ring_contains_ring(const GeomsView& GA, uint32_t ra,
                                                 const GeomsView& GB, uint32_t rb, bool aoe,
                                                 uint32_t& esc) {
   if (ring_npts(GA, ra) < 3 || ring_npts(GB, rb) < 3) return false;
   const Rect64 A = GA.ring_rect[ra], Bq = GB.ring_rect[rb];
   if (Bq.x < A.x || Bq.z > A.z || Bq.y < A.y || Bq.w > A.w) return false;
-  if (kFast) {
+  if (kFast && !kNear) {
     // b's box in clean cells of a: every point of b strictly inside (1) or
     // outside (2) a, and no edge of a meets b, whatever allow_on_edge says
     const int st = grid_rect_status(GA, ra, Bq, GB.ring_rect32[rb]);

@@ -1,0 +1,137 @@
+"""The packet refine (probe rows in Morton order, 32 to a traversal) against the
+candidate pairs' path and the oracle."""
+import numpy as np
+import pytest
+
+from gpu_util import pairs
+
+pytestmark = pytest.mark.gpu
+
+PREDS = ["intersects", "contains", "covers", "within", "coveredby", "touches", "equals", "disjoint"]
+
+
+@pytest.fixture(scope="module")
+def capi():
+    from sedona_gpuspatial import _build, capi
+    _build.build()
+    return capi
+
+
+def _star(rng, c, n, r):
+    ang = np.sort(rng.uniform(0, 2 * np.pi, n))
+    rad = r * rng.uniform(0.6, 1.0, n)
+    ring = c + np.stack([rad * np.cos(ang), rad * np.sin(ang)], 1)
+    return np.vstack([ring, ring[:1]])
+
+
+def _zones(rng, n, holes):
+    """Stars of 5 to 120 points (with and without cell grids), some with a star
+    hole, some multipolygons."""
+    from sedona_gpuspatial import wkb
+    out = []
+    for _ in range(n):
+        c = rng.uniform(0, 200, 2)
+        shell = _star(rng, c, int(rng.integers(5, 120)), rng.uniform(5, 40))
+        rings = [shell]
+        if holes and rng.random() < 0.5:
+            rings.append((c + (shell - c) / 3.0)[::-1])
+        if holes and rng.random() < 0.15:
+            out.append(wkb.wkb_multipolygon([rings, [_star(rng, rng.uniform(0, 200, 2), 30, 10.0)]]))
+        else:
+            out.append(wkb.wkb_polygon(rings))
+    return out
+
+
+def _probes(rng, n, kind, build):
+    """Points or polygons; some rows null or empty, some on a zone's vertices."""
+    from sedona_gpuspatial import wkb
+    out = []
+    for i in range(n):
+        u = rng.random()
+        if u < 0.03:
+            out.append(None)
+        elif u < 0.05:
+            out.append(wkb.wkb_point(np.nan, np.nan))
+        elif kind == "points":
+            out.append(wkb.wkb_point(*rng.uniform(-5, 205, 2)))
+        elif kind == "lattice":
+            out.append(wkb.wkb_point(*rng.integers(0, 200, 2).astype(float)))
+        elif kind == "mixed" and u < 0.3:
+            out.append(wkb.wkb_point(*rng.uniform(0, 200, 2)))
+        elif kind == "mixed" and u < 0.4:
+            out.append(build[int(rng.integers(0, len(build)))])
+        elif kind == "mixed" and u < 0.6:
+            a = _star(rng, rng.uniform(0, 200, 2), 6, 6.0)
+            out.append(wkb.wkb_multipolygon([[a], [_star(rng, rng.uniform(0, 200, 2), 5, 3.0)]]))
+        else:
+            c = rng.uniform(0, 200, 2)
+            a = _star(rng, c, int(rng.integers(3, 20)), np.exp(rng.uniform(-3, 4)))
+            rings = [a]
+            if kind == "mixed" and u < 0.7:
+                rings.append((c + (a - c) / 2.0)[::-1])
+            out.append(wkb.wkb_polygon(rings))
+    return out
+
+
+def _both(capi, build, probe, preds):
+    fast, general = capi.SpatialJoin(probe_order=1), capi.SpatialJoin(probe_order=1)
+    general.set_option("candidate_order", 0)  # (any set order takes the candidate pairs' path)
+    for j in (fast, general):
+        j.build(build)
+    for pred in preds:
+        b, p = fast.probe(probe, pred)
+        gb, gp = general.probe(probe, pred)
+        np.testing.assert_array_equal(b, gb, err_msg=pred)
+        np.testing.assert_array_equal(p, gp, err_msg=pred)
+        yield pred, b, p
+
+
+@pytest.mark.parametrize("kind", ["points", "lattice", "polygons", "mixed"])
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 127, 2500])
+def test_packet_same_pairs_and_positions(capi, oracle_lib, kind, n):
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(n * 7 + len(kind))
+    zones = _zones(rng, 60, holes=True)
+    build = wkb.column_from_values(zones)
+    if kind == "lattice":  # zones on integer vertices: points on edges and corners
+        build = wkb.column_from_values([
+            wkb.wkb_polygon([np.round(_star(rng, rng.integers(0, 200, 2), 40, 30.0))])
+            for _ in range(60)])
+    probe = wkb.column_from_values(_probes(rng, n, kind, zones))
+    for pred, b, p in _both(capi, build, probe, PREDS):
+        if pred != "disjoint" and n <= 127:
+            ob, op = oracle_lib.join(oracle_lib.Geoms(build), oracle_lib.Geoms(probe), pred,
+                                     nthreads=4)
+            assert pairs(b, p) == sorted(zip(op.tolist(), ob.tolist())), pred
+
+
+def test_packet_far_offset_and_huge_probes(capi):
+    """Coordinates whose FP32 copies carry few digits (the undecided sides go
+    to FP64 and to the full tests), and probes larger than the zones."""
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(3)
+    off = np.array([4.0e6, -7.0e6])
+    build = wkb.column_from_values([wkb.wkb_polygon([off + _star(rng, rng.uniform(0, 200, 2), 60, 30.0)])
+                                    for _ in range(40)])
+    probe = wkb.column_from_values(
+        [wkb.wkb_polygon([off + _star(rng, rng.uniform(0, 200, 2), 8, np.exp(rng.uniform(-2, 6)))])
+         for _ in range(1500)] +
+        [wkb.wkb_point(*(off + rng.uniform(0, 200, 2))) for _ in range(500)])
+    for _ in _both(capi, build, probe, PREDS):
+        pass
+
+
+def test_packet_capacities_grow(capi):
+    """More records and more open pairs than the first guess has room for."""
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(4)
+    build = wkb.column_from_values([wkb.wkb_polygon([_star(rng, np.zeros(2), 4, 50.0)])
+                                    for _ in range(40000)])
+    points = wkb.column_from_values([wkb.wkb_point(*rng.uniform(-40, 40, 2)) for _ in range(40)])
+    for _ in _both(capi, build, points, ["intersects"]):
+        pass
+    multi = wkb.column_from_values([
+        wkb.wkb_multipolygon([[_star(rng, rng.uniform(-40, 40, 2), 5, 3.0)],
+                              [_star(rng, rng.uniform(-40, 40, 2), 5, 3.0)]]) for _ in range(40)])
+    for _ in _both(capi, build, multi, ["intersects", "contains"]):
+        pass
