@@ -167,12 +167,14 @@ class JoinEngine {
   uint64_t refine_pairs(Workspace& ws, const GeomsView& probe, const uint32_t* cb,
                         const uint32_t* cp, uint64_t m, int predicate, double distance);
 
+  // Whether probes in Morton order take the packet kernels (packet.cuh).
+  bool packet_path(int predicate, bool points) const;
+
   JoinStats stats();
   void reset_stats();
 
  private:
   void split_points();
-  bool packet_path(int predicate, bool points) const;
   uint64_t packet_probe(Workspace& ws, int predicate, uint32_t probe_base, const uint32_t* order,
                         DeviceStatus& hst, uint64_t& launches);
   int device_;

@@ -115,6 +115,7 @@ StreamJoin::~StreamJoin() {
                     &cand_b_, &cand_p_, &flags_, &sums2_, &out_b_, &out_p_})
     b->release();
   psc_ = ProbeScratch();  // its buffers free on s_ too
+  packet_.release();
   cudaStreamSynchronize(s_);
   cudaStreamDestroy(s_);
   cudaFreeHost(h_tot_);
@@ -174,6 +175,7 @@ void StreamJoin::set_batches(const std::vector<WkbDeviceColumn>& cols) {
     ccap_ = (uint64_t)nrows_ * 8 + 1024;
     ocap_ = (uint64_t)nrows_ * 4 + 1024;
   }
+  chunks_cap_ = std::max<uint64_t>(chunks_cap_, nrows_ / 8 + 1024);
   SPJ_CUDA(cudaStreamSynchronize(s_));
   std::ostringstream sig;
   sig << eng_.build_geoms().n << "x" << eng_.build_geoms().nverts << "|" << nrows_ << "|"
@@ -181,34 +183,44 @@ void StreamJoin::set_batches(const std::vector<WkbDeviceColumn>& cols) {
   signature_ = sig.str();
 }
 
-void StreamJoin::build_graph(int predicate) {
-  destroy_graph();
-  // capacity-sized buffers
-  cand_b_.reserve((ccap_ + 1) * 4, s_);
-  cand_p_.reserve((ccap_ + 1) * 4, s_);
-  flags_.reserve(ccap_ + 1, s_);
-  sums2_.reserve(compact_sums_bytes((int64_t)ccap_), s_);
-  out_b_.reserve((ocap_ + 1) * 4, s_);
-  out_p_.reserve((ocap_ + 1) * 4, s_);
-  const EngineConfig cfg = eng_.config();
-  // probes in Morton order (coherent traversals, and a refine that takes
-  // neighbouring probes' candidates together); everything the ordering
-  // uses is reserved here, so the capture allocates nothing
-  const bool ordered = ccap_ < 0xFFFFFFFFull &&
-                       (cfg.probe_order > 0 || (cfg.probe_order == 0 && nrows_ >= kOrderMinRows));
-  if (ordered) {
-    reserve_probe_order(nrows_, psc_, s_);
-    reserve_candidate_order(nrows_, ccap_, psc_, s_);
-  }
-  SPJ_CUDA(cudaStreamSynchronize(s_));
-
-  const GeomsView B = eng_.build_geoms().view();
-  const LbvhView t = eng_.lbvh().view();
+GeomsView StreamJoin::probe_view() const {
   GeomsView P;  // the stream-wide probe column: points only
   P.n = nrows_;
   P.kind = kind_.as<uint8_t>();
   P.pt = pt_.as<double2>();
   P.box = box_.as<float4>();
+  return P;
+}
+
+void StreamJoin::build_graph(int predicate) {
+  destroy_graph();
+  const EngineConfig cfg = eng_.config();
+  // probes in Morton order (coherent traversals, and a refine that takes
+  // neighbouring probes together); everything the ordering uses is reserved
+  // here, so the capture allocates nothing
+  const bool want = cfg.probe_order > 0 || (cfg.probe_order == 0 && nrows_ >= kOrderMinRows);
+  graph_packet_ = want && nrows_ >= 2 && eng_.packet_path(predicate, true);
+  const bool ordered = want && (graph_packet_ || ccap_ < 0xFFFFFFFFull);
+  // capacity-sized buffers
+  if (graph_packet_) {
+    packet_.reserve(nrows_, chunks_cap_, 0, s_);
+  } else {
+    cand_b_.reserve((ccap_ + 1) * 4, s_);
+    cand_p_.reserve((ccap_ + 1) * 4, s_);
+    flags_.reserve(ccap_ + 1, s_);
+    sums2_.reserve(compact_sums_bytes((int64_t)ccap_), s_);
+  }
+  out_b_.reserve((ocap_ + 1) * 4, s_);
+  out_p_.reserve((ocap_ + 1) * 4, s_);
+  if (ordered) {
+    reserve_probe_order(nrows_, psc_, s_);
+    if (!graph_packet_) reserve_candidate_order(nrows_, ccap_, psc_, s_);
+  }
+  SPJ_CUDA(cudaStreamSynchronize(s_));
+
+  const GeomsView B = eng_.build_geoms().view();
+  const LbvhView t = eng_.lbvh().view();
+  const GeomsView P = probe_view();
   unsigned* queue = ctrl_.as<unsigned>();
   DeviceStatus* st = reinterpret_cast<DeviceStatus*>(ctrl_.as<uint8_t>() + 16);
   const BatchDesc* bd = batches_.as<BatchDesc>();
@@ -227,29 +239,43 @@ void StreamJoin::build_graph(int predicate) {
     k_stream_decode<256><<<grid, 256, 0, s_>>>(bd, cd, nchunks_, queue, kind_.as<uint8_t>(),
                                                pt_.as<double2>(), box_.as<float4>(), st);
   const uint32_t* order = ordered ? probe_order(t, box_.as<float4>(), nrows_, psc_, s_) : nullptr;
-  probe_count_into(t, box_.as<float4>(), nrows_, counts_.as<uint32_t>(), s_, order);
-  scan_u32_u64_into(counts_.as<uint32_t>(), offs_.as<uint64_t>(), nrows_, sums_.as<uint64_t>(),
-                    s_);
-  probe_scatter_from(t, box_.as<float4>(), nrows_, offs_.as<uint64_t>(), 0,
-                     cand_b_.as<uint32_t>(), cand_p_.as<uint32_t>(), s_, ccap_, order);
-  const uint32_t* cperm =
-      order ? candidate_order_into(order, counts_.as<uint32_t>(), offs_.as<uint64_t>(), nrows_,
-                                   ccap_, psc_, s_)
-            : nullptr;
-  // with a permutation the refine visits only the m candidates; the flags of
-  // the rest of the capacity are cleared here for the flag scan
-  if (cperm) SPJ_CUDA(cudaMemsetAsync(flags_.get(), 0, ccap_ + 1, s_));
-  refine_relation(B, P, cand_b_.as<uint32_t>(), cand_p_.as<uint32_t>(), ccap_, 0, predicate,
-                  cfg.refine_form, flags_.as<uint8_t>(), st, s_, d_m, cperm,
-                  refine_blocks(cfg.refine_min_blocks, false));
-  // compaction per 4096-flag tile (the flags past m are clear)
-  compact_count(flags_.as<uint8_t>(), (int64_t)ccap_, sums2_.as<uint64_t>(), s_);
-  compact_pairs_tiles(cand_b_.as<uint32_t>(), cand_p_.as<uint32_t>(), flags_.as<uint8_t>(),
-                      (int64_t)ccap_, sums2_.as<uint64_t>(), out_b_.as<uint32_t>(),
-                      out_p_.as<uint32_t>(), ocap_, s_);
-  SPJ_CUDA(cudaMemcpyAsync(h_tot_, d_m, 8, cudaMemcpyDeviceToHost, s_));
-  SPJ_CUDA(cudaMemcpyAsync(h_tot_ + 1, sums2_.as<uint64_t>() + compact_tiles((int64_t)ccap_), 8,
-                           cudaMemcpyDeviceToHost, s_));
+  const uint32_t* cperm = nullptr;
+  if (graph_packet_) {
+    // filter and refine in one traversal per 32 neighbouring rows
+    const PacketStore a = packet_.store(nrows_);
+    packet_join(t, B, P, true, order, predicate, counts_.as<uint32_t>(), a, st, s_);
+    scan_u32_u64_into(counts_.as<uint32_t>(), offs_.as<uint64_t>(), nrows_, sums_.as<uint64_t>(),
+                      s_);
+    packet_scatter(P, order, offs_.as<uint64_t>(), 0, a, out_b_.as<uint32_t>(),
+                   out_p_.as<uint32_t>(), ocap_, s_);
+    SPJ_CUDA(cudaMemcpyAsync(h_tot_, &st->counters[1], 8, cudaMemcpyDeviceToHost, s_));
+    SPJ_CUDA(cudaMemcpyAsync(h_tot_ + 1, d_m, 8, cudaMemcpyDeviceToHost, s_));
+    SPJ_CUDA(cudaMemcpyAsync(h_tot_ + 4, a.ctrl, 8, cudaMemcpyDeviceToHost, s_));
+  } else {
+    probe_count_into(t, box_.as<float4>(), nrows_, counts_.as<uint32_t>(), s_, order);
+    scan_u32_u64_into(counts_.as<uint32_t>(), offs_.as<uint64_t>(), nrows_, sums_.as<uint64_t>(),
+                      s_);
+    probe_scatter_from(t, box_.as<float4>(), nrows_, offs_.as<uint64_t>(), 0,
+                       cand_b_.as<uint32_t>(), cand_p_.as<uint32_t>(), s_, ccap_, order);
+    cperm =
+        order ? candidate_order_into(order, counts_.as<uint32_t>(), offs_.as<uint64_t>(), nrows_,
+                                     ccap_, psc_, s_)
+              : nullptr;
+    // with a permutation the refine visits only the m candidates; the flags of
+    // the rest of the capacity are cleared here for the flag scan
+    if (cperm) SPJ_CUDA(cudaMemsetAsync(flags_.get(), 0, ccap_ + 1, s_));
+    refine_relation(B, P, cand_b_.as<uint32_t>(), cand_p_.as<uint32_t>(), ccap_, 0, predicate,
+                    cfg.refine_form, flags_.as<uint8_t>(), st, s_, d_m, cperm,
+                    refine_blocks(cfg.refine_min_blocks, false));
+    // compaction per 4096-flag tile (the flags past m are clear)
+    compact_count(flags_.as<uint8_t>(), (int64_t)ccap_, sums2_.as<uint64_t>(), s_);
+    compact_pairs_tiles(cand_b_.as<uint32_t>(), cand_p_.as<uint32_t>(), flags_.as<uint8_t>(),
+                        (int64_t)ccap_, sums2_.as<uint64_t>(), out_b_.as<uint32_t>(),
+                        out_p_.as<uint32_t>(), ocap_, s_);
+    SPJ_CUDA(cudaMemcpyAsync(h_tot_, d_m, 8, cudaMemcpyDeviceToHost, s_));
+    SPJ_CUDA(cudaMemcpyAsync(h_tot_ + 1, sums2_.as<uint64_t>() + compact_tiles((int64_t)ccap_), 8,
+                             cudaMemcpyDeviceToHost, s_));
+  }
   SPJ_CUDA(cudaMemcpyAsync(h_tot_ + 2, &st->first_bad, 8, cudaMemcpyDeviceToHost, s_));
   SPJ_CUDA(cudaMemcpyAsync(h_tot_ + 3, &st->counters[0], 8, cudaMemcpyDeviceToHost, s_));
   SPJ_CUDA(cudaStreamEndCapture(s_, &g));
@@ -259,7 +285,8 @@ void StreamJoin::build_graph(int predicate) {
   graph_pred_ = predicate;
   // memsets 2, decode 1, count 1, scan 3, scatter 1, refine 1, flag counts 2, compact 1;
   // ordered: keys 1 + 4 radix passes of 5, candidate order 5, flags memset 1
-  stats_.launches_per_replay = 12 + (cperm ? 27 : (order ? 21 : 0));
+  // (packets: memsets 3, decode 1, order 21, packets 1, join 1, scan 3, scatter 1)
+  stats_.launches_per_replay = graph_packet_ ? 31 : 12 + (cperm ? 27 : (order ? 21 : 0));
 }
 
 uint64_t StreamJoin::run(int predicate, const uint32_t** d_build, const uint32_t** d_probe) {
@@ -275,7 +302,13 @@ uint64_t StreamJoin::run(int predicate, const uint32_t** d_build, const uint32_t
     check_traversal(eng_.lbvh().view(), s_);
     m = h_tot_[0];
     total = h_tot_[1];
-    if (m > ccap_) {
+    if (graph_packet_ && h_tot_[4] > chunks_cap_) {
+      // the packets' records did not fit: grow, re-capture, replay
+      chunks_cap_ = h_tot_[4] + h_tot_[4] / 8;
+      destroy_graph();
+      continue;
+    }
+    if (!graph_packet_ && m > ccap_) {
       // candidates did not fit: grow, re-capture, replay (results discarded)
       ccap_ = m + m / 8 + 1024;
       destroy_graph();
@@ -288,12 +321,21 @@ uint64_t StreamJoin::run(int predicate, const uint32_t** d_build, const uint32_t
     }
     if (total > ocap_) {
       ocap_ = total + total / 8 + 1024;
+      const bool packet = graph_packet_;
       destroy_graph();
-      continue;
+      if (!packet) continue;
+      // the records are complete: only the pairs are written again
+      out_b_.reserve((ocap_ + 1) * 4, s_);
+      out_p_.reserve((ocap_ + 1) * 4, s_);
+      packet_scatter(probe_view(), psc_.order.as<uint32_t>(), offs_.as<uint64_t>(), 0,
+                     packet_.store(nrows_), out_b_.as<uint32_t>(), out_p_.as<uint32_t>(), ocap_,
+                     s_);
+      SPJ_CUDA(cudaStreamSynchronize(s_));
     }
     break;
   }
-  SPJ_CHECK(m <= ccap_ && total <= ocap_, "stream: capacities did not settle");
+  SPJ_CHECK((graph_packet_ ? h_tot_[4] <= chunks_cap_ : m <= ccap_) && total <= ocap_,
+            "stream: capacities did not settle");
   float ms = 0;
   SPJ_CUDA(cudaEventElapsedTime(&ms, ev0_, ev1_));
   stats_.ms_last = ms;

@@ -64,6 +64,7 @@ class StreamJoin {
 
  private:
   void build_graph(int predicate);
+  GeomsView probe_view() const;
   void destroy_graph();
   JoinEngine& eng_;
   cudaStream_t s_ = nullptr;
@@ -72,8 +73,11 @@ class StreamJoin {
   DevBuf kind_, pt_, box_, counts_, offs_, sums_;  // stream-wide decoded column
   DevBuf cand_b_, cand_p_, flags_, sums2_, out_b_, out_p_;
   ProbeScratch psc_;  // the probes' Morton order and the candidates' permutation
-  uint64_t* h_tot_ = nullptr;  // pinned: candidates, pairs, status, escalations
-  uint64_t ccap_ = 0, ocap_ = 0;
+  PacketBufs packet_;  // records of the packet refine (ordered streams)
+  // pinned: candidates, pairs, status, escalations, packet chunks
+  uint64_t* h_tot_ = nullptr;
+  uint64_t ccap_ = 0, ocap_ = 0, chunks_cap_ = 0;
+  bool graph_packet_ = false;
   uint32_t nrows_ = 0, nchunks_ = 0, nbatches_ = 0;
   std::vector<WkbDeviceColumn> cols_;
   cudaGraphExec_t exec_ = nullptr;
