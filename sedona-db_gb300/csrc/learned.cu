@@ -1,6 +1,7 @@
 // learned.cu — learned point index (see learned.cuh): Hilbert keys, device
 // radix sort, GPU training of the two-stage piecewise-linear model, and the
 // lookup / range kernels with LBVH fallback.
+#include <algorithm>
 #include <cmath>
 
 #include "learned.cuh"
@@ -386,22 +387,16 @@ __device__ __forceinline__ int row_class(uint8_t kind, int predicate, DeviceStat
 constexpr uint32_t kRangeSorted = 0;  // ranks in the key-sorted build points
 constexpr uint32_t kRangeLeaf = 1;    // an LBVH leaf (sorted primitive indices)
 
-// A row's first kRangeCache ranges are kept by the counting pass (start,
-// len | kind << 31), so the writing pass copies them instead of searching
-// again; rows with more ranges search again.
-constexpr uint32_t kRangeCache = 8;
-
 // ranges are written at pos < cap only (the count pass sized them)
 template <int kPass>
 __device__ __forceinline__ void put_range(uint4* ranges, uint64_t& pos, uint32_t& cnt,
                                           uint32_t start, uint32_t len, uint32_t row,
-                                          uint32_t kind, uint64_t cap, uint2* cache) {
+                                          uint32_t kind, uint64_t cap) {
   if (len == 0) return;
   if (kPass) {
     if (pos < cap) ranges[pos] = make_uint4(start, len, row, kind);
     pos++;
   } else {
-    if (cnt < kRangeCache) cache[(size_t)row * kRangeCache + cnt] = make_uint2(start, len | (kind << 31));
     cnt++;
   }
 }
@@ -409,7 +404,7 @@ __device__ __forceinline__ void put_range(uint4* ranges, uint64_t& pos, uint32_t
 // The LBVH leaves whose boxes overlap q, as ranges (the fallback).
 template <int kPass>
 __device__ void leaf_ranges(const LbvhView& t, float4 q, int* stack, uint32_t row, uint4* ranges,
-                            uint64_t& pos, uint32_t& cnt, uint64_t cap, uint2* cache) {
+                            uint64_t& pos, uint32_t& cnt, uint64_t cap) {
   if (t.nprims == 0) return;
   const uint64_t max_steps = 2ull * t.nleaves + 2;
   uint64_t steps = 0;
@@ -426,7 +421,7 @@ __device__ void leaf_ranges(const LbvhView& t, float4 q, int* stack, uint32_t ro
         break;
       }
       const uint32_t b0 = c * t.leaf_size, b1 = min(b0 + t.leaf_size, t.nprims);
-      put_range<kPass>(ranges, pos, cnt, b0, b1 - b0, row, kRangeLeaf, cap, cache);
+      put_range<kPass>(ranges, pos, cnt, b0, b1 - b0, row, kRangeLeaf, cap);
     } else {
       if ((uint32_t)node + 1 >= t.nleaves) {
         traversal_fault(t, kBadNode, (unsigned)node);
@@ -474,99 +469,222 @@ __global__ void k_row_keys(LearnedView v, GeomsView P, uint32_t* __restrict__ ke
 // for a lookup the run of its key among the sorted keys (found through the
 // model), for a box the runs of the grid cells it covers, and LBVH leaves
 // where the model's error exceeds the window or the box covers too many
-// cells.  Pass 0 counts, pass 1 writes at the scanned offsets (row order).
-template <int kPass>
+// cells.
+
+// The grid cells of a range row's box.
+struct BoxCells {
+  uint32_t x0, y0, w;
+  uint64_t n;  // 0: an empty box
+};
+__device__ __forceinline__ BoxCells box_cells(const LearnedView& v, float4 b) {
+  BoxCells c{0, 0, 1, 0};
+  if (!(b.x <= b.z && b.y <= b.w)) return c;
+  c.x0 = cell_of(b.x, v.x0, v.sx);
+  c.y0 = cell_of(b.y, v.y0, v.sy);
+  c.w = cell_of(b.z, v.x0, v.sx) - c.x0 + 1;
+  c.n = (uint64_t)c.w * (cell_of(b.w, v.y0, v.sy) - c.y0 + 1);
+  return c;
+}
+
+// The run of the keys equal to q.  range: a cell of a range row, whose leaf's
+// error was checked against window_box (the lookup window does not apply).
+__device__ __forceinline__ void key_run(const LearnedView& v, uint32_t q, bool range,
+                                        uint32_t& steps, uint32_t& misses, uint32_t& lo,
+                                        uint32_t& hi, bool& bad) {
+  LearnedView w = v;
+  if (range) w.window = 0xFFFFFFFFu;
+  uint32_t rsteps = 0;  // the run after the search (independent of the model, not counted)
+  lo = learned_lower_bound(w, q, steps, misses, bad);
+  hi = bad ? lo : run_end(v.keys, v.n, lo, q, rsteps);
+}
+
+// Counts the ranges, and keeps them: a warp takes 32 rows (in key order) and
+// lists all their cells, which its lanes search 32 at a time, whatever row
+// they belong to (rows hold from one to 256 cells: one row per lane left most
+// of the warp idle, and rows of more than eight ranges were searched again by
+// the writing pass; 2M boxes x 20M points: 3.28 + 1.99 ms, 0.75 + 0.14 now).  The
+// non-empty runs go to consecutive places of `found` (rstart: a row's first;
+// kNotKept: LBVH rows, and rows past its end, which are searched again).
+// check: some leaf's error is over window_box.
+constexpr uint32_t kNotKept = 0xFFFFFFFFu;
 __global__ void __launch_bounds__(128)
-    k_learned_ranges(LearnedView v, LbvhView t, GeomsView P, int predicate,
+    k_learned_search(LearnedView v, LbvhView t, GeomsView P, int predicate, bool check,
                      const uint32_t* __restrict__ order, uint32_t* __restrict__ rcount,
-                     const uint64_t* __restrict__ roff, uint4* __restrict__ ranges,
-                     uint64_t cap, uint2* __restrict__ cache, unsigned long long* __restrict__ ctr,
-                     DeviceStatus* st) {
+                     uint32_t* __restrict__ rstart, uint2* __restrict__ found, uint64_t cap,
+                     unsigned long long* __restrict__ cursor,
+                     unsigned long long* __restrict__ ctr, DeviceStatus* st) {
   __shared__ int stack[kTravStack * 128];
-  // steps: the model-guided lower_bound searches; rsteps: the runs of equal
-  // keys after them (independent of the model, not counted)
-  uint32_t steps = 0, misses = 0, fallbacks = 0, lookups = 0, rsteps = 0;
-  for (uint32_t jj = blockIdx.x * blockDim.x + threadIdx.x; jj < P.n;
-       jj += gridDim.x * blockDim.x) {
-    const uint32_t i = order ? order[jj] : jj;
-    if (i >= P.n) {
-      traversal_fault(t, kBadProbe, i);
-      continue;
-    }
-    const int cls = row_class(P.kind[i], predicate, st, i, kPass == 0);
-    uint32_t cnt = 0;
-    uint64_t pos = kPass ? roff[i] : 0;
-    if (kPass) {
-      const uint64_t nr = roff[i + 1] - pos;
-      if (nr <= kRangeCache) {  // kept by the counting pass
-        for (uint32_t c = 0; c < (uint32_t)nr; c++) {
-          const uint2 e = cache[(size_t)i * kRangeCache + c];
-          if (pos < cap) ranges[pos] = make_uint4(e.x, e.y & 0x7FFFFFFFu, i, e.y >> 31);
-          pos++;
-        }
-        continue;
+  const unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  uint32_t steps = 0, misses = 0, fallbacks = 0, lookups = 0;
+  for (uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; w * 32 < P.n; w += nw) {
+    const uint64_t jj = w * 32 + lane;
+    uint32_t i = jj < P.n ? (order ? order[jj] : (uint32_t)jj) : P.n;
+    if (jj < P.n && i >= P.n) traversal_fault(t, kBadProbe, i);
+    const bool have = i < P.n;
+    int cls = kRowNone;
+    float4 box = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    BoxCells c{0, 0, 1, 0};
+    bool tree = false;
+    uint32_t items = 0;
+    if (have) {
+      cls = row_class(P.kind[i], predicate, st, i, true);
+      box = P.box[i];
+      if (cls == kRowLookup) {
+        items = 1;
+      } else if (cls == kRowRange) {
+        c = box_cells(v, box);
+        tree = c.n > kMaxCells;
+        items = tree ? 0u : (uint32_t)c.n;
       }
     }
-    if (cls == kRowLookup) {
-      const float4 pb = P.box[i];
-      const uint32_t q = key_of(v, make_float2(pb.x, pb.y));
+    const uint32_t incl = warp_inclusive_scan(items), excl = incl - items;
+    const uint32_t total = __shfl_sync(all, incl, 31);
+    // the items among [base, base + 32) that are this lane's row's
+    auto mine = [&](uint32_t base) {
+      const uint32_t a = max(excl, base), b = min(incl, base + 32);
+      if (b <= a) return 0u;
+      return (b - a == 32 ? all : (1u << (b - a)) - 1u) << (a - base);
+    };
+    // item base + lane: its row's lane, and its key
+    auto item = [&](uint32_t base, int& L, uint32_t& q) {
+      const uint32_t x = base + lane;
+      L = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const uint32_t e = __shfl_sync(all, excl, L + step);
+        if (e <= x) L += step;
+      }
+      const int lc = __shfl_sync(all, cls, L);
+      const uint32_t x0 = __shfl_sync(all, c.x0, L), y0 = __shfl_sync(all, c.y0, L);
+      const uint32_t cw = __shfl_sync(all, c.w, L), k = x - __shfl_sync(all, excl, L);
+      const float bx = __shfl_sync(all, box.x, L), by = __shfl_sync(all, box.y, L);
+      q = lc == kRowLookup ? key_of(v, make_float2(bx, by)) : hilbert16(x0 + k % cw, y0 + k / cw);
+      return lc == kRowRange;
+    };
+    if (check) {
+      // a cell whose leaf is over the window sends the row to the LBVH
+      for (uint32_t base = 0; base < total; base += 32) {
+        int L;
+        uint32_t q;
+        const bool range = item(base, L, q);
+        const bool over =
+            range && base + lane < total && v.err[root_leaf(v, q)] > v.window_box;
+        const unsigned o = __ballot_sync(all, over);
+        if (o & mine(base)) tree = true;
+      }
+    }
+    unsigned long long at = 0;
+    if (lane == 0 && total) at = atomicAdd(cursor, (unsigned long long)total);
+    at = __shfl_sync(all, at, 0);
+    const bool keep = at + total <= cap;
+    uint32_t cnt = 0, start = 0, run = 0;
+    for (uint32_t base = 0; base < total; base += 32) {
+      int L;
+      uint32_t q;
+      const bool range = item(base, L, q);
+      const bool skip = __shfl_sync(all, (int)tree, L) != 0;
+      uint32_t lo = 0, hi = 0;
       bool bad = false;
-      lookups++;
-      const uint32_t lo = learned_lower_bound(v, q, steps, misses, bad);
-      if (!bad) {
-        const uint32_t hi = run_end(v.keys, v.n, lo, q, rsteps);
-        put_range<kPass>(ranges, pos, cnt, lo, hi - lo, i, kRangeSorted, cap, cache);
-      } else {
-        fallbacks++;
-        leaf_ranges<kPass>(t, pb, stack + threadIdx.x, i, ranges, pos, cnt, cap, cache);
+      if (base + lane < total && !skip) {
+        lookups++;
+        key_run(v, q, range, steps, misses, lo, hi, bad);
       }
-    } else if (cls == kRowRange) {
-      const float4 bx = P.box[i];  // outward f32 box of the probe polygon
-      const uint32_t cx0 = cell_of(bx.x, v.x0, v.sx), cx1 = cell_of(bx.z, v.x0, v.sx);
-      const uint32_t cy0 = cell_of(bx.y, v.y0, v.sy), cy1 = cell_of(bx.w, v.y0, v.sy);
-      const uint64_t ncell = (uint64_t)(cx1 - cx0 + 1) * (cy1 - cy0 + 1);
-      if (bx.x <= bx.z && bx.y <= bx.w) {  // (an empty box has no pairs)
-        bool use_tree = ncell > kMaxCells;
-        // a cell whose leaf is over the window sends the row to the LBVH
-        for (uint32_t cy = cy0; cy <= cy1 && !use_tree; cy++)
-          for (uint32_t cx = cx0; cx <= cx1 && !use_tree; cx++)
-            use_tree = v.err[root_leaf(v, hilbert16(cx, cy))] > v.window_box;
-        if (!use_tree) {
-          for (uint32_t cy = cy0; cy <= cy1; cy++) {
-            for (uint32_t cx = cx0; cx <= cx1; cx++) {
-              const uint32_t q = hilbert16(cx, cy);
-              bool bad = false;
-              lookups++;
-              // (the leaf's error is within window_box, checked above; the
-              // search below uses it whatever the lookup window is)
-              LearnedView vb = v;
-              vb.window = 0xFFFFFFFFu;
-              const uint32_t lo = learned_lower_bound(vb, q, steps, misses, bad);
-              const uint32_t hi = run_end(v.keys, v.n, lo, q, rsteps);
-              put_range<kPass>(ranges, pos, cnt, lo, hi - lo, i, kRangeSorted, cap, cache);
-            }
-          }
-        } else {
-          fallbacks++;
-          leaf_ranges<kPass>(t, bx, stack + threadIdx.x, i, ranges, pos, cnt, cap, cache);
-        }
+      __syncwarp();
+      const unsigned some = __ballot_sync(all, hi > lo), no = __ballot_sync(all, bad);
+      if (hi > lo && keep)
+        found[at + run + __popc(some & ((1u << lane) - 1u))] = make_uint2(lo, hi - lo);
+      const unsigned m = mine(base);
+      if (m) {
+        if (excl >= base) start = run + __popc(some & ((1u << (excl - base)) - 1u));
+        cnt += __popc(some & m);
+        if (no & m) tree = true;  // (a lookup whose leaf is over its window)
       }
+      run += __popc(some);
     }
-    if (!kPass) rcount[i] = cnt;
+    if (tree) {
+      fallbacks++;
+      uint64_t pos = 0;
+      cnt = 0;
+      leaf_ranges<0>(t, box, stack + threadIdx.x, i, nullptr, pos, cnt, 0);
+    }
+    __syncwarp();
+    if (have) {
+      rcount[i] = cnt;
+      rstart[i] = tree || !keep ? kNotKept : (uint32_t)at + start;
+    }
   }
-  if (kPass == 0) {
-    for (int o = 16; o > 0; o >>= 1) {
-      steps += __shfl_xor_sync(0xffffffffu, steps, o);
-      misses += __shfl_xor_sync(0xffffffffu, misses, o);
-      fallbacks += __shfl_xor_sync(0xffffffffu, fallbacks, o);
-      lookups += __shfl_xor_sync(0xffffffffu, lookups, o);
+  for (int o = 16; o > 0; o >>= 1) {
+    steps += __shfl_xor_sync(all, steps, o);
+    misses += __shfl_xor_sync(all, misses, o);
+    fallbacks += __shfl_xor_sync(all, fallbacks, o);
+    lookups += __shfl_xor_sync(all, lookups, o);
+  }
+  if (lane == 0) {
+    atomicAdd(&ctr[0], (unsigned long long)lookups);
+    atomicAdd(&ctr[1], (unsigned long long)misses);
+    atomicAdd(&ctr[2], (unsigned long long)fallbacks);
+    atomicAdd(&ctr[3], (unsigned long long)steps);
+  }
+}
+
+// The ranges at their places (roff: scan of the counts), in row order: a warp
+// takes 32 consecutive rows, whose ranges are consecutive, and copies what the
+// search kept; a row that was not kept is searched again by its lane.
+__global__ void __launch_bounds__(128)
+    k_learned_write(LearnedView v, LbvhView t, GeomsView P, int predicate,
+                    const uint64_t* __restrict__ roff, const uint32_t* __restrict__ rstart,
+                    const uint2* __restrict__ found, uint4* __restrict__ ranges, uint64_t cap,
+                    DeviceStatus* st) {
+  __shared__ int stack[kTravStack * 128];
+  const unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; w * 32 < P.n; w += nw) {
+    const uint64_t row = w * 32 + lane;
+    const bool have = row < P.n;
+    const uint64_t r0 = have ? roff[row] : ~0ull;
+    const uint64_t r1 = have ? roff[row + 1] : ~0ull;
+    const uint32_t start = have ? rstart[row] : kNotKept;
+    const uint64_t e0 = __shfl_sync(all, r0, 0);
+    const uint64_t e1 = roff[w * 32 + 32 < P.n ? w * 32 + 32 : P.n];
+    for (uint64_t base = e0; base < e1; base += 32) {
+      const uint64_t e = base + lane;
+      int L = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const uint64_t s = __shfl_sync(all, r0, L + step);
+        if (s <= e) L += step;
+      }
+      const uint32_t from = __shfl_sync(all, start, L);
+      const uint64_t k = e - __shfl_sync(all, r0, L);
+      if (e < e1 && e < cap && from != kNotKept) {
+        const uint2 f = found[from + k];
+        ranges[e] = make_uint4(f.x, f.y, (uint32_t)(w * 32) + L, kRangeSorted);
+      }
     }
-    if ((threadIdx.x & 31) == 0) {
-      atomicAdd(&ctr[0], (unsigned long long)lookups);
-      atomicAdd(&ctr[1], (unsigned long long)misses);
-      atomicAdd(&ctr[2], (unsigned long long)fallbacks);
-      atomicAdd(&ctr[3], (unsigned long long)steps);
+    if (have && start == kNotKept && r1 > r0) {
+      const uint32_t i = (uint32_t)row;
+      const int cls = row_class(P.kind[i], predicate, st, i, false);
+      const float4 box = P.box[i];
+      uint64_t pos = r0;
+      uint32_t cnt = 0, steps = 0, misses = 0, lo, hi;
+      bool bad = false;
+      const BoxCells c = cls == kRowRange ? box_cells(v, box) : BoxCells{0, 0, 1, 1};
+      bool tree = cls == kRowRange && c.n > kMaxCells;
+      for (uint32_t k = 0; k < c.n && cls == kRowRange && !tree; k++)
+        tree = v.err[root_leaf(v, hilbert16(c.x0 + k % c.w, c.y0 + k / c.w))] > v.window_box;
+      for (uint32_t k = 0; k < c.n && !tree; k++) {
+        const uint32_t q = cls == kRowLookup ? key_of(v, make_float2(box.x, box.y))
+                                             : hilbert16(c.x0 + k % c.w, c.y0 + k / c.w);
+        key_run(v, q, cls == kRowRange, steps, misses, lo, hi, bad);
+        if (bad) tree = true;
+        else put_range<1>(ranges, pos, cnt, lo, hi - lo, i, kRangeSorted, cap);
+      }
+      if (tree) leaf_ranges<1>(t, box, stack + threadIdx.x, i, ranges, pos, cnt, cap);
     }
+    __syncwarp();
   }
 }
 
@@ -960,20 +1078,26 @@ uint64_t LearnedIndex::query(const GeomsView& probe, uint32_t probe_base, int pr
   // phase A: ranges per row
   counts_.reserve(rb, s);
   offs_.reserve(((size_t)np + 1) * 8, s);
-  rcache_.reserve(((size_t)np + 1) * kRangeCache * sizeof(uint2), s);
+  // room for the kept runs: boxes of the size of a few cells hold six on average
+  const uint64_t kept = std::min<uint64_t>((uint64_t)np * 12 + 4096, kNotKept - 1u);
+  rcache_.reserve(kept * sizeof(uint2), s);
+  rstart_.reserve(rb, s);
   const int ga = grid_for(np, 128, kNumSMs * 16);
-  k_learned_ranges<0><<<ga, 128, 0, s>>>(v, tv_, probe, predicate, order_.as<uint32_t>(),
-                                         counts_.as<uint32_t>(), nullptr, nullptr, 0,
-                                         rcache_.as<uint2>(), ctr, st);
+  const bool check = !host_err_.empty() &&
+                     *std::max_element(host_err_.begin(), host_err_.end()) > window_box_;
+  k_learned_search<<<ga, 128, 0, s>>>(v, tv_, probe, predicate, check,
+                                      order_.as<uint32_t>(), counts_.as<uint32_t>(),
+                                      rstart_.as<uint32_t>(), rcache_.as<uint2>(), kept, ctr + 6,
+                                      ctr, st);
   scan_u32_u64(counts_.as<uint32_t>(), offs_.as<uint64_t>(), np, tmp_, s);
   uint64_t nr = 0;
   SPJ_CUDA(cudaMemcpyAsync(&nr, offs_.as<uint64_t>() + np, 8, cudaMemcpyDeviceToHost, s));
   check_status(scratch_, s, "learned query");  // syncs
   check_traversal(tv_, s);
   ranges_.reserve((nr + 1) * sizeof(uint4), s);
-  k_learned_ranges<1><<<ga, 128, 0, s>>>(v, tv_, probe, predicate, order_.as<uint32_t>(), nullptr,
-                                         offs_.as<uint64_t>(), ranges_.as<uint4>(), nr,
-                                         rcache_.as<uint2>(), ctr, st);
+  k_learned_write<<<ga, 128, 0, s>>>(v, tv_, probe, predicate, offs_.as<uint64_t>(),
+                                     rstart_.as<uint32_t>(), rcache_.as<uint2>(),
+                                     ranges_.as<uint4>(), nr, st);
   SPJ_CUDA(cudaEventRecord(ev_[2], s));
   // phase B: candidates of the ranges, a warp per 32 ranges
   const uint64_t nch = (nr + 31) / 32;

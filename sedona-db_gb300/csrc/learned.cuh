@@ -85,7 +85,7 @@ class LearnedIndex {
       scratch_;
   DevBuf root_tab_;
   DevBuf order_, okeys_, akeys_, avals_, ranges_, ccount_, coff_;  // query scratch
-  DevBuf rcache_, cwords_, woff_, masks_;
+  DevBuf rcache_, rstart_, cwords_, woff_, masks_;
   std::vector<uint32_t> host_err_, host_start_;  // per-leaf errors, leaf starts
   cudaEvent_t ev_[4] = {};
   uint32_t root_shift_ = 0, root_p_ = 1;

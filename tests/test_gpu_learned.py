@@ -138,3 +138,45 @@ def test_window_autotune_keeps_pairs(env):
         for p in ("boxes", "lookups"):
             assert pairs(*device_pairs(*li.query_device(dev[p][0], "intersects"))) == ref[p]
     li.set_window(4096)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 2000])
+@pytest.mark.parametrize("window", [4096, 8])
+def test_learned_rows_of_unlike_cell_counts(env, n, window):
+    """Boxes of one to several hundred grid cells, lookups, nulls and empty rows
+    side by side: warps whose rows' searches are dealt out to all lanes, rows
+    past the room for kept runs, and rows that go to the LBVH (too many cells,
+    or a leaf over a small window)."""
+    capi, oracle, li, dev, cols = env
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(n + window)
+    vals = []
+    for i in range(n):
+        u = rng.random()
+        c = rng.uniform(0, 1e5, 2) if u < 0.3 else np.frombuffer(
+            cols["build"].value(int(rng.integers(0, len(cols["build"]))))[5:], "<f8")
+        if u < 0.04:
+            vals.append(None)
+        elif u < 0.08:
+            vals.append(wkb.wkb_point(np.nan, np.nan))
+        elif u < 0.25 or u > 0.9:
+            vals.append(wkb.wkb_point(*c))
+        else:
+            h = np.exp(rng.uniform(np.log(0.01), np.log(16.0)))
+            vals.append(wkb.wkb_polygon([[(c[0] - h, c[1] - h), (c[0] + h, c[1] - h),
+                                          (c[0] + h, c[1] + h), (c[0] - h, c[1] + h),
+                                          (c[0] - h, c[1] - h)]]))
+    probe = wkb.column_from_values(vals)
+    d, keep = device_column(capi, probe)
+    if probe.validity is not None:
+        import torch
+        valid = torch.from_numpy(probe.validity).cuda()
+        d.validity = valid.data_ptr()
+    li.set_window(window)
+    try:
+        db, dp, m = li.query_device(d, "intersects")
+        b, p = device_pairs(db, dp, m)
+    finally:
+        li.set_window(4096)
+    assert np.all(np.diff(p.astype(np.int64)) >= 0)
+    assert pairs(b, p) == _oracle_pairs(oracle, cols["build"], probe, "intersects")
