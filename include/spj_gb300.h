@@ -120,7 +120,9 @@ int SpjJoinFinishBuild(SpjJoin* join);
  *                       Morton order), 1 on, 0 off: fused ST_DWithin keeps
  *                       the results past a probe's slots in an overflow
  *                       arena (of the slots' size), so only probes it cannot
- *                       hold are traversed again
+ *                       hold are traversed again.  With this and dwithin_slots
+ *                       left alone, probes in Morton order are traversed 32
+ *                       at a time, with neither
  *   "dwithin_slots"     64 (default), 0-1024: fused ST_DWithin keeps up to this
  *                       many build ids per probe from its counting pass
  *   "fuse_dwithin"      1 (default) / 0: point-point ST_DWithin decided inside

@@ -12,6 +12,7 @@
 // decided, any other gets the exact correctly rounded hypot test.
 #pragma once
 #include "lbvh.cuh"
+#include "packet.cuh"
 
 namespace spj {
 
@@ -51,7 +52,14 @@ struct DwithinArena {
   uint32_t* head = nullptr;
 };
 
-// d_row (device, one per probe row) replaces d when given.
+// The probes in Morton order (order: n entries), 32 to a traversal: counts[row]
+// and the packets' records in `a`, for packet_scatter.  d_row (device, one per
+// probe row) replaces d when given.
+void dwithin_packet(const LbvhView& t, const PointSplit& bs, const float4* probe_box,
+                    const double2* probe_pt, uint32_t n, double d, const uint32_t* order,
+                    uint32_t* counts, DeviceStatus* st, const PacketStore& a, cudaStream_t s,
+                    const double* d_row = nullptr);
+
 void dwithin_count(const LbvhView& t, const PointSplit& bs, const float4* probe_box,
                    const double2* probe_pt, uint32_t n, double d, const uint32_t* order,
                    uint32_t* counts, DeviceStatus* st, cudaStream_t s, uint32_t* slots = nullptr,

@@ -95,6 +95,14 @@ static inline float ev_ms(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
+// Fused ST_DWithin of probes in Morton order: one traversal per 32 of them,
+// unless the slots or the arena of the traversal per probe were asked for.
+bool JoinEngine::packet_dwithin() const {
+  const EngineConfig auto_cfg;
+  return cfg_.dwithin_slots == auto_cfg.dwithin_slots &&
+         cfg_.dwithin_arena == auto_cfg.dwithin_arena;
+}
+
 // Relation predicates over a build side with rings, in the FP32 form and with
 // the automatic candidate order and refine: the packet kernels, where they
 // take the probe rows (which have to be in Morton order).
@@ -107,8 +115,11 @@ bool JoinEngine::packet_path(int predicate, bool points) const {
          packet_takes(predicate, points);
 }
 
-uint64_t JoinEngine::packet_probe(Workspace& ws, int predicate, uint32_t probe_base,
-                                  const uint32_t* order, DeviceStatus& hst, uint64_t& launches) {
+// The pairs by the packet kernels; false where their records would pass the
+// limits (the candidate pairs' path then answers).
+bool JoinEngine::packet_probe(Workspace& ws, int predicate, double distance, const double* d_row,
+                              const float4* boxes, uint32_t probe_base, const uint32_t* order,
+                              DeviceStatus& hst, uint64_t& launches, uint64_t& total) {
   struct Readback {
     DeviceStatus st;
     uint64_t total, ctrl[4];
@@ -116,7 +127,7 @@ uint64_t JoinEngine::packet_probe(Workspace& ws, int predicate, uint32_t probe_b
   };
   cudaStream_t s = ws.stream;
   const uint32_t n = ws.probe.n;
-  const bool points = ws.probe.all_points;
+  const bool points = ws.probe.all_points, dwithin = predicate == kPredDWithin;
   const LbvhView tv = bvh_.view();
   const GeomsView bv = bg_.view(), pv = ws.probe.view();
   ws.host.reserve(sizeof(Readback));
@@ -125,13 +136,18 @@ uint64_t JoinEngine::packet_probe(Workspace& ws, int predicate, uint32_t probe_b
   ws.psc.offsets.reserve(((size_t)n + 1) * 8, s);
   // first guesses (2M buildings x 50k zones: 2.4 records and 6 open pairs per
   // probe row); a column that needs more tells how much and runs again
-  uint64_t chunks = n / 8 + 1024, queued = points ? 0 : (uint64_t)n * 8 + 1024;
+  uint64_t chunks = std::min<uint64_t>(n / 8 + 1024, kPacketMaxChunks);
+  uint64_t queued = points ? 0 : std::min<uint64_t>((uint64_t)n * 8 + 1024, kPacketMaxQueue);
   for (int attempt = 0;; attempt++) {
     ws.packet.reserve(n, chunks, queued, s);
     const PacketStore a = ws.packet.store(n);
     reset_status(ws.status, s);
-    packet_join(tv, bv, pv, points, order, predicate, ws.psc.counts.as<uint32_t>(), a,
-                ws.status.as<DeviceStatus>(), s);
+    if (dwithin)
+      dwithin_packet(tv, bsplit_, boxes, ws.probe.pt.as<double2>(), n, distance, order,
+                     ws.psc.counts.as<uint32_t>(), ws.status.as<DeviceStatus>(), a, s, d_row);
+    else
+      packet_join(tv, bv, pv, points, order, predicate, ws.psc.counts.as<uint32_t>(), a,
+                  ws.status.as<DeviceStatus>(), s);
     scan_u32_u64(ws.psc.counts.as<uint32_t>(), ws.psc.offsets.as<uint64_t>(), n, ws.psc.tmp, s);
     SPJ_CUDA(cudaMemcpyAsync(&rb->st, ws.status.get(), sizeof rb->st, cudaMemcpyDeviceToHost, s));
     SPJ_CUDA(cudaMemcpyAsync(&rb->total, ws.psc.offsets.as<uint64_t>() + n, 8,
@@ -143,21 +159,25 @@ uint64_t JoinEngine::packet_probe(Workspace& ws, int predicate, uint32_t probe_b
     check_traversal_word(rb->fault);
     if (rb->ctrl[0] <= a.chunks && rb->ctrl[1] <= a.queue_cap) break;
     SPJ_CHECK(attempt < 2, "packet refine: record capacities did not settle");
-    chunks = rb->ctrl[0] + rb->ctrl[0] / 8;
-    queued = rb->ctrl[1] + rb->ctrl[1] / 8;
+    if (rb->ctrl[0] > kPacketMaxChunks || rb->ctrl[1] > kPacketMaxQueue) {
+      ws.packet.release();
+      return false;
+    }
+    chunks = std::min(rb->ctrl[0] + rb->ctrl[0] / 8, kPacketMaxChunks);
+    queued = std::min(rb->ctrl[1] + rb->ctrl[1] / 8, kPacketMaxQueue);
   }
   hst = rb->st;
-  const uint64_t total = rb->total;
-  SPJ_CHECK(hst.counters[1] < (1ull << 34), "candidate pair count too large");
+  total = rb->total;
+  SPJ_CHECK(dwithin || hst.counters[1] < (1ull << 34), "candidate pair count too large");
   if (hst.first_bad != ~0ull)
     throw Error(std::string("refine: ") + status_message((uint32_t)(hst.first_bad >> 40)));
   if (cfg_.profile) SPJ_CUDA(cudaEventRecord(ws.ev[3], s));
   ws.out_build.reserve((total + 1) * 4, s);
   ws.out_probe.reserve((total + 1) * 4, s);
-  packet_scatter(pv, order, ws.psc.offsets.as<uint64_t>(), probe_base, ws.packet.store(n),
+  packet_scatter(n, order, ws.psc.offsets.as<uint64_t>(), probe_base, ws.packet.store(n),
                  ws.out_build.as<uint32_t>(), ws.out_probe.as<uint32_t>(), total, s);
   launches++;
-  return total;
+  return true;
 }
 
 uint64_t JoinEngine::probe(Workspace& ws, const WkbDeviceColumn& col, int predicate,
@@ -196,10 +216,44 @@ uint64_t JoinEngine::probe(Workspace& ws, const WkbDeviceColumn& col, int predic
     order = probe_order(tv, boxes, n, ws.psc, s);
     if (order) launches += 21;  // keys + 4 radix passes (histogram, 3-kernel scan, scatter)
   }
-  if (predicate == kPredDWithin && cfg_.fuse_dwithin && cfg_.refine_form == kFastF32 &&
-      ws.probe.all_points && bsplit_.n == bvh_.nprims && bvh_.nprims > 0) {
-    // point build and probe sides: the distance test runs inside the
-    // traversal, no candidate pairs are materialized
+  // point build and probe sides: the distance test runs inside the
+  // traversal, no candidate pairs are materialized
+  const bool fused = predicate == kPredDWithin && cfg_.fuse_dwithin &&
+                     cfg_.refine_form == kFastF32 && ws.probe.all_points &&
+                     bsplit_.n == bvh_.nprims && bvh_.nprims > 0;
+  auto count = [&](const DeviceStatus& hst, uint64_t total) {
+    std::lock_guard<std::mutex> lk(stats_mu_);
+    stats_.calls++;
+    stats_.probe_rows += n;
+    stats_.candidates += hst.counters[1];
+    stats_.results += total;
+    stats_.escalations += hst.counters[0];
+    stats_.pairs_evaluated += hst.counters[1];
+    stats_.kernel_launches += launches;
+    stats_.probe_bytes +=
+        (uint64_t)col.data_len + (uint64_t)(col.n + 1) * (col.offsets64 ? 8 : 4);
+    if (prof) {
+      stats_.ms_decode += ev_ms(ws.ev[0], ws.ev[1]);
+      stats_.ms_filter += ev_ms(ws.ev[1], ws.ev[2]);
+      stats_.ms_refine += ev_ms(ws.ev[2], ws.ev[3]);
+      stats_.ms_compact += ev_ms(ws.ev[3], ws.ev[4]);
+    }
+    *d_build = ws.out_build.as<uint32_t>();
+    *d_probe = ws.out_probe.as<uint32_t>();
+  };
+  if (order && (fused ? packet_dwithin() : packet_path(predicate, ws.probe.all_points))) {
+    if (prof) SPJ_CUDA(cudaEventRecord(ws.ev[2], s));
+    DeviceStatus hst;
+    uint64_t total = 0;
+    if (packet_probe(ws, predicate, distance, d_row, boxes, probe_base, order, hst, launches,
+                     total)) {
+      if (prof) SPJ_CUDA(cudaEventRecord(ws.ev[4], s));
+      SPJ_CUDA(cudaStreamSynchronize(s));
+      count(hst, total);
+      return total;
+    }
+  }
+  if (fused) {
     reset_status(ws.status, s);
     ws.psc.counts.reserve(((size_t)n + 1) * 4, s);
     ws.psc.offsets.reserve(((size_t)n + 1) * 8, s);
@@ -248,54 +302,7 @@ uint64_t JoinEngine::probe(Workspace& ws, const WkbDeviceColumn& col, int predic
       SPJ_CUDA(cudaEventRecord(ws.ev[4], s));
     }
     SPJ_CUDA(cudaStreamSynchronize(s));
-    {
-      std::lock_guard<std::mutex> lk(stats_mu_);
-      stats_.calls++;
-      stats_.probe_rows += n;
-      stats_.candidates += hst.counters[1];
-      stats_.results += total;
-      stats_.escalations += hst.counters[0];
-      stats_.pairs_evaluated += hst.counters[1];
-      stats_.kernel_launches += launches;
-      stats_.probe_bytes +=
-          (uint64_t)col.data_len + (uint64_t)(col.n + 1) * (col.offsets64 ? 8 : 4);
-      if (prof) {
-        stats_.ms_decode += ev_ms(ws.ev[0], ws.ev[1]);
-        stats_.ms_filter += ev_ms(ws.ev[1], ws.ev[2]);
-        stats_.ms_refine += ev_ms(ws.ev[2], ws.ev[3]);
-        stats_.ms_compact += ev_ms(ws.ev[3], ws.ev[4]);
-      }
-    }
-    *d_build = ws.out_build.as<uint32_t>();
-    *d_probe = ws.out_probe.as<uint32_t>();
-    return total;
-  }
-  if (order && packet_path(predicate, ws.probe.all_points)) {
-    if (prof) SPJ_CUDA(cudaEventRecord(ws.ev[2], s));
-    DeviceStatus hst;
-    const uint64_t total = packet_probe(ws, predicate, probe_base, order, hst, launches);
-    if (prof) SPJ_CUDA(cudaEventRecord(ws.ev[4], s));
-    SPJ_CUDA(cudaStreamSynchronize(s));
-    {
-      std::lock_guard<std::mutex> lk(stats_mu_);
-      stats_.calls++;
-      stats_.probe_rows += n;
-      stats_.candidates += hst.counters[1];
-      stats_.results += total;
-      stats_.escalations += hst.counters[0];
-      stats_.pairs_evaluated += hst.counters[1];
-      stats_.kernel_launches += launches;
-      stats_.probe_bytes +=
-          (uint64_t)col.data_len + (uint64_t)(col.n + 1) * (col.offsets64 ? 8 : 4);
-      if (prof) {
-        stats_.ms_decode += ev_ms(ws.ev[0], ws.ev[1]);
-        stats_.ms_filter += ev_ms(ws.ev[1], ws.ev[2]);
-        stats_.ms_refine += ev_ms(ws.ev[2], ws.ev[3]);
-        stats_.ms_compact += ev_ms(ws.ev[3], ws.ev[4]);
-      }
-    }
-    *d_build = ws.out_build.as<uint32_t>();
-    *d_probe = ws.out_probe.as<uint32_t>();
+    count(hst, total);
     return total;
   }
   const uint64_t m = probe_count(tv, boxes, n, ws.psc, s, order);  // syncs

@@ -169,14 +169,16 @@ class JoinEngine {
 
   // Whether probes in Morton order take the packet kernels (packet.cuh).
   bool packet_path(int predicate, bool points) const;
+  bool packet_dwithin() const;
 
   JoinStats stats();
   void reset_stats();
 
  private:
   void split_points();
-  uint64_t packet_probe(Workspace& ws, int predicate, uint32_t probe_base, const uint32_t* order,
-                        DeviceStatus& hst, uint64_t& launches);
+  bool packet_probe(Workspace& ws, int predicate, double distance, const double* d_row,
+                    const float4* boxes, uint32_t probe_base, const uint32_t* order,
+                    DeviceStatus& hst, uint64_t& launches, uint64_t& total);
   int device_;
   EngineConfig cfg_;
   DeviceGeoms bg_;

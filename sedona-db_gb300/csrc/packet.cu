@@ -44,7 +44,6 @@ using namespace pred;
 
 constexpr int kPacketThreads = 128;
 constexpr unsigned kAll = 0xffffffffu;
-constexpr uint32_t kNoChunk = 0xffffffffu;
 // flags of a queued pair above its lane
 constexpr uint32_t kOpenNear = 32;  // two single rings, an edge near the probe's box
 
@@ -367,12 +366,15 @@ __device__ __forceinline__ bool isolated_result(int predicate, bool in) {
 // Packets: runs of up to 32 consecutive rows of the Morton order.  A run whose
 // box is wide would meet many more build rows than its rows do (a cluster's
 // thin tail, a gap of the order) and one warp would still be at it when the
-// others are done, so it is cut in halves, down to 4 rows: each aligned group
-// of lanes whose box may meet more than `most` build rows (by their mean size
-// and density over the tree's box) is split.
+// others are done, so it is cut in halves, down to 4 rows: an aligned group of
+// rows is split where its box, widened by the mean build box, is over
+// kPacketGrowth times one row's and may meet over kPacketRows build rows (by
+// their mean density over the tree; with fewer, splitting costs more than it
+// saves).
+constexpr float kPacketRows = 64.0f, kPacketGrowth = 4.0f;
 __global__ void __launch_bounds__(256)
     k_packets(LbvhView t, const float4* __restrict__ box, const uint32_t* __restrict__ order,
-              uint32_t n, float mean_w, float mean_h, float per_area, float most,
+              uint32_t n, float mean_w, float mean_h, float per_area,
               uint2* __restrict__ packets, unsigned long long* __restrict__ ctrl) {
   const int lane = threadIdx.x & 31;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -385,6 +387,7 @@ __global__ void __launch_bounds__(256)
     const bool live = b.x <= b.z && b.y <= b.w;
     float x0 = live ? b.x : INFINITY, y0 = live ? b.y : INFINITY;
     float x1 = live ? b.z : -INFINITY, y1 = live ? b.w : -INFINITY;
+    float own = live ? (b.z - b.x + mean_w) * (b.w - b.y + mean_h) : 0.0f;
     int size = 1;  // of the group taken so far
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -392,9 +395,13 @@ __global__ void __launch_bounds__(256)
       y0 = fminf(y0, __shfl_xor_sync(kAll, y0, o));
       x1 = fmaxf(x1, __shfl_xor_sync(kAll, x1, o));
       y1 = fmaxf(y1, __shfl_xor_sync(kAll, y1, o));
+      own = fmaxf(own, __shfl_xor_sync(kAll, own, o));
       const float w = fmaxf(x1 - x0, 0.0f) + mean_w, h = fmaxf(y1 - y0, 0.0f) + mean_h;
-      // (a wide group's union is wide too; NaN and overflow count as wide)
-      if (size == o && (o < 4 || w * h * per_area <= most)) size = 2 * o;
+      // (both halves whole; an overflow to NaN counts as wide)
+      const int other = __shfl_xor_sync(kAll, size, o);
+      const bool whole = size == o && other == o;
+      if (whole && (o < 4 || w * h * per_area <= kPacketRows || w * h <= kPacketGrowth * own))
+        size = 2 * o;
     }
     const bool leader = (lane & (size - 1)) == 0 && j < n;
     const unsigned lead = __ballot_sync(kAll, leader);
@@ -404,10 +411,6 @@ __global__ void __launch_bounds__(256)
     if (leader) packets[at] = make_uint2((uint32_t)j, min((uint32_t)size, n - (uint32_t)j));
   }
 }
-
-// (the mean number that one row meets, kPacketGrowth times over, and a floor
-// below which splitting costs more than the long packet)
-constexpr float kPacketRows = 64.0f, kPacketGrowth = 3.0f;
 
 // What a packet holds of the 32 build rows it works on next (lane u: row u).
 struct PacketRow {
@@ -663,23 +666,8 @@ __global__ void __launch_bounds__(kPacketThreads, kPoints ? 8 : 6)
       // records of the rows with something to say, in order
       const unsigned say = __ballot_sync(kAll, (me.hits | me.opens) != 0);
       if (say == 0) continue;
-      const uint32_t nsay = (uint32_t)__popc(say);
-      const uint32_t room = (32u - (nrec & 31u)) & 31u;  // in the current chunk
-      uint32_t fresh = kNoChunk;
-      if (nsay > room) {
-        if (lane == 0) {
-          fresh = (uint32_t)min(atomicAdd(&A.ctrl[0], 1ull), (unsigned long long)kNoChunk);
-          if (nrec == 0) A.head[g] = fresh;
-          else if (chunk < A.chunks) A.next[chunk] = fresh;
-        }
-        fresh = __shfl_sync(kAll, fresh, 0);
-      }
-      const uint32_t rank = (uint32_t)__popc(say & lower);
-      const uint32_t into = rank < room ? chunk : fresh;
-      const uint32_t at = into * 32u + ((nrec + rank) & 31u);
-      if (((say >> lane) & 1u) && into < A.chunks) A.rec[at] = make_uint2(me.b, me.hits);
-      nrec += nsay;
-      if (nsay > room) chunk = fresh;
+      const uint32_t at = packet_append(A, g, lane, (say >> lane) & 1u, make_uint2(me.b, me.hits),
+                                        nrec, chunk);
       for (unsigned s = say; s;) {
         const int u = __ffs(s) - 1;
         s &= s - 1;
@@ -1035,7 +1023,8 @@ void PacketBufs::reserve(uint32_t n, uint64_t chunks, uint64_t queued, cudaStrea
   const uint64_t most = most_packets(n);
   chunk_cap = std::max(chunk_cap, chunks);
   queue_cap = std::max(queue_cap, queued);
-  SPJ_CHECK(chunk_cap < (1ull << 27) && queue_cap < 0xFFFFFFFFull, "packet records exceed 32 bits");
+  SPJ_CHECK(chunk_cap <= kPacketMaxChunks && queue_cap <= kPacketMaxQueue,
+            "packet records exceed their limit");
   rec.reserve(chunk_cap * 32 * sizeof(uint2), s);
   next.reserve(chunk_cap * 4, s);
   queue.reserve((queue_cap + 1) * sizeof(uint4), s);
@@ -1068,17 +1057,21 @@ bool packet_takes(int predicate, bool points) {
          predicate == kDisjoint;
 }
 
+void packet_runs(const LbvhView& t, const float4* box, const uint32_t* order, uint32_t n,
+                 const PacketStore& a, cudaStream_t s) {
+  SPJ_CUDA(cudaMemsetAsync(a.ctrl, 0, kPacketCtrlBytes, s));
+  if (n == 0) return;
+  const float per_area = t.extent_area > 0.0f ? (float)t.nprims / t.extent_area : 0.0f;
+  k_packets<<<grid_for(n, 256, kNumSMs * 8), 256, 0, s>>>(t, box, order, n, t.mean_w, t.mean_h,
+                                                          per_area, a.packets, a.ctrl);
+  SPJ_CUDA(cudaGetLastError());
+}
+
 void packet_join(const LbvhView& t, const GeomsView& build, const GeomsView& probe, bool points,
                  const uint32_t* order, int predicate, uint32_t* counts, const PacketStore& a,
                  DeviceStatus* st, cudaStream_t s) {
-  SPJ_CUDA(cudaMemsetAsync(a.ctrl, 0, kPacketCtrlBytes, s));
+  packet_runs(t, probe.box, order, probe.n, a, s);
   if (probe.n == 0) return;
-  // build rows that a box of no size meets on average, and how many a
-  // packet's box may
-  const float per_area = t.extent_area > 0.0f ? (float)t.nprims / t.extent_area : 0.0f;
-  const float most = kPacketRows + kPacketGrowth * t.mean_w * t.mean_h * per_area;
-  k_packets<<<grid_for(probe.n, 256, kNumSMs * 8), 256, 0, s>>>(
-      t, probe.box, order, probe.n, t.mean_w, t.mean_h, per_area, most, a.packets, a.ctrl);
   const int g = grid_for(probe.n, kPacketThreads, kNumSMs * 8);
   if (points) {
     k_packet<true><<<g, kPacketThreads, 0, s>>>(t, build, probe, order, predicate, counts, a, st);
@@ -1089,12 +1082,12 @@ void packet_join(const LbvhView& t, const GeomsView& build, const GeomsView& pro
   SPJ_CUDA(cudaGetLastError());
 }
 
-void packet_scatter(const GeomsView& probe, const uint32_t* order, const uint64_t* offs,
-                    uint32_t probe_base, const PacketStore& a, uint32_t* out_build,
+void packet_scatter(uint32_t n, const uint32_t* order, const uint64_t* offs, uint32_t probe_base,
+                    const PacketStore& a, uint32_t* out_build,
                     uint32_t* out_probe, uint64_t cap, cudaStream_t s) {
-  if (probe.n == 0) return;
-  k_packet_scatter<<<grid_for(probe.n, 256, kNumSMs * 16), 256, 0, s>>>(
-      probe.n, order, offs, probe_base, a, out_build, out_probe, cap);
+  if (n == 0) return;
+  k_packet_scatter<<<grid_for(n, 256, kNumSMs * 16), 256, 0, s>>>(
+      n, order, offs, probe_base, a, out_build, out_probe, cap);
   SPJ_CUDA(cudaGetLastError());
 }
 

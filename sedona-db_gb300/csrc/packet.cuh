@@ -26,6 +26,42 @@ struct PacketStore {
 };
 constexpr size_t kPacketCtrlBytes = 4 * sizeof(unsigned long long);
 
+// Adds the records of the lanes with `say` (in lane order) to packet g's list
+// (nrec records so far, the last of them in `chunk`); all 32 lanes call.
+// Returns where the lane's record lies, written only within the store's room.
+constexpr uint32_t kNoChunk = 0xffffffffu;
+#ifdef __CUDACC__
+__device__ __forceinline__ uint32_t packet_append(const PacketStore& A, uint32_t g, int lane,
+                                                  bool say, uint2 rec, uint32_t& nrec,
+                                                  uint32_t& chunk) {
+  const unsigned all = 0xffffffffu;
+  const unsigned who = __ballot_sync(all, say);
+  const uint32_t n = (uint32_t)__popc(who);
+  if (n == 0) return 0;
+  const uint32_t room = (32u - (nrec & 31u)) & 31u;  // in the current chunk
+  uint32_t fresh = kNoChunk;
+  if (n > room) {
+    if (lane == 0) {
+      fresh = (uint32_t)min(atomicAdd(&A.ctrl[0], 1ull), (unsigned long long)kNoChunk);
+      if (nrec == 0) A.head[g] = fresh;
+      else if (chunk < A.chunks) A.next[chunk] = fresh;
+    }
+    fresh = __shfl_sync(all, fresh, 0);
+  }
+  const uint32_t rank = (uint32_t)__popc(who & ((1u << lane) - 1u));
+  const uint32_t into = rank < room ? chunk : fresh;
+  const uint32_t at = into * 32u + ((nrec + rank) & 31u);
+  if (say && into < A.chunks) A.rec[at] = rec;
+  nrec += n;
+  if (n > room) chunk = fresh;
+  return at;
+}
+#endif
+
+// Most chunks and queued pairs a join keeps (16 GB each); one that needs more
+// takes the candidate pairs' path, which has no records.
+constexpr uint64_t kPacketMaxChunks = 1ull << 26, kPacketMaxQueue = 1ull << 30;
+
 struct PacketBufs {
   DevBuf rec, next, heads, queue, ctrl;
   uint64_t chunk_cap = 0, queue_cap = 0;
@@ -46,9 +82,14 @@ void packet_join(const LbvhView& t, const GeomsView& build, const GeomsView& pro
                  const uint32_t* order, int predicate, uint32_t* counts, const PacketStore& a,
                  DeviceStatus* st, cudaStream_t s);
 
-// The pairs, grouped by probe row in ascending order (offs: exclusive scan of
-// counts), writes bounded by cap.
-void packet_scatter(const GeomsView& probe, const uint32_t* order, const uint64_t* offs,
+// Cuts the n probe rows' Morton order into packets (a.packets, a.ctrl[3]) and
+// clears a's counts.
+void packet_runs(const LbvhView& t, const float4* box, const uint32_t* order, uint32_t n,
+                 const PacketStore& a, cudaStream_t s);
+
+// The pairs of the n probe rows, grouped by probe row in ascending order (offs:
+// exclusive scan of counts), writes bounded by cap.
+void packet_scatter(uint32_t n, const uint32_t* order, const uint64_t* offs,
                     uint32_t probe_base, const PacketStore& a, uint32_t* out_build,
                     uint32_t* out_probe, uint64_t cap, cudaStream_t s);
 

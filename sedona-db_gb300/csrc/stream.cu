@@ -175,7 +175,8 @@ void StreamJoin::set_batches(const std::vector<WkbDeviceColumn>& cols) {
     ccap_ = (uint64_t)nrows_ * 8 + 1024;
     ocap_ = (uint64_t)nrows_ * 4 + 1024;
   }
-  chunks_cap_ = std::max<uint64_t>(chunks_cap_, nrows_ / 8 + 1024);
+  chunks_cap_ = std::max(chunks_cap_, std::min<uint64_t>(nrows_ / 8 + 1024, kPacketMaxChunks));
+  packet_off_ = false;
   SPJ_CUDA(cudaStreamSynchronize(s_));
   std::ostringstream sig;
   sig << eng_.build_geoms().n << "x" << eng_.build_geoms().nverts << "|" << nrows_ << "|"
@@ -199,7 +200,7 @@ void StreamJoin::build_graph(int predicate) {
   // neighbouring probes together); everything the ordering uses is reserved
   // here, so the capture allocates nothing
   const bool want = cfg.probe_order > 0 || (cfg.probe_order == 0 && nrows_ >= kOrderMinRows);
-  graph_packet_ = want && nrows_ >= 2 && eng_.packet_path(predicate, true);
+  graph_packet_ = want && nrows_ >= 2 && !packet_off_ && eng_.packet_path(predicate, true);
   const bool ordered = want && (graph_packet_ || ccap_ < 0xFFFFFFFFull);
   // capacity-sized buffers
   if (graph_packet_) {
@@ -246,7 +247,7 @@ void StreamJoin::build_graph(int predicate) {
     packet_join(t, B, P, true, order, predicate, counts_.as<uint32_t>(), a, st, s_);
     scan_u32_u64_into(counts_.as<uint32_t>(), offs_.as<uint64_t>(), nrows_, sums_.as<uint64_t>(),
                       s_);
-    packet_scatter(P, order, offs_.as<uint64_t>(), 0, a, out_b_.as<uint32_t>(),
+    packet_scatter(nrows_, order, offs_.as<uint64_t>(), 0, a, out_b_.as<uint32_t>(),
                    out_p_.as<uint32_t>(), ocap_, s_);
     SPJ_CUDA(cudaMemcpyAsync(h_tot_, &st->counters[1], 8, cudaMemcpyDeviceToHost, s_));
     SPJ_CUDA(cudaMemcpyAsync(h_tot_ + 1, d_m, 8, cudaMemcpyDeviceToHost, s_));
@@ -293,7 +294,7 @@ uint64_t StreamJoin::run(int predicate, const uint32_t** d_build, const uint32_t
   SPJ_CHECK(eng_.built(), "stream run before the build side was finished");
   SPJ_CHECK(predicate >= 0 && predicate <= 7, "the stream path takes relation predicates");
   uint64_t m = 0, total = 0;
-  for (int attempt = 0; attempt < 4; attempt++) {
+  for (int attempt = 0; attempt < 6; attempt++) {
     if (!exec_ || graph_pred_ != predicate) build_graph(predicate);
     SPJ_CUDA(cudaEventRecord(ev0_, s_));
     SPJ_CUDA(cudaGraphLaunch(exec_, s_));
@@ -303,8 +304,14 @@ uint64_t StreamJoin::run(int predicate, const uint32_t** d_build, const uint32_t
     m = h_tot_[0];
     total = h_tot_[1];
     if (graph_packet_ && h_tot_[4] > chunks_cap_) {
-      // the packets' records did not fit: grow, re-capture, replay
-      chunks_cap_ = h_tot_[4] + h_tot_[4] / 8;
+      // the packets' records did not fit: grow, re-capture, replay (past the
+      // limit: with the candidate pairs)
+      if (h_tot_[4] > kPacketMaxChunks) {
+        packet_off_ = true;
+        packet_.release();
+      } else {
+        chunks_cap_ = std::min(h_tot_[4] + h_tot_[4] / 8, kPacketMaxChunks);
+      }
       destroy_graph();
       continue;
     }
@@ -327,7 +334,7 @@ uint64_t StreamJoin::run(int predicate, const uint32_t** d_build, const uint32_t
       // the records are complete: only the pairs are written again
       out_b_.reserve((ocap_ + 1) * 4, s_);
       out_p_.reserve((ocap_ + 1) * 4, s_);
-      packet_scatter(probe_view(), psc_.order.as<uint32_t>(), offs_.as<uint64_t>(), 0,
+      packet_scatter(nrows_, psc_.order.as<uint32_t>(), offs_.as<uint64_t>(), 0,
                      packet_.store(nrows_), out_b_.as<uint32_t>(), out_p_.as<uint32_t>(), ocap_,
                      s_);
       SPJ_CUDA(cudaStreamSynchronize(s_));

@@ -77,7 +77,8 @@ class StreamJoin {
   // pinned: candidates, pairs, status, escalations, packet chunks
   uint64_t* h_tot_ = nullptr;
   uint64_t ccap_ = 0, ocap_ = 0, chunks_cap_ = 0;
-  bool graph_packet_ = false;
+  bool graph_packet_ = false;  // the graph holds the packet kernels
+  bool packet_off_ = false;    // these batches pass the packets' limits
   uint32_t nrows_ = 0, nchunks_ = 0, nbatches_ = 0;
   std::vector<WkbDeviceColumn> cols_;
   cudaGraphExec_t exec_ = nullptr;

@@ -135,3 +135,39 @@ def test_packet_capacities_grow(capi):
                               [_star(rng, rng.uniform(-40, 40, 2), 5, 3.0)]]) for _ in range(40)])
     for _ in _both(capi, build, multi, ["intersects", "contains"]):
         pass
+
+
+@pytest.mark.parametrize("n,leaf", [(2, 16), (31, 1), (32, 16), (33, 64), (127, 33), (2500, 16)])
+def test_packet_dwithin_same_pairs_and_positions(capi, n, leaf):
+    """ST_DWithin of points by the packet traversal against the traversal per
+    probe: pairs exactly at d, rows with no box, points and distances outside
+    the FP32 test's range, more records than the first guess holds."""
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(n)
+
+    def points(m):
+        xy = np.concatenate([rng.integers(0, 40, (m // 2, 2)).astype(np.float64),
+                             rng.normal(20, 8, (m - m // 2, 2))])
+        vals = [wkb.wkb_point(*v) for v in xy]
+        for i, v in enumerate([None, wkb.wkb_point(1e30, 3.0), wkb.wkb_point(np.nan, np.nan),
+                               wkb.wkb_point(1e-40, -1e-40)]):
+            if m > 30:
+                vals[i * 7] = v
+        return vals
+
+    near = [wkb.wkb_point(*v) for v in rng.integers(0, 40, (3000, 2)).astype(np.float64)]
+    for vals in (near, points(3000)):  # (without and with the exact test for every pair)
+        build, probe = wkb.column_from_values(vals), wkb.column_from_values(points(n))
+        js = [capi.SpatialJoin(probe_order=1, leaf_size=leaf) for _ in range(2)]
+        js[1].set_option("dwithin_arena", 0)  # (any set arena takes the traversal per probe)
+        for j in js:
+            j.build(build)
+        rows = rng.choice([0.0, 1.0, 5.0, 100.0, np.inf, np.nan, -1.0, 1e-30], n)
+        for d in (0.0, 5.0, np.nextafter(5.0, 0), 1e-40, 60.0, 1e200, np.inf, rows):
+            got = []
+            for j in js:
+                if d is rows:
+                    j.set_probe_distances(rows)
+                got.append(j.probe(probe, "dwithin", distance=0.0 if d is rows else d))
+            np.testing.assert_array_equal(got[0][0], got[1][0])
+            np.testing.assert_array_equal(got[0][1], got[1][1])
