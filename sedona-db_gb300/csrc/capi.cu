@@ -470,12 +470,13 @@ int ref_refine(SedonaSpatialRefiner* self, const ArrowSchema* probe_schema,
     // include/gpuspatial/refine/rt_spatial_refiner.hpp:48); the sort is
     // stable, so pairs of one probe keep their input order
     if (kept > 1) {
-      DevBuf ak(kept * 4, s), av(kept * 4, s), tmp;
+      ws->psc.akeys.reserve(kept * 4, s);
+      ws->psc.avals.reserve(kept * 4, s);
       int bits = 1;
       while (bits < 32 && ((uint64_t)pc.n >> bits) != 0) bits++;
       radix_sort_pairs(ws->out_probe.as<uint32_t>(), ws->out_build.as<uint32_t>(),
-                       ak.as<uint32_t>(), av.as<uint32_t>(), (int64_t)kept, (bits + 7) / 8 * 8,
-                       tmp, s);
+                       ws->psc.akeys.as<uint32_t>(), ws->psc.avals.as<uint32_t>(), (int64_t)kept,
+                       (bits + 7) / 8 * 8, ws->psc.tmp, s);
     }
     if (kept) {
       SPJ_CUDA(cudaMemcpyAsync(build_indices, ws->out_build.get(), kept * 4,

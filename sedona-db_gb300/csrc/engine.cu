@@ -13,6 +13,9 @@ Workspace::Workspace() {
   SPJ_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   own_stream = true;
   for (auto& e : ev) SPJ_CUDA(cudaEventCreate(&e));
+  host.reserve(sizeof(Readback));
+  dsc.host = &back()->decode;
+  psc.host = back()->filter;
 }
 
 Workspace::~Workspace() {
@@ -120,18 +123,12 @@ bool JoinEngine::packet_path(int predicate, bool points) const {
 bool JoinEngine::packet_probe(Workspace& ws, int predicate, double distance, const double* d_row,
                               const float4* boxes, uint32_t probe_base, const uint32_t* order,
                               DeviceStatus& hst, uint64_t& launches, uint64_t& total) {
-  struct Readback {
-    DeviceStatus st;
-    uint64_t total, ctrl[4];
-    unsigned fault[2];
-  };
   cudaStream_t s = ws.stream;
   const uint32_t n = ws.probe.n;
   const bool points = ws.probe.all_points, dwithin = predicate == kPredDWithin;
   const LbvhView tv = bvh_.view();
   const GeomsView bv = bg_.view(), pv = ws.probe.view();
-  ws.host.reserve(sizeof(Readback));
-  Readback* rb = ws.host.as<Readback>();
+  Workspace::Readback* rb = ws.back();
   ws.psc.counts.reserve(((size_t)n + 1) * 4, s);
   ws.psc.offsets.reserve(((size_t)n + 1) * 8, s);
   // first guesses (2M buildings x 50k zones: 2.4 records and 6 open pairs per
@@ -283,13 +280,15 @@ uint64_t JoinEngine::probe(Workspace& ws, const WkbDeviceColumn& col, int predic
     dwithin_count(tv, bsplit_, boxes, ppt, n, distance, order, ws.psc.counts.as<uint32_t>(),
                   ws.status.as<DeviceStatus>(), s, slots, K, arena, d_row);
     scan_u32_u64(ws.psc.counts.as<uint32_t>(), ws.psc.offsets.as<uint64_t>(), n, ws.psc.tmp, s);
-    uint64_t total = 0;
-    DeviceStatus hst;
-    SPJ_CUDA(cudaMemcpyAsync(&total, ws.psc.offsets.as<uint64_t>() + n, 8,
+    Workspace::Readback* rb = ws.back();
+    SPJ_CUDA(cudaMemcpyAsync(&rb->total, ws.psc.offsets.as<uint64_t>() + n, 8,
                              cudaMemcpyDeviceToHost, s));
-    SPJ_CUDA(cudaMemcpyAsync(&hst, ws.status.get(), sizeof hst, cudaMemcpyDeviceToHost, s));
+    SPJ_CUDA(cudaMemcpyAsync(&rb->st, ws.status.get(), sizeof rb->st, cudaMemcpyDeviceToHost, s));
+    SPJ_CUDA(cudaMemcpyAsync(rb->fault, tv.fault, 8, cudaMemcpyDeviceToHost, s));
     SPJ_CUDA(cudaStreamSynchronize(s));
-    check_traversal(tv, s);
+    check_traversal_word(rb->fault);
+    const uint64_t total = rb->total;
+    const DeviceStatus hst = rb->st;
     if (prof) SPJ_CUDA(cudaEventRecord(ws.ev[2], s));
     ws.out_build.reserve((total + 1) * 4, s);
     ws.out_probe.reserve((total + 1) * 4, s);
@@ -364,12 +363,13 @@ uint64_t JoinEngine::probe(Workspace& ws, const WkbDeviceColumn& col, int predic
   ws.scan_tmp.reserve(compact_sums_bytes((int64_t)m), s);
   uint64_t* sums = ws.scan_tmp.as<uint64_t>();
   compact_count(ws.flags.as<uint8_t>(), (int64_t)m, sums, s);
-  uint64_t total = 0;
-  DeviceStatus hst;
-  SPJ_CUDA(cudaMemcpyAsync(&total, sums + compact_tiles((int64_t)m), 8, cudaMemcpyDeviceToHost,
-                           s));
-  SPJ_CUDA(cudaMemcpyAsync(&hst, ws.status.get(), sizeof hst, cudaMemcpyDeviceToHost, s));
+  Workspace::Readback* rb = ws.back();
+  SPJ_CUDA(cudaMemcpyAsync(&rb->total, sums + compact_tiles((int64_t)m), 8,
+                           cudaMemcpyDeviceToHost, s));
+  SPJ_CUDA(cudaMemcpyAsync(&rb->st, ws.status.get(), sizeof rb->st, cudaMemcpyDeviceToHost, s));
   SPJ_CUDA(cudaStreamSynchronize(s));
+  const uint64_t total = rb->total;
+  const DeviceStatus hst = rb->st;
   if (hst.first_bad != ~0ull) {
     throw Error(std::string("refine: ") + status_message((uint32_t)(hst.first_bad >> 40)));
   }
@@ -421,12 +421,13 @@ uint64_t JoinEngine::refine_pairs(Workspace& ws, const GeomsView& pv, const uint
   ws.scan_tmp.reserve(compact_sums_bytes((int64_t)m), s);
   uint64_t* sums = ws.scan_tmp.as<uint64_t>();
   compact_count(ws.flags.as<uint8_t>(), (int64_t)m, sums, s);
-  uint64_t total = 0;
-  DeviceStatus hst;
-  SPJ_CUDA(cudaMemcpyAsync(&total, sums + compact_tiles((int64_t)m), 8, cudaMemcpyDeviceToHost,
-                           s));
-  SPJ_CUDA(cudaMemcpyAsync(&hst, ws.status.get(), sizeof hst, cudaMemcpyDeviceToHost, s));
+  Workspace::Readback* rb = ws.back();
+  SPJ_CUDA(cudaMemcpyAsync(&rb->total, sums + compact_tiles((int64_t)m), 8,
+                           cudaMemcpyDeviceToHost, s));
+  SPJ_CUDA(cudaMemcpyAsync(&rb->st, ws.status.get(), sizeof rb->st, cudaMemcpyDeviceToHost, s));
   SPJ_CUDA(cudaStreamSynchronize(s));
+  const uint64_t total = rb->total;
+  const DeviceStatus hst = rb->st;
   if (hst.first_bad != ~0ull)
     throw Error(std::string("refine: ") + status_message((uint32_t)(hst.first_bad >> 40)));
   ws.out_build.reserve((total + 1) * 4, s);

@@ -127,7 +127,17 @@ struct Workspace {
   DevBuf rqueue;  // pairs left open by the refine's cheap pass, then its count
   DevBuf wkb_data, wkb_offsets, wkb_validity;  // H2D staging of host columns
   PacketBufs packet;  // records and open pairs of the packet refine
-  PinnedBuf host;     // counts and status read back by a probe
+  // pinned words that a probe reads back: the decode's status, the filter's
+  // counts, the refine's status and counts
+  struct Readback {
+    DeviceStatus decode;
+    uint64_t filter[2];
+    DeviceStatus st;
+    uint64_t total, ctrl[4];
+    unsigned fault[2];
+  };
+  PinnedBuf host;
+  Readback* back() const { return host.as<Readback>(); }
   cudaEvent_t ev[6] = {};
   bool last_probe_points = true;
   Workspace();

@@ -165,6 +165,9 @@ struct WkbDeviceColumn {
 
 struct DecodeScratch {
   DevBuf counts, scans, ring_src, tmp, status;
+  // pinned room for a DeviceStatus, where the owner has some (a copy to
+  // pageable memory holds the host up and costs it 10 us)
+  void* host = nullptr;
 };
 
 // Decode a device WKB column into `out`.  points_hint: the caller expects a
@@ -188,6 +191,7 @@ void build_cell_grid(DeviceGeoms& g, DecodeScratch& scratch, cudaStream_t s);
 
 // Reads the device status word; throws with a message if a kernel failed.
 void check_status(DevBuf& status, cudaStream_t s, const char* what);
+void check_status(const DeviceStatus& st, const char* what);
 void reset_status(DevBuf& status, cudaStream_t s);
 
 }  // namespace spj

@@ -724,11 +724,15 @@ uint64_t probe_count(const LbvhView& t, const float4* probe_box, uint32_t nprobe
   k_probe<false><<<g, kTravThreads, 0, s>>>(t, probe_box, nprobe, sc.counts.as<uint32_t>(),
                                             nullptr, 0, nullptr, nullptr, ~0ull, order);
   scan_u32_u64(sc.counts.as<uint32_t>(), sc.offsets.as<uint64_t>(), nprobe, sc.tmp, s);
-  uint64_t total = 0;
-  SPJ_CUDA(cudaMemcpyAsync(&total, sc.offsets.as<uint64_t>() + nprobe, 8, cudaMemcpyDeviceToHost,
-                           s));
+  uint64_t own[2], *h = sc.host ? sc.host : own;
+  h[1] = 0;
+  SPJ_CUDA(cudaMemcpyAsync(h, sc.offsets.as<uint64_t>() + nprobe, 8, cudaMemcpyDeviceToHost, s));
+  if (t.fault) SPJ_CUDA(cudaMemcpyAsync(h + 1, t.fault, 8, cudaMemcpyDeviceToHost, s));
   SPJ_CUDA(cudaStreamSynchronize(s));
-  check_traversal(t, s);
+  const uint64_t total = h[0];
+  unsigned fault[2];
+  memcpy(fault, h + 1, 8);
+  check_traversal_word(fault);
   return total;
 }
 

@@ -137,6 +137,7 @@ struct ProbeScratch {
   DevBuf order, okeys, akeys, avals;  // probe_order
   DevBuf ocount, opos, cperm;         // candidate_order
   DevBuf ckeys, ckeys_alt, cvals_alt, rank;  // build_major_order
+  uint64_t* host = nullptr;  // pinned room for 2 words, where the owner has some
 };
 // Throws if a traversal over t recorded an out-of-range index (syncs s).
 void check_traversal(const LbvhView& t, cudaStream_t s);

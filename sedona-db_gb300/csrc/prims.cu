@@ -3,11 +3,12 @@
 // Scan: reduce-then-scan over 4096-element tiles (256 threads x 16 items);
 // the tile sums are scanned by one 1024-thread block that walks them in
 // chunks, then each tile is rescanned with its prefix.  Two reads of the
-// input plus one write of the output: the scan is HBM-bound.
+// input plus one write of the output: the scan is HBM-bound.  Up to 16,384
+// elements one block does it all (below).
 //
 // Radix sort: per 8-bit digit, (1) a per-tile 256-bin histogram, (2) a scan of
 // the digit-major histogram table, (3) a stable block-local ranking of the
-// tile by digit (warp match + per-warp digit counters), a reorder in shared
+// tile by digit (ballots and per-warp digit counters), a reorder in shared
 // memory, then a scatter whose runs of equal digits land on consecutive
 // addresses.  With segments, the table is segment-major, so the same passes
 // sort each segment of consecutive tiles in place.
@@ -26,26 +27,42 @@ constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;
 static_assert(kScanTile == 4096, "compact_tiles (prims.cuh) counts tiles of 4096 flags");
 
+// Several arrays of one length are scanned by the same launches: array y
+// (blockIdx.y) lies y * in_step / y * out_step elements on, its tile sums
+// y * sums_step on, and totals (where given) gets its total at [y].
 template <class Tin, class Tout>
-__global__ void k_tile_reduce(const Tin* __restrict__ in, int64_t n, Tout* __restrict__ sums) {
+struct ScanArgs {
+  const Tin* in;
+  Tout* out;
+  Tout* sums;
+  Tout* totals;
+  int64_t n, in_step, out_step, sums_step;
+};
+
+template <class Tin, class Tout>
+__global__ void k_tile_reduce(ScanArgs<Tin, Tout> a) {
   __shared__ Tout sm[9];
+  const Tin* in = a.in + blockIdx.y * a.in_step;
   const int64_t base = (int64_t)blockIdx.x * kScanTile;
   Tout acc = 0;
 #pragma unroll
   for (int j = 0; j < kScanItems; j++) {
     int64_t i = base + j * kScanThreads + threadIdx.x;
-    if (i < n) acc += (Tout)in[i];
+    if (i < a.n) acc += (Tout)in[i];
   }
   Tout total;
   block_exclusive_scan_256<Tout>(acc, sm, &total);
-  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+  if (threadIdx.x == 0) a.sums[blockIdx.y * a.sums_step + blockIdx.x] = total;
 }
 
+// One block of 1024 threads per array scans its nt tile sums in place
+// (exclusive); total_out + y * out_step and totals[y] get the total.
 template <class T>
-__global__ void k_scan_sums(T* __restrict__ sums, int64_t nt, T* __restrict__ total_out) {
-  // one block of 1024 threads scans all tile sums in place (exclusive)
+__global__ void k_scan_sums(T* __restrict__ sums, int64_t nt, T* __restrict__ total_out,
+                            int64_t sums_step, int64_t out_step, T* __restrict__ totals) {
   __shared__ T warp_tot[32];
   __shared__ T carry;
+  sums += blockIdx.y * sums_step;
   if (threadIdx.x == 0) carry = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -67,30 +84,91 @@ __global__ void k_scan_sums(T* __restrict__ sums, int64_t nt, T* __restrict__ to
     if (threadIdx.x == blockDim.x - 1) carry = ex + v;
     __syncthreads();
   }
-  if (threadIdx.x == 0) *total_out = carry;
+  if (threadIdx.x == 0) {
+    total_out[blockIdx.y * out_step] = carry;
+    if (totals) totals[blockIdx.y] = carry;
+  }
+}
+
+// The exclusive prefixes within a warp's 32 * kItems elements (lane l of round
+// j: element 32 j + l), in place; returns their sum.
+template <class T, int kItems>
+__device__ __forceinline__ T scan_rounds(T* v) {
+  T run = 0;
+#pragma unroll
+  for (int j = 0; j < kItems; j++) {
+    const T inc = warp_inclusive_scan(v[j]);
+    v[j] = run + inc - v[j];
+    run += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  return run;
+}
+
+// Scans one tile of 32 * kItems elements per warp from `base` on; a warp's
+// elements are consecutive and its loads and stores coalesced.  (With 16
+// consecutive elements per thread each store touched 32 sectors: 4M counts
+// 27 us, 9.4 this way.)  The shuffles bound a block of 32 warps (one a clock
+// per SM), so sums that fit are added in 32 bits.
+template <class Tin, class Tout, int kWarps, int kItems>
+__device__ __forceinline__ Tout scan_tile(const Tin* __restrict__ in, int64_t base, int64_t n,
+                                          Tout start, Tout* __restrict__ out) {
+  __shared__ Tout warp_sum[kWarps + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t i0 = base + (int64_t)warp * (32 * kItems) + lane;
+  uint32_t v[kItems], most = 0;
+#pragma unroll
+  for (int j = 0; j < kItems; j++) {
+    v[j] = i0 + j * 32 < n ? (uint32_t)in[i0 + j * 32] : 0u;
+    most |= v[j];
+  }
+  Tout ex[kItems];
+  Tout run;
+  constexpr uint32_t kFits = 0xffffffffu / (32 * kItems);
+  if (sizeof(Tout) == 4 || !__any_sync(0xffffffffu, most > kFits)) {
+    run = (Tout)scan_rounds<uint32_t, kItems>(v);
+#pragma unroll
+    for (int j = 0; j < kItems; j++) ex[j] = (Tout)v[j];
+  } else {
+#pragma unroll
+    for (int j = 0; j < kItems; j++) ex[j] = (Tout)v[j];
+    run = scan_rounds<Tout, kItems>(ex);
+  }
+  if (lane == 0) warp_sum[warp] = run;
+  __syncthreads();
+  if (warp == 0) {
+    const Tout w = lane < kWarps ? warp_sum[lane] : Tout(0);
+    const Tout wi = warp_inclusive_scan(w);
+    if (lane < kWarps) warp_sum[lane] = wi - w;
+    if (lane == kWarps - 1) warp_sum[kWarps] = wi;
+  }
+  __syncthreads();
+  start += warp_sum[warp];
+#pragma unroll
+  for (int j = 0; j < kItems; j++)
+    if (i0 + j * 32 < n) out[i0 + j * 32] = start + ex[j];
+  return warp_sum[kWarps];
 }
 
 template <class Tin, class Tout>
-__global__ void k_tile_scan(const Tin* __restrict__ in, int64_t n, const Tout* __restrict__ sums,
-                            Tout* __restrict__ out) {
-  __shared__ Tout sm[9];
-  const int64_t base = (int64_t)blockIdx.x * kScanTile;
-  // blocked arrangement: thread t owns items [t*16, t*16+16) of the tile
-  Tout v[kScanItems];
-  Tout acc = 0;
-  const int64_t mybase = base + (int64_t)threadIdx.x * kScanItems;
-#pragma unroll
-  for (int j = 0; j < kScanItems; j++) {
-    int64_t i = mybase + j;
-    v[j] = i < n ? (Tout)in[i] : Tout(0);
-    acc += v[j];
-  }
-  Tout ex = block_exclusive_scan_256<Tout>(acc, sm, nullptr) + sums[blockIdx.x];
-#pragma unroll
-  for (int j = 0; j < kScanItems; j++) {
-    int64_t i = mybase + j;
-    if (i < n) out[i] = ex;
-    ex += v[j];
+__global__ void __launch_bounds__(kScanThreads) k_tile_scan(ScanArgs<Tin, Tout> a) {
+  scan_tile<Tin, Tout, kScanThreads / 32, kScanItems>(
+      a.in + blockIdx.y * a.in_step, (int64_t)blockIdx.x * kScanTile, a.n,
+      a.sums[blockIdx.y * a.sums_step + blockIdx.x], a.out + blockIdx.y * a.out_step);
+}
+
+// The whole scan of up to kScanOne elements by one block per array: a small
+// call is bound by its launches (three of them with their gaps took 14 us for
+// 8,192 counts, this one 3.7), and no tile sums are needed.
+constexpr int kScanOneThreads = 1024;
+constexpr int64_t kScanOne = kScanOneThreads * kScanItems;
+template <class Tin, class Tout, int kItems>
+__global__ void __launch_bounds__(kScanOneThreads) k_scan_one(ScanArgs<Tin, Tout> a) {
+  Tout* out = a.out + blockIdx.y * a.out_step;
+  const Tout total = scan_tile<Tin, Tout, kScanOneThreads / 32, kItems>(
+      a.in + blockIdx.y * a.in_step, 0, a.n, Tout(0), out);
+  if (threadIdx.x == 0) {
+    out[a.n] = total;
+    if (a.totals) a.totals[blockIdx.y] = total;
   }
 }
 
@@ -139,34 +217,37 @@ __global__ void __launch_bounds__(kScanThreads)
   }
 }
 
-// Scan with caller-owned tile sums ((tiles + 1) entries of Tout).
+// Scans of `count` arrays with caller-owned tile sums (sums_step entries of
+// Tout for each).
 template <class Tin, class Tout>
-void scan_into_impl(const Tin* in, Tout* out, int64_t n, Tout* sums, cudaStream_t s) {
-  if (n == 0) {
-    SPJ_CUDA(cudaMemsetAsync(out, 0, sizeof(Tout), s));
-    return;
+void scan_launch(const ScanArgs<Tin, Tout>& a, unsigned count, cudaStream_t s) {
+  const dim3 one(1, count);
+  if (a.n <= kScanOne / 4) {
+    k_scan_one<Tin, Tout, kScanItems / 4><<<one, kScanOneThreads, 0, s>>>(a);
+  } else if (a.n <= kScanOne / 2) {
+    k_scan_one<Tin, Tout, kScanItems / 2><<<one, kScanOneThreads, 0, s>>>(a);
+  } else if (a.n <= kScanOne) {
+    k_scan_one<Tin, Tout, kScanItems><<<one, kScanOneThreads, 0, s>>>(a);
+  } else {
+    const int64_t nt = (a.n + kScanTile - 1) / kScanTile;
+    const dim3 g((unsigned)nt, count);
+    k_tile_reduce<Tin, Tout><<<g, kScanThreads, 0, s>>>(a);
+    k_scan_sums<Tout><<<dim3(1, count), 1024, 0, s>>>(a.sums, nt, a.out + a.n, a.sums_step,
+                                                      a.out_step, a.totals);
+    k_tile_scan<Tin, Tout><<<g, kScanThreads, 0, s>>>(a);
   }
-  const int64_t nt = (n + kScanTile - 1) / kScanTile;
-  k_tile_reduce<Tin, Tout><<<(unsigned)nt, kScanThreads, 0, s>>>(in, n, sums);
-  k_scan_sums<Tout><<<1, 1024, 0, s>>>(sums, nt, out + n);
-  k_tile_scan<Tin, Tout><<<(unsigned)nt, kScanThreads, 0, s>>>(in, n, sums, out);
   SPJ_CUDA(cudaGetLastError());
 }
 
 template <class Tin, class Tout>
+void scan_into_impl(const Tin* in, Tout* out, int64_t n, Tout* sums, cudaStream_t s) {
+  scan_launch<Tin, Tout>({in, out, sums, nullptr, n, 0, 0, 0}, 1, s);
+}
+
+template <class Tin, class Tout>
 void scan_impl(const Tin* in, Tout* out, int64_t n, DevBuf& tmp, cudaStream_t s) {
-  int64_t nt = (n + kScanTile - 1) / kScanTile;
-  if (nt < 1) nt = 1;
-  tmp.reserve((size_t)(nt + 1) * sizeof(Tout), s);
-  Tout* sums = tmp.as<Tout>();
-  if (n == 0) {
-    SPJ_CUDA(cudaMemsetAsync(out, 0, sizeof(Tout), s));
-    return;
-  }
-  k_tile_reduce<Tin, Tout><<<(unsigned)nt, kScanThreads, 0, s>>>(in, n, sums);
-  k_scan_sums<Tout><<<1, 1024, 0, s>>>(sums, nt, out + n);
-  k_tile_scan<Tin, Tout><<<(unsigned)nt, kScanThreads, 0, s>>>(in, n, sums, out);
-  SPJ_CUDA(cudaGetLastError());
+  tmp.reserve(scan_tile_sums_bytes(n), s);
+  scan_into_impl<Tin, Tout>(in, out, n, tmp.as<Tout>(), s);
 }
 
 // ---------------------------------------------------------------------------
@@ -203,8 +284,23 @@ __global__ void k_digit_hist(const uint32_t* __restrict__ keys, int64_t n, int s
   hist[hist_slot(threadIdx.x, blockIdx.x, ntiles, seg_tiles)] = h[threadIdx.x];
 }
 
+// The lanes whose digit (8 bits) is the lane's own; all 32 lanes call.  Eight
+// ballots: one __match_any_sync took as long as some 70 instructions and held
+// up the other warps of its SM (1M pairs: 22.3 us a pass of k_digit_scatter
+// with it, 9.7 this way).
+__device__ __forceinline__ unsigned same_digit(uint32_t d) {
+  unsigned peers = 0xffffffffu;
+#pragma unroll
+  for (int b = 0; b < 8; b++) {
+    const bool on = (d >> b) & 1u;
+    const unsigned who = __ballot_sync(0xffffffffu, on);
+    peers &= on ? who : ~who;
+  }
+  return peers;
+}
+
 // One 8-bit LSD pass over a tile of kSortTile items: stable local ranking by
-// digit (warp w ranks its 256 items in 8 rounds of 32 with __match_any_sync
+// digit (warp w ranks its 256 items in 8 rounds of 32 with same_digit
 // and per-warp digit counters; a scan over warps and digits gives each item
 // its place in the tile's digit-sorted order), a reorder in shared memory,
 // and a write of each digit run to its global offset (scan of the tile
@@ -236,14 +332,11 @@ __global__ void __launch_bounds__(kSortThreads)
     k[j] = valid ? keys[base + li] : 0xFFFFFFFFu;
     v[j] = valid ? vals[base + li] : 0u;
     const uint32_t d = (k[j] >> shift) & 0xFFu;
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    const unsigned peers = same_digit(d);
     const int leader = __ffs(peers) - 1;
-    uint32_t b = 0;
-    if (lane == leader) {
-      b = wcnt[w][d];
-      wcnt[w][d] = b + (uint32_t)__popc(peers);
-    }
-    b = __shfl_sync(peers, b, leader);
+    const uint32_t b = wcnt[w][d];
+    __syncwarp();
+    if (lane == leader) wcnt[w][d] = b + (uint32_t)__popc(peers);
     pos[j] = b + (uint32_t)__popc(peers & ((1u << lane) - 1u));
     __syncwarp();  // the counters' updates before the next round reads them
   }
@@ -281,8 +374,112 @@ __global__ void __launch_bounds__(kSortThreads)
   }
 }
 
+// The whole sort of up to 1024 * kItems pairs by one block: keys and values
+// stay in shared memory and registers over all passes (ranked per pass as in
+// k_digit_scatter, 32 warps of 32 * kItems consecutive items).  A small sort
+// is bound by its launches: 4,096 pairs took 5 of them and 29 us a pass, 3.8
+// us this way.  Up to kSortOne pairs, where one SM's shared memory ends and so
+// does the gain: 16,384 pairs take 12.3 us a pass, by tiles 14.
+constexpr int kSortOneThreads = 1024;
+constexpr int64_t kSortOne = 16 * kSortOneThreads;
+constexpr size_t sort_one_smem(int items) {
+  return (size_t)kSortOneThreads * items * 8 + 32 * 256 * 2 + 256 * 4;
+}
+template <int kItems>
+__global__ void __launch_bounds__(kSortOneThreads)
+    k_sort_one(uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, int n, int key_bits,
+               bool keys_out) {
+  extern __shared__ __align__(16) uint32_t sort_smem[];
+  uint32_t* sk = sort_smem;
+  uint32_t* sv = sk + kSortOneThreads * kItems;
+  uint32_t* doff = sv + kSortOneThreads * kItems;
+  uint16_t* wcnt = reinterpret_cast<uint16_t*>(doff + 256);  // [warp][digit]
+  __shared__ uint32_t scan_sm[9];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i0 = w * (32 * kItems) + lane;
+  uint32_t k[kItems], v[kItems], pos[kItems];
+#pragma unroll
+  for (int j = 0; j < kItems; j++) {
+    const int i = i0 + j * 32;
+    k[j] = i < n ? keys[i] : 0xFFFFFFFFu;  // (pads stay behind every key)
+    v[j] = i < n ? vals[i] : 0u;
+  }
+  for (int shift = 0; shift < key_bits; shift += 8) {
+    uint32_t* zero = reinterpret_cast<uint32_t*>(wcnt);
+    for (int t = threadIdx.x; t < 32 * 256 / 2; t += kSortOneThreads) zero[t] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kItems; j++) {
+      const uint32_t d = (k[j] >> shift) & 0xFFu;
+      const unsigned peers = same_digit(d);
+      const uint32_t b = wcnt[w * 256 + d];
+      __syncwarp();
+      if (lane == __ffs(peers) - 1) wcnt[w * 256 + d] = (uint16_t)(b + __popc(peers));
+      pos[j] = b + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+      __syncwarp();  // the counters' updates before the next round reads them
+    }
+    __syncthreads();
+    uint32_t run = 0;
+    if (threadIdx.x < 256) {
+#pragma unroll
+      for (int ww = 0; ww < 32; ww++) {
+        const uint32_t c = wcnt[ww * 256 + threadIdx.x];
+        wcnt[ww * 256 + threadIdx.x] = (uint16_t)run;
+        run += c;
+      }
+      const uint32_t inc = warp_inclusive_scan(run);
+      if (lane == 31) scan_sm[w] = inc;
+      run = inc - run;
+    }
+    __syncthreads();
+    if (threadIdx.x < 256) {
+      for (int ww = 0; ww < w; ww++) run += scan_sm[ww];
+      doff[threadIdx.x] = run;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kItems; j++) {
+      const uint32_t d = (k[j] >> shift) & 0xFFu;
+      const uint32_t to = doff[d] + wcnt[w * 256 + d] + pos[j];
+      sk[to] = k[j];
+      sv[to] = v[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kItems; j++) {
+      k[j] = sk[i0 + j * 32];
+      v[j] = sv[i0 + j * 32];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kItems; j++) {
+    const int i = i0 + j * 32;
+    if (i < n) {
+      if (keys_out) keys[i] = k[j];
+      vals[i] = v[j];
+    }
+  }
+}
+
+template <int kItems>
+void sort_one(uint32_t* keys, uint32_t* vals, int64_t n, int key_bits, bool keys_out,
+              cudaStream_t s) {
+  constexpr size_t smem = sort_one_smem(kItems);
+  SPJ_CUDA(cudaFuncSetAttribute(k_sort_one<kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)smem));
+  k_sort_one<kItems><<<1, kSortOneThreads, smem, s>>>(keys, vals, (int)n, key_bits, keys_out);
+  SPJ_CUDA(cudaGetLastError());
+}
+
 }  // namespace
 
+void scan_u32_u64_many(const uint32_t* in, int64_t in_step, uint64_t* out, int64_t out_step,
+                       int64_t n, int count, uint64_t* totals, DevBuf& tmp, cudaStream_t s) {
+  const int64_t step = (int64_t)(scan_tile_sums_bytes(n) / sizeof(uint64_t));
+  tmp.reserve((size_t)count * step * sizeof(uint64_t), s);
+  scan_launch<uint32_t, uint64_t>({in, out, tmp.as<uint64_t>(), totals, n, in_step, out_step, step},
+                                  (unsigned)count, s);
+}
 void scan_u32_u64(const uint32_t* in, uint64_t* out, int64_t n, DevBuf& tmp, cudaStream_t s) {
   scan_impl<uint32_t, uint64_t>(in, out, n, tmp, s);
 }
@@ -296,15 +493,7 @@ size_t scan_tile_sums_bytes(int64_t n) {
 
 void scan_u32_u64_into(const uint32_t* in, uint64_t* out, int64_t n, uint64_t* sums,
                        cudaStream_t s) {
-  if (n == 0) {
-    SPJ_CUDA(cudaMemsetAsync(out, 0, sizeof(uint64_t), s));
-    return;
-  }
-  const int64_t nt = (n + kScanTile - 1) / kScanTile;
-  k_tile_reduce<uint32_t, uint64_t><<<(unsigned)nt, kScanThreads, 0, s>>>(in, n, sums);
-  k_scan_sums<uint64_t><<<1, 1024, 0, s>>>(sums, nt, out + n);
-  k_tile_scan<uint32_t, uint64_t><<<(unsigned)nt, kScanThreads, 0, s>>>(in, n, sums, out);
-  SPJ_CUDA(cudaGetLastError());
+  scan_into_impl<uint32_t, uint64_t>(in, out, n, sums, s);
 }
 
 void scan_u32_u32(const uint32_t* in, uint32_t* out, int64_t n, DevBuf& tmp, cudaStream_t s) {
@@ -322,8 +511,9 @@ void compact_count(const uint8_t* flags, int64_t n, uint64_t* sums, cudaStream_t
     return;
   }
   const int64_t nt = (n + kScanTile - 1) / kScanTile;
-  k_tile_reduce<uint8_t, uint64_t><<<(unsigned)nt, kScanThreads, 0, s>>>(flags, n, sums);
-  k_scan_sums<uint64_t><<<1, 1024, 0, s>>>(sums, nt, sums + nt);
+  k_tile_reduce<uint8_t, uint64_t>
+      <<<(unsigned)nt, kScanThreads, 0, s>>>({flags, nullptr, sums, nullptr, n, 0, 0, 0});
+  k_scan_sums<uint64_t><<<1, 1024, 0, s>>>(sums, nt, sums + nt, 0, 0, nullptr);
   SPJ_CUDA(cudaGetLastError());
 }
 
@@ -348,6 +538,12 @@ void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* alt_keys, uint32
                       bool keys_out) {
   if (n <= 1) return;
   SPJ_CHECK(n < (int64_t)0xFFFFFFFF, "radix sort: too many keys");
+  if (n <= kSortOne && segments <= 1) {
+    if (n <= 4 * kSortOneThreads) sort_one<4>(keys, vals, n, key_bits, keys_out, s);
+    else if (n <= 8 * kSortOneThreads) sort_one<8>(keys, vals, n, key_bits, keys_out, s);
+    else sort_one<16>(keys, vals, n, key_bits, keys_out, s);
+    return;
+  }
   const int64_t ntiles = (n + kSortTile - 1) / kSortTile;
   const int64_t seg_tiles =
       segments > 1 ? (ntiles + segments - 1) / segments : ntiles;

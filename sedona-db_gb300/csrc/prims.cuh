@@ -1,7 +1,7 @@
 // prims.cuh — device-wide scan and radix sort used by the decode, LBVH and
 // two-pass count/scatter stages.  Written for sm_103a: 256-thread blocks,
 // warp-shuffle block scans, 8-bit LSD radix passes with block-local stable
-// ranking (warp match) and a reorder in shared memory.
+// ranking (ballots) and a reorder in shared memory.
 #pragma once
 #include "common.cuh"
 
@@ -11,6 +11,10 @@ namespace spj {
 void scan_u32_u64(const uint32_t* in, uint64_t* out, int64_t n, DevBuf& tmp, cudaStream_t s);
 void scan_u8_u64(const uint8_t* in, uint64_t* out, int64_t n, DevBuf& tmp, cudaStream_t s);
 void scan_u32_u32(const uint32_t* in, uint32_t* out, int64_t n, DevBuf& tmp, cudaStream_t s);
+// The same for `count` arrays of n elements, in_step / out_step elements
+// apart, by the same launches; totals[i] (device, may be null) = array i's total.
+void scan_u32_u64_many(const uint32_t* in, int64_t in_step, uint64_t* out, int64_t out_step,
+                       int64_t n, int count, uint64_t* totals, DevBuf& tmp, cudaStream_t s);
 // Same scan with caller-owned tile-sum scratch of scan_tile_sums_bytes(n) bytes.
 size_t scan_tile_sums_bytes(int64_t n);
 void scan_u32_u64_into(const uint32_t* in, uint64_t* out, int64_t n, uint64_t* tile_sums,

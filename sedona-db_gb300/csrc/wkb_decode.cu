@@ -369,14 +369,23 @@ __global__ void k_ring_flags(uint32_t nrings, const uint32_t* __restrict__ ring_
   }
 }
 
-__global__ void k_u64_to_u32(const uint64_t* __restrict__ in, uint32_t* __restrict__ out,
-                             int64_t n) {
+// out = in (null: zeros); *pa = a and *pb = b, where given, ride along
+__global__ void k_u64_to_u32(const uint64_t* __restrict__ in, uint32_t* __restrict__ out, int64_t n,
+                             uint32_t* pa = nullptr, uint32_t a = 0, uint32_t* pb = nullptr,
+                             uint32_t b = 0) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (pa) *pa = a;
+    if (pb) *pb = b;
+  }
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = (uint32_t)in[i];
+    out[i] = in ? (uint32_t)in[i] : 0u;
 }
 
-__global__ void k_set_u32(uint32_t* p, uint32_t v) { *p = v; }
+__global__ void k_reset_status(DeviceStatus* st) {
+  if (threadIdx.x < 8) st->counters[threadIdx.x] = 0;
+  else st->first_bad = ~0ull;  // no failure
+}
 
 // ---------------------------------------------------------------------------
 // y-band edge index
@@ -605,15 +614,19 @@ __global__ void k_band_permute(uint32_t n, const uint32_t* __restrict__ perm,
 
 void reset_status(DevBuf& status, cudaStream_t s) {
   status.reserve(sizeof(DeviceStatus), s);
-  SPJ_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(DeviceStatus), s));
-  // first_bad = all ones (no failure)
-  SPJ_CUDA(cudaMemsetAsync(status.get(), 0xFF, sizeof(unsigned long long), s));
+  k_reset_status<<<1, 9, 0, s>>>(status.as<DeviceStatus>());
+  SPJ_CUDA(cudaGetLastError());
 }
 
 void check_status(DevBuf& status, cudaStream_t s, const char* what) {
-  unsigned long long v = 0;
-  SPJ_CUDA(cudaMemcpyAsync(&v, status.get(), sizeof v, cudaMemcpyDeviceToHost, s));
+  DeviceStatus st;
+  SPJ_CUDA(cudaMemcpyAsync(&st, status.get(), sizeof st, cudaMemcpyDeviceToHost, s));
   SPJ_CUDA(cudaStreamSynchronize(s));
+  check_status(st, what);
+}
+
+void check_status(const DeviceStatus& st, const char* what) {
+  const unsigned long long v = st.first_bad;
   if (v != ~0ull) {
     uint32_t code = (uint32_t)(v >> 40);
     uint64_t row = v & 0xFFFFFFFFFFull;
@@ -648,20 +661,21 @@ void decode_wkb(const WkbDeviceColumn& col, DeviceGeoms& out, DecodeScratch& sc,
                                                 nullptr, nullptr, nullptr,
                                                 sc.status.as<DeviceStatus>(), true);
     SPJ_CUDA(cudaGetLastError());
-    unsigned long long v = 0;
-    SPJ_CUDA(cudaMemcpyAsync(&v, sc.status.get(), sizeof v, cudaMemcpyDeviceToHost, s));
+    DeviceStatus own, *st = sc.host ? static_cast<DeviceStatus*>(sc.host) : &own;
+    SPJ_CUDA(cudaMemcpyAsync(st, sc.status.get(), sizeof own, cudaMemcpyDeviceToHost, s));
     SPJ_CUDA(cudaStreamSynchronize(s));
-    if (v == ~0ull) {
+    if (st->first_bad == ~0ull) {
       out.nparts = out.nrings = out.nverts = 0;
       out.all_points = true;
       out.any_points = n > 0;
       out.any_polys = false;
       out.row_part.reserve((n + 1) * 4, s);
-      SPJ_CUDA(cudaMemsetAsync(out.row_part.get(), 0, (n + 1) * 4, s));
       out.part_ring.reserve(4, s);
-      SPJ_CUDA(cudaMemsetAsync(out.part_ring.get(), 0, 4, s));
       out.ring_vtx.reserve(4, s);
-      SPJ_CUDA(cudaMemsetAsync(out.ring_vtx.get(), 0, 4, s));
+      k_u64_to_u32<<<grid_for(n + 1, 256), 256, 0, s>>>(nullptr, out.row_part.as<uint32_t>(),
+                                                        n + 1, out.part_ring.as<uint32_t>(), 0,
+                                                        out.ring_vtx.as<uint32_t>(), 0);
+      SPJ_CUDA(cudaGetLastError());
       out.has_bands = false;
       out.has_row_flags = false;
       out.has_ring_flags = false;
@@ -693,15 +707,16 @@ void decode_wkb(const WkbDeviceColumn& col, DeviceGeoms& out, DecodeScratch& sc,
                                               crings, cverts, sc.status.as<DeviceStatus>(), false,
                                               out.row_flags.as<uint8_t>(), any_rflag);
   SPJ_CUDA(cudaGetLastError());
-  scan_u32_u64(cparts, spart, n, sc.tmp, s);
-  scan_u32_u64(crings, sring, n, sc.tmp, s);
-  scan_u32_u64(cverts, svert, n, sc.tmp, s);
-  uint64_t tot[4];
-  SPJ_CUDA(cudaMemcpyAsync(&tot[3], any_rflag, 8, cudaMemcpyDeviceToHost, s));
-  SPJ_CUDA(cudaMemcpyAsync(&tot[0], spart + n, 8, cudaMemcpyDeviceToHost, s));
-  SPJ_CUDA(cudaMemcpyAsync(&tot[1], sring + n, 8, cudaMemcpyDeviceToHost, s));
-  SPJ_CUDA(cudaMemcpyAsync(&tot[2], svert + n, 8, cudaMemcpyDeviceToHost, s));
-  check_status(sc.status, s, "WKB decode");  // syncs
+  // the totals of parts, rings and vertices go to counters[4..6], so that one
+  // copy and one wait bring back all that the host needs
+  scan_u32_u64_many(cparts, n + 1, spart, n + 1, n, 3,
+                    reinterpret_cast<uint64_t*>(&sc.status.as<DeviceStatus>()->counters[4]),
+                    sc.tmp, s);
+  DeviceStatus own, *st = sc.host ? static_cast<DeviceStatus*>(sc.host) : &own;
+  SPJ_CUDA(cudaMemcpyAsync(st, sc.status.get(), sizeof own, cudaMemcpyDeviceToHost, s));
+  SPJ_CUDA(cudaStreamSynchronize(s));
+  check_status(*st, "WKB decode");
+  const unsigned long long* tot = &st->counters[4];
   SPJ_CHECK(tot[2] < 0xFFFFFFFFull && tot[1] < 0xFFFFFFFFull, "decode: too many vertices");
   out.nparts = (uint32_t)tot[0];
   out.nrings = (uint32_t)tot[1];
@@ -714,7 +729,6 @@ void decode_wkb(const WkbDeviceColumn& col, DeviceGeoms& out, DecodeScratch& sc,
   out.has_ring_flags = false;
 
   out.row_part.reserve((n + 1) * 4, s);
-  k_u64_to_u32<<<grid_for(n + 1, 256), 256, 0, s>>>(spart, out.row_part.as<uint32_t>(), n + 1);
   out.part_ring.reserve(((size_t)out.nparts + 1) * 4, s);
   out.ring_vtx.reserve(((size_t)out.nrings + 1) * 4, s);
   out.ring_nsegs.reserve(((size_t)out.nrings + 1) * 4, s);
@@ -725,8 +739,9 @@ void decode_wkb(const WkbDeviceColumn& col, DeviceGeoms& out, DecodeScratch& sc,
   sc.ring_src.reserve(((size_t)out.nrings + 1) * 12, s);
   uint64_t* ring_src = sc.ring_src.as<uint64_t>();
   uint32_t* ring_npts = reinterpret_cast<uint32_t*>(ring_src + out.nrings + 1);
-  k_set_u32<<<1, 1, 0, s>>>(out.part_ring.as<uint32_t>() + out.nparts, out.nrings);
-  k_set_u32<<<1, 1, 0, s>>>(out.ring_vtx.as<uint32_t>() + out.nrings, out.nverts);
+  k_u64_to_u32<<<grid_for(n + 1, 256), 256, 0, s>>>(
+      spart, out.row_part.as<uint32_t>(), n + 1, out.part_ring.as<uint32_t>() + out.nparts,
+      out.nrings, out.ring_vtx.as<uint32_t>() + out.nrings, out.nverts);
   if (out.nparts > 0) {
     if (col.offsets64)
       k_wkb_struct<true><<<grid, block, 0, s>>>(col, al, out.kind.as<uint8_t>(), spart, sring,
@@ -788,8 +803,7 @@ void build_band_index(DeviceGeoms& g, DecodeScratch& sc, cudaStream_t s) {
   k_band_count<<<grid_for((int64_t)nr * 32, 128, kNumSMs * 16), 128, 0, s>>>(
       nr, g.ring_nsegs.as<int32_t>(), g.ring_vtx.as<uint32_t>(), g.ring_rect.as<Rect64>(),
       g.xy32.as<float2>(), nbp1, nent, g.band_param.as<float2>(), largest);
-  scan_u32_u64(nbp1, sb, nr, sc.tmp, s);
-  scan_u32_u64(nent, se, nr, sc.tmp, s);
+  scan_u32_u64_many(nbp1, nr + 1, sb, nr + 1, nr, 2, nullptr, sc.tmp, s);
   uint64_t tb = 0, te = 0;
   uint32_t most = 0;
   SPJ_CUDA(cudaMemcpyAsync(&tb, sb + nr, 8, cudaMemcpyDeviceToHost, s));

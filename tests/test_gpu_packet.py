@@ -171,3 +171,49 @@ def test_packet_dwithin_same_pairs_and_positions(capi, n, leaf):
                 got.append(j.probe(probe, "dwithin", distance=0.0 if d is rows else d))
             np.testing.assert_array_equal(got[0][0], got[1][0])
             np.testing.assert_array_equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("n", [1, 31, 4096, 4097, 8193, 16384, 16385, 20001])
+@pytest.mark.parametrize("order", [-1, 1])
+def test_scans_and_sorts_at_the_sizes_of_one_block(capi, n, order):
+    """Build and probe rows of both sides of the sizes that one block scans and
+    sorts: row i of a shuffled grid of squares meets the point of its centre."""
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(n)
+    at = rng.permutation(n)
+    x, y = (at % 150) * 3.0, (at // 150) * 3.0
+    build = wkb.column_from_values([
+        wkb.wkb_polygon([np.array([(a, b), (a + 1, b), (a + 1, b + 1), (a, b + 1), (a, b)])])
+        for a, b in zip(x, y)])
+    to = rng.permutation(n)
+    probe = wkb.points_column(x[to] + 0.5, y[to] + 0.5)
+    j = capi.SpatialJoin(probe_order=order)
+    j.build(build)
+    b, p = j.probe(probe, "intersects")
+    np.testing.assert_array_equal(p, np.arange(n))
+    np.testing.assert_array_equal(b, to)
+
+
+@pytest.mark.parametrize("pred,n", [("dwithin", 2047), ("dwithin", 2048), ("contains", 8191),
+                                    ("contains", 8192), ("touches", 8192)])
+def test_packet_from_the_first_row_counts(capi, pred, n):
+    """The sizes from which the packets are taken, against the candidate pairs."""
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(n)
+    if pred == "dwithin":
+        build, probe = (wkb.points_column(*rng.uniform(0, 200, (2, m))) for m in (3000, n))
+    else:
+        zones = _zones(rng, 60, holes=True)
+        build = wkb.column_from_values(zones)
+        probe = wkb.column_from_values(_probes(rng, n, "polygons", zones))
+    got = []
+    for option in (None, "candidate_order", "dwithin_arena"):
+        j = capi.SpatialJoin()
+        if option:
+            j.set_option(option, 0)
+        j.build(build)
+        got.append(j.probe(probe, pred, distance=4.0))
+    for other in got[1:]:
+        np.testing.assert_array_equal(got[0][0], other[0])
+        np.testing.assert_array_equal(got[0][1], other[1])
+    assert len(got[0][0]) > 0 or pred == "touches"
