@@ -545,7 +545,7 @@ void dwithin_packet(const LbvhView& t, const PointSplit& bs, const float4* probe
   if (n == 0) return;
   float lo, hi;
   float_neighbours(d, lo, hi);
-  k_dwithin_packet<<<grid_for(n, kTravThreads, kNumSMs * 16), kTravThreads, 0, s>>>(
+  k_dwithin_packet<<<grid_for((int64_t)n * 32, kTravThreads, kNumSMs * 16), kTravThreads, 0, s>>>(
       t, bs.xy.as<double2>(), bs.hl.as<float4>(), bs.bmag, bs.ok ? 1 : 0, probe_box, probe_pt, n,
       d, lo, hi, d_row, order, counts, a, st);
   SPJ_CUDA(cudaGetLastError());

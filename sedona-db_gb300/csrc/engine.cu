@@ -98,6 +98,14 @@ static inline float ev_ms(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
+// (ST_Intersects and ST_Disjoint stop at the first edge that decides, and
+// points visit few edges: their pairs are cheap.)
+static uint32_t packet_min_rows(int predicate, bool points) {
+  if (predicate == kPredDWithin) return kPacketRowsDWithin;
+  return points || predicate == kIntersects || predicate == kDisjoint ? kOrderMinRows
+                                                                      : kPacketRowsFull;
+}
+
 // Fused ST_DWithin of probes in Morton order: one traversal per 32 of them,
 // unless the slots or the arena of the traversal per probe were asked for.
 bool JoinEngine::packet_dwithin() const {
@@ -152,7 +160,7 @@ bool JoinEngine::packet_probe(Workspace& ws, int predicate, double distance, con
     SPJ_CUDA(cudaMemcpyAsync(rb->ctrl, a.ctrl, sizeof rb->ctrl, cudaMemcpyDeviceToHost, s));
     SPJ_CUDA(cudaMemcpyAsync(rb->fault, tv.fault, 8, cudaMemcpyDeviceToHost, s));
     SPJ_CUDA(cudaStreamSynchronize(s));
-    launches += points ? 5 : 6;
+    launches += 3 + scan_launches(n) + (points || dwithin ? 0 : 1);
     check_traversal_word(rb->fault);
     if (rb->ctrl[0] <= a.chunks && rb->ctrl[1] <= a.queue_cap) break;
     SPJ_CHECK(attempt < 2, "packet refine: record capacities did not settle");
@@ -195,9 +203,13 @@ uint64_t JoinEngine::probe(Workspace& ws, const WkbDeviceColumn& col, int predic
 
   const bool hint = ws.last_probe_points;
   decode_wkb(col, ws.probe, ws.dsc, hint, s);
-  launches += ws.probe.all_points && hint ? 1 : 17;
   ws.last_probe_points = ws.probe.all_points;
   const uint32_t n = ws.probe.n;
+  // points as expected: status, decode, row_part; else (after the failed
+  // attempt) with the scans, and the parts' structure, vertices and boxes
+  launches += ws.probe.all_points && hint
+                  ? 3
+                  : 3 + scan_launches(n) + (ws.probe.nparts ? 3 : 0) + (hint ? 2 : 0);
   if (prof) SPJ_CUDA(cudaEventRecord(ws.ev[1], s));
 
   const float4* boxes = ws.probe.box.as<float4>();
@@ -208,16 +220,20 @@ uint64_t JoinEngine::probe(Workspace& ws, const WkbDeviceColumn& col, int predic
     launches++;
   }
   const LbvhView tv = bvh_.view();
-  const uint32_t* order = nullptr;
-  if (cfg_.probe_order > 0 || (cfg_.probe_order == 0 && n >= kOrderMinRows)) {
-    order = probe_order(tv, boxes, n, ws.psc, s);
-    if (order) launches += 21;  // keys + 4 radix passes (histogram, 3-kernel scan, scatter)
-  }
   // point build and probe sides: the distance test runs inside the
   // traversal, no candidate pairs are materialized
   const bool fused = predicate == kPredDWithin && cfg_.fuse_dwithin &&
                      cfg_.refine_form == kFastF32 && ws.probe.all_points &&
                      bsplit_.n == bvh_.nprims && bvh_.nprims > 0;
+  const bool packet =
+      fused ? packet_dwithin() : packet_path(predicate, ws.probe.all_points);
+  const uint32_t* order = nullptr;
+  if (cfg_.probe_order > 0 ||
+      (cfg_.probe_order == 0 &&
+       n >= (packet ? packet_min_rows(predicate, ws.probe.all_points) : kOrderMinRows))) {
+    order = probe_order(tv, boxes, n, ws.psc, s);
+    if (order) launches += 1 + radix_sort_launches(n, 32);
+  }
   auto count = [&](const DeviceStatus& hst, uint64_t total) {
     std::lock_guard<std::mutex> lk(stats_mu_);
     stats_.calls++;
@@ -238,7 +254,7 @@ uint64_t JoinEngine::probe(Workspace& ws, const WkbDeviceColumn& col, int predic
     *d_build = ws.out_build.as<uint32_t>();
     *d_probe = ws.out_probe.as<uint32_t>();
   };
-  if (order && (fused ? packet_dwithin() : packet_path(predicate, ws.probe.all_points))) {
+  if (order && packet) {
     if (prof) SPJ_CUDA(cudaEventRecord(ws.ev[2], s));
     DeviceStatus hst;
     uint64_t total = 0;
@@ -434,7 +450,6 @@ uint64_t JoinEngine::refine_pairs(Workspace& ws, const GeomsView& pv, const uint
   ws.out_probe.reserve((total + 1) * 4, s);
   compact_pairs_tiles(cb, cp, ws.flags.as<uint8_t>(), (int64_t)m, sums,
                       ws.out_build.as<uint32_t>(), ws.out_probe.as<uint32_t>(), total, s);
-  SPJ_CUDA(cudaStreamSynchronize(s));
   {
     std::lock_guard<std::mutex> lk(stats_mu_);
     stats_.candidates += m;

@@ -85,6 +85,17 @@ struct EngineConfig {
   int host_slices = 0;
 };
 constexpr uint32_t kOrderMinRows = 1u << 16;
+// Rows from which the packet kernels are taken, by what a candidate costs
+// (packet_min_rows).  A packet's warp goes through its build rows one after
+// the other, so below some size the longest packet takes longer than the
+// candidate pairs spread over all threads.  Packets against pairs, us per
+// call: ST_DWithin with 400k points 720 / 857 at 2,000 rows; buildings
+// touching 50k zones 1,940 / 2,488 at 8,000 rows, in 20k holed zones
+// 1,242 / 1,228 at 8,000 and 1,298 / 1,497 at 12,000; intersecting 50k zones
+// 2,227 / 2,157 at 48,000 and 2,377 / 2,888 at 66,000; points in 50k zones
+// 1,298 / 1,100 at 66,000 and 1,341 / 1,600 at 100,000 (kOrderMinRows).
+constexpr uint32_t kPacketRowsDWithin = 1u << 11;
+constexpr uint32_t kPacketRowsFull = 1u << 13;
 constexpr uint64_t kBuildMajorMin = 1ull << 22;  // candidates before build-major order pays
 constexpr uint64_t kOrderTileCandidates = 1ull << 19;  // auto order_tiles: candidates per tile
 

@@ -366,11 +366,12 @@ __device__ __forceinline__ bool isolated_result(int predicate, bool in) {
 // Packets: runs of up to 32 consecutive rows of the Morton order.  A run whose
 // box is wide would meet many more build rows than its rows do (a cluster's
 // thin tail, a gap of the order) and one warp would still be at it when the
-// others are done, so it is cut in halves, down to 4 rows: an aligned group of
+// others are done, so it is cut in halves, down to one row: an aligned group of
 // rows is split where its box, widened by the mean build box, is over
 // kPacketGrowth times one row's and may meet over kPacketRows build rows (by
 // their mean density over the tree; with fewer, splitting costs more than it
-// saves).
+// saves).  (8,000 buildings, whose neighbours lie far apart: 1,667 us with
+// packets of 4 rows and up, 1,242 with single rows; 2M alike.)
 constexpr float kPacketRows = 64.0f, kPacketGrowth = 4.0f;
 __global__ void __launch_bounds__(256)
     k_packets(LbvhView t, const float4* __restrict__ box, const uint32_t* __restrict__ order,
@@ -400,7 +401,7 @@ __global__ void __launch_bounds__(256)
       // (both halves whole; an overflow to NaN counts as wide)
       const int other = __shfl_xor_sync(kAll, size, o);
       const bool whole = size == o && other == o;
-      if (whole && (o < 4 || w * h * per_area <= kPacketRows || w * h <= kPacketGrowth * own))
+      if (whole && (w * h * per_area <= kPacketRows || w * h <= kPacketGrowth * own))
         size = 2 * o;
     }
     const bool leader = (lane & (size - 1)) == 0 && j < n;
@@ -1017,7 +1018,7 @@ __global__ void __launch_bounds__(256)
 
 }  // namespace
 
-static uint64_t most_packets(uint32_t n) { return ((uint64_t)n + 31) / 32 * 8; }
+static uint64_t most_packets(uint32_t n) { return ((uint64_t)n + 31) / 32 * 32; }
 
 void PacketBufs::reserve(uint32_t n, uint64_t chunks, uint64_t queued, cudaStream_t s) {
   const uint64_t most = most_packets(n);
@@ -1072,7 +1073,8 @@ void packet_join(const LbvhView& t, const GeomsView& build, const GeomsView& pro
                  DeviceStatus* st, cudaStream_t s) {
   packet_runs(t, probe.box, order, probe.n, a, s);
   if (probe.n == 0) return;
-  const int g = grid_for(probe.n, kPacketThreads, kNumSMs * 8);
+  // (a warp per packet, and a packet may hold one row)
+  const int g = grid_for((int64_t)probe.n * 32, kPacketThreads, kNumSMs * 8);
   if (points) {
     k_packet<true><<<g, kPacketThreads, 0, s>>>(t, build, probe, order, predicate, counts, a, st);
   } else {

@@ -526,6 +526,13 @@ void compact_pairs_tiles(const uint32_t* cb, const uint32_t* cp, const uint8_t* 
   SPJ_CUDA(cudaGetLastError());
 }
 
+int scan_launches(int64_t n) { return n <= kScanOne ? 1 : 3; }
+
+int radix_sort_launches(int64_t n, int key_bits) {
+  if (n <= kSortOne) return 1;
+  return (key_bits + 7) / 8 * (2 + scan_launches((n + kSortTile - 1) / kSortTile * 256));
+}
+
 size_t radix_sort_tmp_bytes(int64_t n) {
   const int64_t ntiles = (n + kSortTile - 1) / kSortTile;
   const int64_t nh = 256 * (ntiles < 1 ? 1 : ntiles);

@@ -42,6 +42,9 @@ void compact_pairs_tiles(const uint32_t* cb, const uint32_t* cp, const uint8_t* 
 void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* alt_keys, uint32_t* alt_vals,
                       int64_t n, int key_bits, DevBuf& tmp, cudaStream_t s,
                       int64_t segments = 0, bool keys_out = true);
+// Launches of a scan of n elements and of a sort of n pairs.
+int scan_launches(int64_t n);
+int radix_sort_launches(int64_t n, int key_bits);
 // Bytes of tmp that radix_sort_pairs uses for n keys (reserve them before a
 // stream capture so that the sort allocates nothing inside it).
 size_t radix_sort_tmp_bytes(int64_t n);
