@@ -529,6 +529,34 @@ int SpjGatherBinary(const void* d_offsets, int32_t offsets_are_64bit, const uint
                     uint64_t n_values, const uint32_t* d_idx, uint64_t n,
                     int64_t* d_out_offsets, uint8_t* d_out_data, uint64_t capacity,
                     uint64_t* out_bytes, void* stream);
+/* The columns of one output batch together: with fewer launches and waits the
+ * same as SpjGatherValidity and SpjGatherFixed or SpjGatherBinary for each.
+ * The call fills values, validity bitmaps and offsets, and per column
+ * null_count and out_bytes; the caller then gives each binary column d_out_data
+ * of out_bytes bytes and SpjGatherColumnsData, with the same columns, fills
+ * them. */
+typedef struct SpjGatherColumn SpjGatherColumn;
+struct SpjGatherColumn {
+  const uint32_t* d_idx;   /* n rows */
+  uint64_t n;
+  const void* d_offsets;   /* binary column: its n_values + 1 offsets; else NULL */
+  const uint8_t* d_data;
+  int32_t offsets_are_64bit;
+  uint32_t width;          /* fixed width: bytes of a value */
+  const void* d_values;
+  uint64_t n_values;
+  const uint8_t* d_validity; /* of n_validity rows; NULL = all valid */
+  int64_t validity_offset;
+  uint64_t n_validity;
+  void* d_out_values;
+  int64_t* d_out_offsets;
+  uint8_t* d_out_data;
+  uint8_t* d_out_validity; /* ceil(n / 32) 32-bit words */
+  uint64_t out_bytes;
+  uint64_t null_count;
+};
+int SpjGatherColumns(SpjGatherColumn* cols, uint32_t n_cols, void* stream);
+int SpjGatherColumnsData(const SpjGatherColumn* cols, uint32_t n_cols, void* stream);
 /* Set bit idx[i] of a row bitmap (ceil(n_rows / 32) 32-bit words, LSB
  * order, which is Arrow's bitmap layout on a little-endian machine; the
  * caller zeroes it once per build side).  Indices >= n_rows are skipped. */

@@ -9,11 +9,15 @@
 //
 // All HBM-bound: a gathered fixed-width value reads its width once and writes
 // it once (the index 4 B); a binary value reads and writes its bytes once,
-// with a length pass, a scan and a copy pass (8 lanes per value, the
+// with a length pass, a scan and a copy pass (a lane group per value, the
 // destination written as whole 4-byte words whatever the alignments).
+// SpjGatherColumns takes the columns of a batch together: one launch for all
+// values, lengths and validity words, and one wait for all sizes.
 #include <errno.h>
 
+#include <algorithm>
 #include <string>
+#include <vector>
 
 #include "../../include/spj_gb300.h"
 #include "common.cuh"
@@ -30,43 +34,41 @@ int fail(const std::exception& e) {
   return EINVAL;
 }
 
-template <class T>
-__global__ void k_gather_fixed(const T* __restrict__ src, const uint32_t* __restrict__ idx,
-                               uint64_t n, uint64_t nsrc, T* __restrict__ out) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t j = idx[i];
-    T v{};
-    if (j != SPJ_NULL_INDEX && j < nsrc) v = src[j];
-    out[i] = v;
-  }
-}
+// One column of a gather.  Fixed width: values -> out; binary (width 0): the
+// rows' lengths -> len; validity words -> out_valid and the count of null rows
+// -> *nulls, where asked for.
+struct GatherCol {
+  const uint32_t* idx = nullptr;
+  uint64_t n = 0;
+  const void* values = nullptr;  // fixed width: the values; binary: the offsets
+  uint64_t n_values = 0;
+  uint32_t width = 0;
+  int off64 = 0;
+  void* out = nullptr;
+  uint32_t* len = nullptr;
+  const uint8_t* valid = nullptr;
+  int64_t voff = 0;
+  uint64_t n_valid = 0;
+  uint32_t* out_valid = nullptr;
+  unsigned long long* nulls = nullptr;
+};
+constexpr uint32_t kGatherCols = 8;
+struct GatherCols {
+  GatherCol c[kGatherCols];
+};
+constexpr int kGatherRows = 4;  // rows of a lane in flight
 
-// validity bits of the gathered rows: 32 rows per thread, one word out
-__global__ void k_gather_valid(const uint8_t* __restrict__ valid, int64_t voff,
-                               const uint32_t* __restrict__ idx, uint64_t n, uint64_t nsrc,
-                               uint32_t* __restrict__ out, unsigned long long* __restrict__ nulls) {
-  uint32_t cnt = 0;
-  const uint64_t nw = (n + 31) / 32;
-  for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nw;
-       w += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t bits = 0;
-    for (int b = 0; b < 32; b++) {
-      const uint64_t i = w * 32 + b;
-      if (i >= n) break;
-      const uint32_t j = idx[i];
-      bool ok = j != SPJ_NULL_INDEX && j < nsrc;
-      if (ok && valid) {
-        const uint64_t bit = (uint64_t)voff + j;
-        ok = (valid[bit >> 3] >> (bit & 7)) & 1;
-      }
-      if (ok) bits |= 1u << b;
-      else cnt++;
-    }
-    out[w] = bits;
+template <class T>
+__device__ __forceinline__ void gather_rows(const GatherCol& c, const uint32_t* j, uint64_t i) {
+  T v[kGatherRows];
+#pragma unroll
+  for (int u = 0; u < kGatherRows; u++) {
+    v[u] = T{};
+    if (j[u] != SPJ_NULL_INDEX && j[u] < c.n_values) v[u] = static_cast<const T*>(c.values)[j[u]];
   }
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-  if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(nulls, (unsigned long long)cnt);
+#pragma unroll
+  for (int u = 0; u < kGatherRows; u++)
+    if (i + u * 32 < c.n) static_cast<T*>(c.out)[i + u * 32] = v[u];
 }
 
 template <bool kOff64>
@@ -83,61 +85,137 @@ __device__ __forceinline__ void bin_range(const void* off, uint32_t j, uint64_t&
 }
 
 template <bool kOff64>
-__global__ void k_bin_lengths(const void* __restrict__ off, const uint32_t* __restrict__ idx,
-                              uint64_t n, uint64_t nsrc, uint32_t* __restrict__ len) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t j = idx[i];
-    uint32_t l = 0;
-    if (j != SPJ_NULL_INDEX && j < nsrc) {
-      uint64_t s, e;
-      bin_range<kOff64>(off, j, s, e);
-      l = e > s ? (uint32_t)(e - s) : 0;
+__device__ __forceinline__ void gather_lengths(const GatherCol& c, const uint32_t* j, uint64_t i) {
+  uint32_t l[kGatherRows];
+#pragma unroll
+  for (int u = 0; u < kGatherRows; u++) {
+    uint64_t s = 0, e = 0;
+    if (j[u] != SPJ_NULL_INDEX && j[u] < c.n_values) bin_range<kOff64>(c.values, j[u], s, e);
+    l[u] = e > s ? (uint32_t)(e - s) : 0;
+  }
+#pragma unroll
+  for (int u = 0; u < kGatherRows; u++)
+    if (i + u * 32 < c.n) c.len[i + u * 32] = l[u];
+}
+
+// Column blockIdx.y: a warp takes 128 rows at a time, a lane 4 of them 32
+// apart, so the index, the output and the validity word (a ballot of 32 rows)
+// are coalesced and 4 gathered values are in flight.  Bound by L2 and HBM: 4M
+// rows, 5 columns with validity, 171 us in passes of their own (32 rows per
+// thread for the validity words), 63 this way.
+__global__ void __launch_bounds__(256) k_gather_columns(const __grid_constant__ GatherCols cols) {
+  const GatherCol& c = cols.c[blockIdx.y];
+  const int lane = threadIdx.x & 31;
+  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  uint32_t nulls = 0;
+  for (uint64_t i0 = ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5) * (32 * kGatherRows);
+       i0 < c.n; i0 += nwarps * (32 * kGatherRows)) {
+    const uint64_t i = i0 + lane;
+    uint32_t j[kGatherRows];
+#pragma unroll
+    for (int u = 0; u < kGatherRows; u++)
+      j[u] = i + u * 32 < c.n ? c.idx[i + u * 32] : SPJ_NULL_INDEX;
+    if (c.out) {
+      switch (c.width) {
+        case 1: gather_rows<uint8_t>(c, j, i); break;
+        case 2: gather_rows<uint16_t>(c, j, i); break;
+        case 4: gather_rows<uint32_t>(c, j, i); break;
+        case 8: gather_rows<uint64_t>(c, j, i); break;
+        default: gather_rows<uint4>(c, j, i); break;
+      }
+    } else if (c.len) {
+      if (c.off64) gather_lengths<true>(c, j, i);
+      else gather_lengths<false>(c, j, i);
     }
-    len[i] = l;
+    if (c.out_valid) {
+#pragma unroll
+      for (int u = 0; u < kGatherRows; u++) {
+        const bool row = i + u * 32 < c.n;
+        bool ok = j[u] != SPJ_NULL_INDEX && j[u] < c.n_valid;
+        if (ok && c.valid) {
+          const uint64_t bit = (uint64_t)c.voff + j[u];
+          ok = (c.valid[bit >> 3] >> (bit & 7)) & 1;
+        }
+        const uint32_t word = __ballot_sync(0xffffffffu, ok);
+        nulls += row && !ok ? 1u : 0u;
+        if (lane == 0 && row) c.out_valid[(i >> 5) + u] = word;
+      }
+    }
+  }
+  if (c.out_valid) {
+    for (int o = 16; o > 0; o >>= 1) nulls += __shfl_xor_sync(0xffffffffu, nulls, o);
+    if (lane == 0 && nulls) atomicAdd(c.nulls, (unsigned long long)nulls);
+  }
+}
+
+void gather_columns(const GatherCol* c, size_t count, cudaStream_t s) {
+  for (size_t k = 0; k < count; k += kGatherCols) {
+    GatherCols a;
+    uint64_t most = 0;
+    const unsigned m = (unsigned)std::min<size_t>(kGatherCols, count - k);
+    for (unsigned q = 0; q < m; q++) {
+      a.c[q] = c[k + q];
+      most = std::max(most, c[k + q].n);
+    }
+    if (most == 0) continue;
+    const int g = grid_for((int64_t)(most + kGatherRows - 1) / kGatherRows, 256, kNumSMs * 8);
+    k_gather_columns<<<dim3((unsigned)g, m), 256, 0, s>>>(a);
+    SPJ_CUDA(cudaGetLastError());
   }
 }
 
 // A warp takes 32 values: lane k reads value k's index, source range and
-// output position (one memory latency for all 32), then lane groups of 8
-// copy 4 values at a time (group_copy: whole destination words, any
-// alignment).
-template <bool kOff64>
-__global__ void k_bin_copy(const void* __restrict__ off, const uint8_t* __restrict__ data,
-                           const uint32_t* __restrict__ idx, uint64_t n, uint64_t nsrc,
-                           const uint64_t* __restrict__ pos, uint8_t* __restrict__ out,
-                           uint64_t cap) {
-  constexpr int G = 8;
+// output position (one memory latency for all 32), then lane groups of G
+// copy a value each (group_copy_once: whole destination words, any alignment).
+// Bound by the requests to L1 and the latency of each value; two or four
+// values of a group in flight cost more in registers than they hid (4M WKB
+// values of 157 bytes: 220 and 403 us), as did the warp's run of the output in
+// 16-byte blocks (346 us).
+template <bool kOff64, int G, int U>
+__global__ void __launch_bounds__(256)
+    k_bin_copy(const void* __restrict__ off, const uint8_t* __restrict__ data,
+               const uint32_t* __restrict__ idx, uint64_t n, uint64_t nsrc,
+               const int64_t* __restrict__ pos, uint8_t* __restrict__ out, uint64_t cap) {
   const int lane = threadIdx.x & 31, grp = lane / G, gl = lane % G;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t i0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; i0 < n;
        i0 += nwarps * 32) {
     const uint64_t i = i0 + lane;
-    uint64_t s = 0, d = 0, l = 0;
+    uint64_t s = 0, d = 0;
+    uint32_t l = 0;
     if (i < n) {
       const uint32_t j = idx[i];
       if (j != SPJ_NULL_INDEX && j < nsrc) {
         uint64_t e;
         bin_range<kOff64>(off, j, s, e);
-        d = pos[i];
-        l = e > s ? e - s : 0;
+        d = (uint64_t)pos[i];
+        l = e > s ? (uint32_t)(e - s) : 0;
         if (d + l > cap) l = 0;  // bounded by the output buffer
       }
     }
-    for (int v = 0; v < 32; v += 32 / G) {
-      const uint64_t vs = __shfl_sync(0xffffffffu, s, v + grp);
-      const uint64_t vd = __shfl_sync(0xffffffffu, d, v + grp);
-      const uint64_t vl = __shfl_sync(0xffffffffu, l, v + grp);
-      if (vl) group_copy<G>(data + vs, out + vd, vl, gl);
+    for (int k = 0; k < 32; k += 32 / G) {
+      const uint64_t vs = __shfl_sync(0xffffffffu, s, k + grp);
+      const uint64_t vd = __shfl_sync(0xffffffffu, d, k + grp);
+      const uint32_t vl = __shfl_sync(0xffffffffu, l, k + grp);
+      if (vl) group_copy_once<G, U>(data + vs, out + vd, vl, gl);
     }
   }
 }
 
-__global__ void k_u64_to_i64_offsets(const uint64_t* __restrict__ pos, uint64_t n,
-                                     int64_t* __restrict__ out) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i <= n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    out[i] = (int64_t)pos[i];
+// Copies the gathered values of n rows to out (positions: the output offsets;
+// total bytes, at most cap of them written).  Values of up to 32 bytes on
+// average by groups of 4 lanes, which take 32 bytes in one go, longer ones by
+// groups of 8, which take 224: 4M names of 14 bytes 73 and 143 us, 4M WKB
+// values of 157 bytes 267 and 196 us.
+void copy_values(const void* off, bool off64, const uint8_t* data, uint64_t n_values,
+                 const uint32_t* idx, uint64_t n, const int64_t* pos, uint64_t total, uint8_t* out,
+                 uint64_t cap, cudaStream_t s) {
+  if (!n || !total) return;
+  const int g = grid_for((int64_t)n, 256, kNumSMs * 16);
+  const auto copy = total <= n * 32 ? (off64 ? k_bin_copy<true, 4, 2> : k_bin_copy<false, 4, 2>)
+                                    : (off64 ? k_bin_copy<true, 8, 7> : k_bin_copy<false, 8, 7>);
+  copy<<<g, 256, 0, s>>>(off, data, idx, n, n_values, pos, out, cap);
+  SPJ_CUDA(cudaGetLastError());
 }
 
 __global__ void k_mark(uint32_t* __restrict__ bits, uint64_t nbuild,
@@ -191,49 +269,39 @@ bool aligned(const void* p, size_t a) { return reinterpret_cast<uintptr_t>(p) % 
 }  // namespace
 
 uint64_t gather_binary(const WkbDeviceColumn& col, const uint32_t* d_idx, uint64_t n,
-                       DevBuf& out_off, DevBuf& out_data, DevBuf& scratch_len,
-                       DevBuf& scratch_pos, DevBuf& scan_tmp, cudaStream_t s) {
+                       DevBuf& out_off, DevBuf& out_data, DevBuf& scratch_len, DevBuf& scan_tmp,
+                       cudaStream_t s) {
   scratch_len.reserve(((size_t)n + 1) * 4, s);
-  scratch_pos.reserve(((size_t)n + 1) * 8, s);
   out_off.reserve(((size_t)n + 1) * 8, s);
-  const int g = grid_for((int64_t)n, 256, kNumSMs * 16);
-  if (n) {
-    if (col.offsets64)
-      k_bin_lengths<true><<<g, 256, 0, s>>>(col.offsets, d_idx, n, (uint64_t)col.n,
-                                            scratch_len.as<uint32_t>());
-    else
-      k_bin_lengths<false><<<g, 256, 0, s>>>(col.offsets, d_idx, n, (uint64_t)col.n,
-                                             scratch_len.as<uint32_t>());
-  }
-  scan_u32_u64(scratch_len.as<uint32_t>(), scratch_pos.as<uint64_t>(), (int64_t)n, scan_tmp, s);
+  GatherCol c;
+  c.idx = d_idx;
+  c.n = n;
+  c.values = col.offsets;
+  c.n_values = (uint64_t)col.n;
+  c.off64 = col.offsets64;
+  c.len = scratch_len.as<uint32_t>();
+  gather_columns(&c, 1, s);
+  scan_u32_u64(c.len, out_off.as<uint64_t>(), (int64_t)n, scan_tmp, s);
   uint64_t total = 0;
-  SPJ_CUDA(cudaMemcpyAsync(&total, scratch_pos.as<uint64_t>() + n, 8, cudaMemcpyDeviceToHost, s));
+  SPJ_CUDA(cudaMemcpyAsync(&total, out_off.as<uint64_t>() + n, 8, cudaMemcpyDeviceToHost, s));
   SPJ_CUDA(cudaStreamSynchronize(s));
-  k_u64_to_i64_offsets<<<grid_for((int64_t)n + 1, 256), 256, 0, s>>>(
-      scratch_pos.as<uint64_t>(), n, out_off.as<int64_t>());
   out_data.reserve(total + 16, s);
-  if (n && total) {
-    const int gw = grid_for((int64_t)n * 32, 256, kNumSMs * 32);
-    if (col.offsets64)
-      k_bin_copy<true><<<gw, 256, 0, s>>>(col.offsets, col.data, d_idx, n, (uint64_t)col.n,
-                                          scratch_pos.as<uint64_t>(), out_data.as<uint8_t>(),
-                                          total);
-    else
-      k_bin_copy<false><<<gw, 256, 0, s>>>(col.offsets, col.data, d_idx, n, (uint64_t)col.n,
-                                           scratch_pos.as<uint64_t>(), out_data.as<uint8_t>(),
-                                           total);
-  }
-  SPJ_CUDA(cudaGetLastError());
+  copy_values(col.offsets, col.offsets64, col.data, (uint64_t)col.n, d_idx, n,
+              out_off.as<int64_t>(), total, out_data.as<uint8_t>(), total, s);
   SPJ_CUDA(cudaStreamSynchronize(s));
   return total;
 }
 
 void gather_u64(const uint64_t* values, uint64_t n_values, const uint32_t* d_idx, uint64_t n,
                 uint64_t* out, cudaStream_t s) {
-  if (!n) return;
-  k_gather_fixed<uint64_t><<<grid_for((int64_t)n, 256, kNumSMs * 16), 256, 0, s>>>(
-      values, d_idx, n, n_values, out);
-  SPJ_CUDA(cudaGetLastError());
+  GatherCol c;
+  c.idx = d_idx;
+  c.n = n;
+  c.values = values;
+  c.n_values = n_values;
+  c.width = 8;
+  c.out = out;
+  gather_columns(&c, 1, s);
 }
 
 }  // namespace spj
@@ -251,23 +319,14 @@ extern "C" int SpjGatherFixed(const void* d_values, uint32_t width, uint64_t n_v
     SPJ_CHECK(aligned(d_values, width) && aligned(d_out, width) && aligned(d_idx, 4),
               "values and output must be aligned to the width, indices to 4 bytes");
     const cudaStream_t s = as_stream(stream);
-    if (n_values == 0) d_values = nullptr;
-    if (n) {
-      const int g = grid_for((int64_t)n, 256, kNumSMs * 16);
-#define SPJ_GF(T)                                                                          \
-  k_gather_fixed<T><<<g, 256, 0, s>>>(static_cast<const T*>(d_values), d_idx, n, n_values, \
-                                       static_cast<T*>(d_out))
-      switch (width) {
-        case 1: SPJ_GF(uint8_t); break;
-        case 2: SPJ_GF(uint16_t); break;
-        case 4: SPJ_GF(uint32_t); break;
-        case 8: SPJ_GF(uint64_t); break;
-        case 16: SPJ_GF(uint4); break;
-        default: throw Error("width must be 1, 2, 4, 8 or 16 bytes");
-      }
-#undef SPJ_GF
-      SPJ_CUDA(cudaGetLastError());
-    }
+    GatherCol c;
+    c.idx = d_idx;
+    c.n = n;
+    c.values = d_values;
+    c.n_values = n_values;
+    c.width = width;
+    c.out = d_out;
+    gather_columns(&c, 1, s);
     SPJ_CUDA(cudaStreamSynchronize(s));
     g_error.clear();
     return 0;
@@ -288,13 +347,15 @@ extern "C" int SpjGatherValidity(const uint8_t* d_validity, int64_t validity_off
     const cudaStream_t s = as_stream(stream);
     DevBuf cnt(8, s);
     SPJ_CUDA(cudaMemsetAsync(cnt.get(), 0, 8, s));
-    if (n) {
-      const uint64_t nw = (n + 31) / 32;
-      k_gather_valid<<<grid_for((int64_t)nw, 256, kNumSMs * 16), 256, 0, s>>>(
-          d_validity, validity_offset, d_idx, n, n_values,
-          reinterpret_cast<uint32_t*>(d_out_bitmap), cnt.as<unsigned long long>());
-      SPJ_CUDA(cudaGetLastError());
-    }
+    GatherCol c;
+    c.idx = d_idx;
+    c.n = n;
+    c.valid = d_validity;
+    c.voff = validity_offset;
+    c.n_valid = n_values;
+    c.out_valid = reinterpret_cast<uint32_t*>(d_out_bitmap);
+    c.nulls = cnt.as<unsigned long long>();
+    gather_columns(&c, 1, s);
     unsigned long long h = 0;
     SPJ_CUDA(cudaMemcpyAsync(&h, cnt.get(), 8, cudaMemcpyDeviceToHost, s));
     SPJ_CUDA(cudaStreamSynchronize(s));
@@ -318,38 +379,118 @@ extern "C" int SpjGatherBinary(const void* d_offsets, int32_t offsets_are_64bit,
                   aligned(d_idx, 4),
               "offsets and indices must be aligned to their element size");
     const cudaStream_t s = as_stream(stream);
-    DevBuf len(((size_t)n + 1) * 4, s), pos(((size_t)n + 1) * 8, s), tmp;
-    const int g = grid_for((int64_t)n, 256, kNumSMs * 16);
-    if (n) {
-      if (offsets_are_64bit)
-        k_bin_lengths<true><<<g, 256, 0, s>>>(d_offsets, d_idx, n, n_values, len.as<uint32_t>());
-      else
-        k_bin_lengths<false><<<g, 256, 0, s>>>(d_offsets, d_idx, n, n_values, len.as<uint32_t>());
-    }
-    scan_u32_u64(len.as<uint32_t>(), pos.as<uint64_t>(), (int64_t)n, tmp, s);
+    DevBuf len(((size_t)n + 1) * 4, s), tmp;
+    GatherCol c;
+    c.idx = d_idx;
+    c.n = n;
+    c.values = d_offsets;
+    c.n_values = n_values;
+    c.off64 = offsets_are_64bit != 0;
+    c.len = len.as<uint32_t>();
+    gather_columns(&c, 1, s);
+    scan_u32_u64(c.len, reinterpret_cast<uint64_t*>(d_out_offsets), (int64_t)n, tmp, s);
     uint64_t total = 0;
-    SPJ_CUDA(cudaMemcpyAsync(&total, pos.as<uint64_t>() + n, 8, cudaMemcpyDeviceToHost, s));
+    SPJ_CUDA(cudaMemcpyAsync(&total, d_out_offsets + n, 8, cudaMemcpyDeviceToHost, s));
     SPJ_CUDA(cudaStreamSynchronize(s));
     *out_bytes = total;
-    k_u64_to_i64_offsets<<<grid_for((int64_t)n + 1, 256), 256, 0, s>>>(pos.as<uint64_t>(), n,
-                                                                       d_out_offsets);
     if (total > capacity) {
-      SPJ_CUDA(cudaStreamSynchronize(s));
       g_error = "output capacity " + std::to_string(capacity) + " < " + std::to_string(total) +
                 " bytes";
       return ENOSPC;
     }
     if (n && total) {
       SPJ_CHECK(d_out_data != nullptr && d_data != nullptr, "null data buffer");
-      const int gw = grid_for((int64_t)n * 32, 256, kNumSMs * 32);
-      if (offsets_are_64bit)
-        k_bin_copy<true><<<gw, 256, 0, s>>>(d_offsets, d_data, d_idx, n, n_values,
-                                            pos.as<uint64_t>(), d_out_data, capacity);
-      else
-        k_bin_copy<false><<<gw, 256, 0, s>>>(d_offsets, d_data, d_idx, n, n_values,
-                                             pos.as<uint64_t>(), d_out_data, capacity);
+      copy_values(d_offsets, offsets_are_64bit != 0, d_data, n_values, d_idx, n, d_out_offsets,
+                  total, d_out_data, capacity, s);
     }
-    SPJ_CUDA(cudaGetLastError());
+    SPJ_CUDA(cudaStreamSynchronize(s));
+    g_error.clear();
+    return 0;
+  } catch (const std::exception& e) {
+    return fail(e);
+  }
+}
+
+extern "C" int SpjGatherColumns(SpjGatherColumn* cols, uint32_t n_cols, void* stream) {
+  try {
+    SPJ_CHECK(n_cols == 0 || cols != nullptr, "null columns");
+    const cudaStream_t s = as_stream(stream);
+    uint64_t lens = 0;
+    for (uint32_t k = 0; k < n_cols; k++) {
+      const SpjGatherColumn& c = cols[k];
+      SPJ_CHECK(c.n == 0 || (c.d_idx && c.d_out_validity), "null buffer");
+      SPJ_CHECK(aligned(c.d_out_validity, 4) && aligned(c.d_idx, 4),
+                "the output bitmap (written as 32-bit words) and the indices must be 4-byte "
+                "aligned");
+      if (c.d_offsets) {
+        SPJ_CHECK(c.d_out_offsets != nullptr, "null buffer");
+        SPJ_CHECK(aligned(c.d_offsets, c.offsets_are_64bit ? 8 : 4) && aligned(c.d_out_offsets, 8),
+                  "offsets and indices must be aligned to their element size");
+        lens += c.n + 1;
+      } else {
+        SPJ_CHECK(c.n == 0 || (c.d_out_values && (c.d_values || c.n_values == 0)), "null buffer");
+        SPJ_CHECK(c.width == 1 || c.width == 2 || c.width == 4 || c.width == 8 || c.width == 16,
+                  "width must be 1, 2, 4, 8 or 16 bytes");
+        SPJ_CHECK(aligned(c.d_values, c.width) && aligned(c.d_out_values, c.width),
+                  "values and output must be aligned to the width, indices to 4 bytes");
+      }
+    }
+    // per column: null rows, then data bytes
+    std::vector<unsigned long long> h(2 * (size_t)n_cols + 1);
+    DevBuf cnt(h.size() * 8, s), len(lens * 4, s), tmp;
+    SPJ_CUDA(cudaMemsetAsync(cnt.get(), 0, h.size() * 8, s));
+    std::vector<GatherCol> g(n_cols);
+    uint64_t at = 0;
+    for (uint32_t k = 0; k < n_cols; k++) {
+      const SpjGatherColumn& c = cols[k];
+      g[k].idx = c.d_idx;
+      g[k].n = c.n;
+      g[k].n_values = c.n_values;
+      if (c.d_offsets) {
+        g[k].values = c.d_offsets;
+        g[k].off64 = c.offsets_are_64bit != 0;
+        g[k].len = len.as<uint32_t>() + at;
+        at += c.n + 1;
+      } else {
+        g[k].values = c.d_values;
+        g[k].width = c.width;
+        g[k].out = c.d_out_values;
+      }
+      g[k].valid = c.d_validity;
+      g[k].voff = c.validity_offset;
+      g[k].n_valid = c.n_validity;
+      g[k].out_valid = reinterpret_cast<uint32_t*>(c.d_out_validity);
+      g[k].nulls = cnt.as<unsigned long long>() + 2 * k;
+    }
+    gather_columns(g.data(), n_cols, s);
+    for (uint32_t k = 0; k < n_cols; k++)
+      if (g[k].len)
+        scan_u32_u64_many(g[k].len, 0, reinterpret_cast<uint64_t*>(cols[k].d_out_offsets), 0,
+                          (int64_t)g[k].n, 1, cnt.as<uint64_t>() + 2 * k + 1, tmp, s);
+    SPJ_CUDA(cudaMemcpyAsync(h.data(), cnt.get(), h.size() * 8, cudaMemcpyDeviceToHost, s));
+    SPJ_CUDA(cudaStreamSynchronize(s));
+    for (uint32_t k = 0; k < n_cols; k++) {
+      cols[k].null_count = h[2 * k];
+      cols[k].out_bytes = h[2 * k + 1];
+    }
+    g_error.clear();
+    return 0;
+  } catch (const std::exception& e) {
+    return fail(e);
+  }
+}
+
+extern "C" int SpjGatherColumnsData(const SpjGatherColumn* cols, uint32_t n_cols, void* stream) {
+  try {
+    SPJ_CHECK(n_cols == 0 || cols != nullptr, "null columns");
+    const cudaStream_t s = as_stream(stream);
+    for (uint32_t k = 0; k < n_cols; k++) {
+      const SpjGatherColumn& c = cols[k];
+      if (!c.d_offsets || !c.n || !c.out_bytes) continue;
+      SPJ_CHECK(c.d_out_data != nullptr && c.d_data != nullptr, "null data buffer");
+      copy_values(c.d_offsets, c.offsets_are_64bit != 0, c.d_data, c.n_values, c.d_idx, c.n,
+                  c.d_out_offsets, c.out_bytes, c.d_out_data, c.out_bytes, s);
+    }
     SPJ_CUDA(cudaStreamSynchronize(s));
     g_error.clear();
     return 0;

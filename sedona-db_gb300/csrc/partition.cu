@@ -471,7 +471,7 @@ void column_boxes(const ColumnAccess& a, DevBuf& boxes, bool expand, double dist
 // column: read by the device from host memory, or gathered by host threads
 // into page-locked memory and copied.
 struct RowGather {
-  DevBuf off, data, len, pos, tmp;
+  DevBuf off, data, len, tmp;
   PinnedBuf hdata, hoff;
   size_t hdata_cap = 0, hoff_cap = 0;
   std::vector<uint32_t> hidx;
@@ -481,7 +481,7 @@ struct RowGather {
     c.n = (int64_t)n;
     c.offsets64 = true;
     if (a.direct) {
-      c.data_len = gather_binary(a.whole(), d_idx, n, off, data, len, pos, tmp, s);
+      c.data_len = gather_binary(a.whole(), d_idx, n, off, data, len, tmp, s);
       c.offsets = off.get();
       c.data = data.as<uint8_t>();
       return c;

@@ -119,4 +119,38 @@ __device__ __forceinline__ void group_copy(const uint8_t* __restrict__ src,
   if (t0 + gl < l) dst[t0 + gl] = src[t0 + gl];
 }
 
+// The same with all of a value's first G * U words, its head and its tail
+// loaded before anything is stored, so that a value of up to G * U * 4 bytes
+// costs one memory latency; the rest of a longer one follows by group_copy.
+template <int G, int U>
+__device__ __forceinline__ void group_copy_once(const uint8_t* __restrict__ src,
+                                                uint8_t* __restrict__ dst, uint32_t l, int gl) {
+  static_assert(G >= 4, "head and tail bytes take one lane each");
+  const uint32_t head = min(l, (0u - (uint32_t)reinterpret_cast<uintptr_t>(dst)) & 3u);
+  const uint32_t words = (l - head) >> 2, t0 = head + words * 4u + gl;
+  const uint8_t hb = (uint32_t)gl < head ? src[gl] : 0, tb = t0 < l ? src[t0] : 0;
+  const uintptr_t sa = reinterpret_cast<uintptr_t>(src + head);
+  const uint32_t sh = (uint32_t)(sa & 3) * 8;
+  const uint32_t* sw = reinterpret_cast<const uint32_t*>(sa & ~uintptr_t(3));
+  uint32_t lo[U], hi[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const uint32_t w = u * G + gl;
+    lo[u] = w < words ? sw[w] : 0u;
+    hi[u] = w < words && sh ? sw[w + 1] : 0u;
+  }
+  if ((uint32_t)gl < head) dst[gl] = hb;
+  if (t0 < l) dst[t0] = tb;
+  uint32_t* dw = reinterpret_cast<uint32_t*>(dst + head);
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const uint32_t w = u * G + gl;
+    if (w < words) dw[w] = __funnelshift_r(lo[u], hi[u], sh);
+  }
+  if (words > G * U) {
+    const uint32_t done = head + G * U * 4;
+    group_copy<G>(src + done, dst + done, (uint64_t)(words - G * U) * 4, gl);
+  }
+}
+
 }  // namespace spj

@@ -21,6 +21,28 @@ pub const SPJ_REFINE_FAST_F32: i32 = 1;
 const ENOSPC: c_int = 28;
 
 #[repr(C)]
+#[derive(Clone, Copy)]
+pub struct SpjGatherColumn {
+    pub d_idx: *const u32,
+    pub n: u64,
+    pub d_offsets: *const c_void,
+    pub d_data: *const u8,
+    pub offsets_are_64bit: i32,
+    pub width: u32,
+    pub d_values: *const c_void,
+    pub n_values: u64,
+    pub d_validity: *const u8,
+    pub validity_offset: i64,
+    pub n_validity: u64,
+    pub d_out_values: *mut c_void,
+    pub d_out_offsets: *mut i64,
+    pub d_out_data: *mut u8,
+    pub d_out_validity: *mut u8,
+    pub out_bytes: u64,
+    pub null_count: u64,
+}
+
+#[repr(C)]
 pub struct SpjJoinConfig {
     pub runtime: *const GpuSpatialRuntime,
     pub leaf_size: u32,
@@ -414,6 +436,16 @@ extern "C" {
         d_out_data: *mut u8,
         capacity: u64,
         out_bytes: *mut u64,
+        stream: *mut c_void,
+    ) -> c_int;
+    pub fn SpjGatherColumns(
+        cols: *mut SpjGatherColumn,
+        n_cols: u32,
+        stream: *mut c_void,
+    ) -> c_int;
+    pub fn SpjGatherColumnsData(
+        cols: *const SpjGatherColumn,
+        n_cols: u32,
         stream: *mut c_void,
     ) -> c_int;
     pub fn SpjVisitedMark(

@@ -153,6 +153,16 @@ class SpjHostWkb(C.Structure):
                 ("data", C.c_void_p), ("validity", C.c_void_p), ("validity_offset", C.c_int64)]
 
 
+class SpjGatherColumn(C.Structure):
+    _fields_ = [("d_idx", C.c_void_p), ("n", C.c_uint64), ("d_offsets", C.c_void_p),
+                ("d_data", C.c_void_p), ("offsets_are_64bit", C.c_int32), ("width", C.c_uint32),
+                ("d_values", C.c_void_p), ("n_values", C.c_uint64), ("d_validity", C.c_void_p),
+                ("validity_offset", C.c_int64), ("n_validity", C.c_uint64),
+                ("d_out_values", C.c_void_p), ("d_out_offsets", C.c_void_p),
+                ("d_out_data", C.c_void_p), ("d_out_validity", C.c_void_p),
+                ("out_bytes", C.c_uint64), ("null_count", C.c_uint64)]
+
+
 class SpjPartitionOptions(C.Structure):
     _fields_ = [("num_partitions", C.c_uint32), ("sample_rows", C.c_uint32),
                 ("build_budget_bytes", C.c_uint64), ("seed", C.c_uint64),
@@ -184,7 +194,7 @@ EXPORTS = [
     "SpjKnnStream", "SpjKnnGetStats", "SpjHostRegister", "SpjHostUnregister", "SpjVersion",
     "SpjIndexProbeNoAlloc", "SpjAllocationCount",
     "SpjMaterializeLastError", "SpjGatherFixed", "SpjGatherValidity", "SpjGatherBinary",
-    "SpjVisitedMark", "SpjVisitedCollect",
+    "SpjGatherColumns", "SpjGatherColumnsData", "SpjVisitedMark", "SpjVisitedCollect",
     "SpjJoinPartitioned", "SpjJoinPartitionLayout",
     "SpjParquetOpen", "SpjParquetRelease", "SpjParquetLastError", "SpjParquetInfo",
     "SpjParquetColumnName", "SpjParquetRowGroupRows", "SpjParquetReadWkb", "SpjParquetGetStats", "SpjParquetGetPhases",
@@ -287,6 +297,8 @@ def lib() -> C.CDLL:
             L.SpjGatherBinary.argtypes = [C.c_void_p, C.c_int32, C.c_void_p, C.c_uint64,
                                           C.c_void_p, C.c_uint64, C.c_void_p, C.c_void_p,
                                           C.c_uint64, C.POINTER(C.c_uint64), C.c_void_p]
+            for f in (L.SpjGatherColumns, L.SpjGatherColumnsData):
+                f.argtypes = [C.POINTER(SpjGatherColumn), C.c_uint32, C.c_void_p]
             L.SpjVisitedMark.argtypes = [C.c_void_p, C.c_uint64, C.c_void_p, C.c_uint64,
                                          C.c_void_p]
             L.SpjVisitedCollect.argtypes = [C.c_void_p, C.c_uint64, C.c_int32, C.c_void_p,

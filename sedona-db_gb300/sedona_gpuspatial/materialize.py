@@ -21,7 +21,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from .capi import GpuSpatialError, lib
+from .capi import GpuSpatialError, SpjGatherColumn, lib
 
 NULL_INDEX = -1  # 0xFFFFFFFF as uint32
 ENOSPC = 28
@@ -119,24 +119,67 @@ def take_binary(offsets: torch.Tensor, data: torch.Tensor,
     return out_off, out
 
 
+def _take_all(items):
+    """take() of (column, index) pairs, the columns together: the values,
+    lengths and validity words of all of them, then the bytes of the binary
+    ones once their sizes are known."""
+    if not items:
+        return []
+    args = (SpjGatherColumn * len(items))()
+    outs, keep = [], []
+    for a, (col, idx) in zip(args, items):
+        idx = _index(idx)
+        n, dev = idx.numel(), idx.device
+        out = DeviceColumn(n)
+        words = torch.empty(((n + 31) // 32,), dtype=torch.int32, device=dev)
+        if col.is_binary:
+            if col.offsets.dtype not in (torch.int32, torch.int64):
+                raise GpuSpatialError("binary offsets are int32 or int64")
+            src = col.offsets.contiguous()
+            out.offsets = torch.empty((n + 1,), dtype=torch.int64, device=dev)
+            a.d_offsets, a.d_data = _ptr(src), _ptr(col.data)
+            a.offsets_are_64bit = int(src.dtype == torch.int64)
+            a.n_values = src.numel() - 1
+            a.d_out_offsets = _ptr(out.offsets)
+        else:
+            src = col.values.contiguous()
+            a.width = src.element_size()
+            for d in src.shape[1:]:
+                a.width *= d
+            out.values = torch.empty((n,) + tuple(src.shape[1:]), dtype=src.dtype, device=dev)
+            a.d_values, a.n_values = _ptr(src), src.shape[0]
+            a.d_out_values = _ptr(out.values)
+        a.d_idx, a.n = _ptr(idx), n
+        a.d_validity, a.validity_offset = _ptr(col.validity), col.validity_offset
+        a.n_validity = col.length
+        a.d_out_validity = _ptr(words)
+        out.validity = words.view(torch.uint8)
+        outs.append(out)
+        keep.append((idx, src))
+    s = _stream(keep[0][0])
+    _check(lib().SpjGatherColumns(args, len(items), s), "gather")
+    for a, out in zip(args, outs):
+        out.null_count = int(a.null_count)
+        if out.is_binary:
+            out.data = torch.empty((int(a.out_bytes),), dtype=torch.uint8,
+                                   device=out.offsets.device)
+            a.d_out_data = _ptr(out.data)
+    if any(a.out_bytes for a in args):
+        _check(lib().SpjGatherColumnsData(args, len(items), s), "gather binary")
+    return outs
+
+
 def take(col: DeviceColumn, idx: torch.Tensor) -> DeviceColumn:
     """Arrow ``take`` of one column by an index array with nulls."""
-    if col.is_binary:
-        off, data = take_binary(col.offsets, col.data, idx)
-        out = DeviceColumn(idx.numel(), offsets=off, data=data)
-    else:
-        out = DeviceColumn(idx.numel(), values=take_fixed(col.values, idx))
-    out.validity, out.null_count = take_validity(col.validity, col.validity_offset,
-                                                 col.length, idx)
-    return out
+    return _take_all([(col, idx)])[0]
 
 
 def build_joined_columns(build_cols, probe_cols, build_idx: torch.Tensor,
                          probe_idx: torch.Tensor):
     """The output columns of one joined batch, build side first then probe
     side (build_batch_from_indices with every column projected)."""
-    return ([take(c, build_idx) for c in build_cols] +
-            [take(c, probe_idx) for c in probe_cols])
+    return _take_all([(c, build_idx) for c in build_cols] +
+                     [(c, probe_idx) for c in probe_cols])
 
 
 class VisitedBitmap:
@@ -156,16 +199,19 @@ class VisitedBitmap:
         left anti and full joins), ascending, as int32."""
         count = C.c_uint64(0)
         s = _stream(self.words)
-        rc = lib().SpjVisitedCollect(_ptr(self.words), self.n_rows, int(visited), None, 0,
+        # room for all rows where that is little memory, else their count first
+        cap = self.n_rows if self.n_rows <= (1 << 22) else 0
+        out = torch.empty((cap,), dtype=torch.int32, device=self.words.device)
+        rc = lib().SpjVisitedCollect(_ptr(self.words), self.n_rows, int(visited), _ptr(out), cap,
                                      C.byref(count), s)
         if rc not in (0, ENOSPC):
             _check(rc, "visited collect")
-        out = torch.empty((int(count.value),), dtype=torch.int32, device=self.words.device)
-        if out.numel():
+        if rc == ENOSPC:
+            out = torch.empty((int(count.value),), dtype=torch.int32, device=self.words.device)
             _check(lib().SpjVisitedCollect(_ptr(self.words), self.n_rows, int(visited),
                                            _ptr(out), out.numel(), C.byref(count), s),
                    "visited collect")
-        return out
+        return out[:int(count.value)]
 
     def bitmap(self) -> torch.Tensor:
         """The mark column of a mark join: Arrow LSB bits, one per row."""

@@ -212,3 +212,45 @@ def test_joined_batch_and_left_outer_join(mat, oracle_lib):
     assert tail[1].null_count == un.numel()
     assert int(tail[1].offsets[-1]) == 0
     del keep
+
+
+@pytest.mark.parametrize("n", [0, 1, 31, 127, 128, 129, 5000])
+@pytest.mark.parametrize("mean", [3, 32, 36, 180, 900])
+def test_columns_together_as_one_by_one(mat, n, mean):
+    """A batch of more columns than one launch takes, of every width, with and
+    without validity, and values on both sides of the copies' limits, against
+    the gathers of single columns."""
+    import torch
+    rng = np.random.default_rng(n + mean)
+    nv, npr = 777, 1501
+    bi, pi = (_t(_idx(rng, n, m).view(np.int32)) for m in (nv, npr))
+
+    def column(rows, k):
+        valid = _t(rng.integers(0, 256, (rows + 20) // 8 + 1, dtype=np.uint8)) if k % 2 else None
+        if k < 5:
+            w = 1 << k
+            vals = rng.integers(0, 256, (rows, w), dtype=np.uint8)
+            return mat.DeviceColumn(rows, values=_t(vals), validity=valid, validity_offset=k)
+        lens = rng.integers(0, 2 * mean + 1, rows)
+        if k == 6:
+            lens[rows // 2:] = 0
+        off = np.zeros(rows + 1, np.int64 if k == 5 else np.int32)
+        np.cumsum(lens, out=off[1:])
+        data = rng.integers(0, 256, int(off[-1]) + 1, dtype=np.uint8)
+        return mat.DeviceColumn(rows, offsets=_t(off), data=_t(data), validity=valid)
+
+    build, probe = [column(nv, k) for k in range(8)], [column(npr, k) for k in range(6)]
+    got = mat.build_joined_columns(build, probe, bi, pi)
+    assert len(got) == 14
+    for c, col, idx in zip(got, build + probe, [bi] * 8 + [pi] * 6):
+        words, nulls = mat.take_validity(col.validity, col.validity_offset, col.length, idx)
+        assert torch.equal(c.validity, words) and c.null_count == nulls and c.length == n
+        if col.is_binary:
+            o, d = mat.take_binary(col.offsets, col.data, idx)
+            assert torch.equal(c.offsets, o) and torch.equal(c.data, d)
+            ii = idx.cpu().numpy().view(np.uint32).astype(np.int64)
+            so, sd = col.offsets.cpu().numpy().astype(np.int64), col.data.cpu().numpy()
+            exp = b"".join(sd[so[r]:so[r + 1]].tobytes() for r in ii if r < len(so) - 1)
+            assert d.cpu().numpy().tobytes() == exp
+        else:
+            assert torch.equal(c.values, mat.take_fixed(col.values, idx))
