@@ -83,15 +83,16 @@ struct PageInfo {
   uint32_t num_values = 0;
   uint32_t lvl_bytes = 0;  // v2: definition + repetition level bytes (never compressed)
   uint32_t def_len = 0;    // v2: definition level bytes
+  uint32_t seg0 = 0;       // the page's first segment (of kSegBytes) in the read
   int32_t dict = -1;       // the chunk's dictionary (index into the dictionary table)
   uint8_t kind = 0;        // 0 dictionary, 1 data v1, 2 data v2
   uint8_t codec = 0;
   uint8_t encoding = 0;
   uint8_t max_def = 0;
   uint8_t in_src = 0;      // not compressed: decoded straight from the staging buffer
-  uint8_t pad[3] = {};
+  uint8_t pad[7] = {};
 };
-static_assert(sizeof(PageInfo) == 56, "PageInfo layout");
+static_assert(sizeof(PageInfo) == 64, "PageInfo layout");
 
 // Walks the page headers of one column chunk held at buf[begin, end) and
 // appends its pages (data pages numbered from *row on).  The chunk's

@@ -17,10 +17,15 @@
 //                  elements cross block ends
 //   k_dict_pages   warp per dictionary page: PLAIN byte arrays -> entries
 //   k_data_pages   warp per data page: RLE / bit-packed definition levels ->
-//                  per-row validity; PLAIN values (equal-length values are
-//                  located in parallel after a parallel check of every length
-//                  word, others by a walk) or dictionary indices -> per-row
-//                  (address, length)
+//                  per-row validity; PLAIN values of equal lengths (located
+//                  in parallel after a parallel check of every length word) or
+//                  dictionary indices -> per-row (address, length)
+//   k_seg_walk     PLAIN values of unequal lengths are a chain of length
+//                  words: warp per 4 KiB segment of a page, from a guess of its
+//                  first value; k_seg_chain: warp per page, which checks each
+//                  guess against the end of the segment before and walks again
+//                  where one was wrong; k_seg_write: the values' spans;
+//                  k_seg_rows: to the rows of pages with nulls
 //   scan           lengths -> int64 offsets
 //   k_copy_values  8 lanes per row, 4 rows at a time per warp: value bytes ->
 //                  the output data buffer
@@ -439,19 +444,52 @@ struct RowArrays {
   unsigned long long* nulls;
 };
 
+// A page's PLAIN values that are left to the segment kernels (m = 0: none):
+// the values' bytes start at vp of the page.
+struct PageWalk {
+  uint32_t vp, m, nulls;
+};
+
+// Rows of a page with nulls: the rank of each valid row among the page's valid
+// rows picks its span.
+__device__ __forceinline__ void page_rows(const PageInfo& pg, const RowArrays& ra) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const uint64_t fr = pg.first_row;
+  const uint32_t nv = pg.num_values;
+  uint32_t base = 0, nnull = 0;
+  for (uint32_t i0 = 0; i0 < nv; i0 += 32) {
+    const uint32_t i = i0 + lane;
+    const bool v = i < nv && ra.valid[fr + i];
+    const unsigned b = __ballot_sync(0xffffffffu, v);
+    if (i < nv) {
+      if (v) {
+        const uint32_t r = base + __popc(b & lt);
+        ra.vptr[fr + i] = ra.tmp_ptr[fr + r];
+        ra.vlen[fr + i] = ra.tmp_len[fr + r];
+      } else {
+        ra.vptr[fr + i] = 0;
+        ra.vlen[fr + i] = 0;
+      }
+    }
+    base += __popc(b);
+    nnull += __popc(__ballot_sync(0xffffffffu, i < nv && !v));
+  }
+  if (lane == 0 && nnull) atomicAdd(ra.nulls, (unsigned long long)nnull);
+}
+
 __global__ void k_data_pages(const PageInfo* __restrict__ pages, uint32_t np,
                              const uint8_t* __restrict__ src, const uint8_t* __restrict__ dst,
                              const uint64_t* __restrict__ dict_base,
                              const uint32_t* __restrict__ dict_n,
                              const uint64_t* __restrict__ dict_ptr,
                              const uint32_t* __restrict__ dict_len, RowArrays ra,
-                             uint32_t* status) {
-  extern __shared__ __align__(16) uint8_t smem[];
+                             PageWalk* __restrict__ walks, uint32_t* status) {
   const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < np; p += nwarps) {
     const PageInfo pg = pages[p];
+    if (lane == 0) walks[p] = PageWalk{0, 0, 0};
     if (pg.kind == 0) continue;
     const uint8_t* raw = page_bytes(pg, src, dst);
     const uint8_t* end = raw + pg.raw_size;
@@ -496,6 +534,10 @@ __global__ void k_data_pages(const PageInfo* __restrict__ pages, uint32_t np,
     const bool all_valid = m == nv;
     uint64_t* tptr = all_valid ? ra.vptr + fr : ra.tmp_ptr + fr;
     uint32_t* tlen = all_valid ? ra.vlen + fr : ra.tmp_len + fr;
+    if (vp > end) {
+      if (lane == 0) set_error(status, kErrLevels, p);
+      continue;
+    }
     if (pg.encoding == kPlain) {
       const uint64_t avail = (uint64_t)(end - vp);
       bool fixed = false;
@@ -513,42 +555,9 @@ __global__ void k_data_pages(const PageInfo* __restrict__ pages, uint32_t np,
             }
         }
       }
-      if (!fixed) {
-        // every lane walks the length words through the warp's window
-        Win w;
-        const uint32_t avail32 = (uint32_t)avail;
-        win_init(w, vp, avail32, smem + (threadIdx.x >> 5) * (kWalkWin + 16), kWalkWin);
-        // lane j keeps the span of value k0 + j of each group of 32 and the
-        // warp stores a group at once (no per-value divergent store)
-        bool good = true;
-        uint32_t q = 0, my_q = 0, my_l = 0;
-        for (uint32_t k = 0; k < m; k++) {
-          if (avail32 - q < 4) {
-            good = false;
-            break;
-          }
-          win_need(w, q, 4);
-          const uint32_t l = win_u32(w, q);
-          if (avail32 - q - 4 < l) {
-            good = false;
-            break;
-          }
-          const bool mine = (k & 31) == (uint32_t)lane;
-          my_q = mine ? q + 4 : my_q;
-          my_l = mine ? l : my_l;
-          if ((k & 31) == 31 || k + 1 == m) {
-            const uint32_t k0 = k & ~31u;
-            if (k0 + lane <= k) {
-              tptr[k0 + lane] = reinterpret_cast<uint64_t>(vp + my_q);
-              tlen[k0 + lane] = my_l;
-            }
-          }
-          q += 4 + l;
-        }
-        if (!good) {
-          if (lane == 0) set_error(status, kErrPlain, p);
-          continue;
-        }
+      if (!fixed) {  // (m = 0: nothing to find)
+        if (lane == 0) walks[p] = PageWalk{(uint32_t)(vp - raw), m, all_valid ? 0u : 1u};
+        if (m) continue;
       }
     } else {
       // dictionary indices: a bit-width byte, then the hybrid runs
@@ -579,31 +588,197 @@ __global__ void k_data_pages(const PageInfo* __restrict__ pages, uint32_t np,
     }
     if (all_valid) continue;
     __syncwarp();
-    // rows: the rank of each valid row among the page's valid rows
-    uint32_t base = 0, nnull = 0;
-    for (uint32_t i0 = 0; i0 < nv; i0 += 32) {
-      const uint32_t i = i0 + lane;
-      const bool v = i < nv && valid[i];
-      const unsigned b = __ballot_sync(0xffffffffu, v);
-      if (i < nv) {
-        if (v) {
-          const uint32_t r = base + __popc(b & lt);
-          ra.vptr[fr + i] = tptr[r];
-          ra.vlen[fr + i] = tlen[r];
-        } else {
-          ra.vptr[fr + i] = 0;
-          ra.vlen[fr + i] = 0;
-        }
+    page_rows(pg, ra);
+  }
+}
+
+// Segments of the PLAIN values' bytes.  A value can only be found from the one
+// before it, so a page's walk was a chain of its length words by one warp
+// (400k polygons in 65 pages: 680 us at 110 ns a value); the segments' walks
+// are short and run together (85 us in all), bound by the latency of their
+// length words.
+constexpr uint32_t kSegBytes = 4096;
+constexpr uint32_t kSegNone = 0xffffffffu;   // no value starts in the segment, as far as known
+constexpr uint32_t kSegStuck = 0xfffffffeu;  // the walk met the end of the page
+struct Segment {
+  uint32_t start, count, exit;  // first value, values, the first value behind it
+};
+
+// u32 at any address (the aligned words that hold its bytes)
+__device__ __forceinline__ uint32_t ld_u32(const uint8_t* p) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
+  const uint32_t sh = (uint32_t)(a & 3) * 8;
+  return __funnelshift_r(w[0], sh ? w[1] : 0u, sh);
+}
+
+// Walks from q to the segment's end at seg_end; each(k, start, length) for its k-th value.
+template <class Each>
+__device__ __forceinline__ Segment seg_walk(const uint8_t* vp, uint32_t avail, uint32_t q,
+                                            uint32_t seg_end, Each&& each) {
+  Segment r{q, 0, q};
+  while (q < seg_end) {
+    if (avail - q < 4) break;
+    const uint32_t l = ld_u32(vp + q);
+    if (avail - q - 4 < l) break;
+    each(r.count, q + 4, l);
+    r.count++;
+    q += 4 + l;
+  }
+  r.exit = q < seg_end ? kSegStuck : q;
+  return r;
+}
+
+// Whether a WKB value may start at q: only a guess, k_seg_chain has the proof.
+__device__ __forceinline__ bool seg_value(const uint8_t* vp, uint32_t avail, uint32_t q,
+                                          uint32_t& next) {
+  if (avail - q < 9) return false;
+  const uint32_t l = ld_u32(vp + q);
+  if (l < 5 || avail - q - 4 < l) return false;
+  const uint8_t order = vp[q + 4];
+  if (order > 1) return false;
+  const uint32_t t = ld_u32(vp + q + 5), type = order ? t : __byte_perm(t, 0, 0x0123);
+  next = q + 4 + l;
+  return type >= 1 && type <= 7;
+}
+
+__device__ __forceinline__ uint32_t seg_page(const PageInfo* pages, uint32_t np, uint32_t seg) {
+  uint32_t lo = 0, hi = np - 1;  // the last page with seg0 <= seg
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi + 1) / 2;
+    if (pages[mid].seg0 <= seg) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+__global__ void __launch_bounds__(256)
+    k_seg_walk(const PageInfo* __restrict__ pages, uint32_t np, uint32_t nseg,
+               const uint8_t* __restrict__ src, const uint8_t* __restrict__ dst,
+               const PageWalk* __restrict__ walks, Segment* __restrict__ segs) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nseg; i += nwarps) {
+    const uint32_t p = seg_page(pages, np, i);
+    const PageWalk w = walks[p];
+    if (w.m == 0) continue;
+    const PageInfo pg = pages[p];
+    const uint8_t* vp = page_bytes(pg, src, dst) + w.vp;
+    const uint32_t avail = pg.raw_size - w.vp, q0 = (i - pg.seg0) * kSegBytes;
+    Segment r{kSegNone, 0, kSegNone};
+    if (q0 < avail) {
+      const uint32_t q1 = min(avail, q0 + kSegBytes);
+      uint32_t start = q0 == 0 ? 0u : kSegNone;
+      for (uint32_t q = q0; start == kSegNone && q < q1; q += 32) {
+        uint32_t next = 0, after = 0;
+        const bool may = q + lane < q1 && seg_value(vp, avail, q + lane, next) &&
+                         (avail - next < 9 || seg_value(vp, avail, next, after));
+        const unsigned who = __ballot_sync(0xffffffffu, may);
+        if (who) start = q + (uint32_t)__ffs(who) - 1;
       }
-      base += __popc(b);
-      nnull += __popc(__ballot_sync(0xffffffffu, i < nv && !v));
+      if (start != kSegNone) r = seg_walk(vp, avail, start, q1, [](uint32_t, uint32_t, uint32_t) {});
     }
-    if (lane == 0 && nnull) atomicAdd(ra.nulls, (unsigned long long)nnull);
+    if (lane == 0) segs[i] = r;
+  }
+}
+
+// Proves a page's segments in order: the first starts with the first value,
+// every other one with the value behind the one before it.  Where the guess
+// was another value the segment is walked again from there.  Leaves each
+// segment's start and, as its count, the values before it (m: past the last).
+__global__ void __launch_bounds__(128)
+    k_seg_chain(const PageInfo* __restrict__ pages, uint32_t np, const uint8_t* __restrict__ src,
+                const uint8_t* __restrict__ dst, const PageWalk* __restrict__ walks,
+                Segment* __restrict__ segs, uint32_t* status) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < np; p += nwarps) {
+    const PageWalk w = walks[p];
+    if (w.m == 0) continue;
+    const PageInfo pg = pages[p];
+    const uint8_t* vp = page_bytes(pg, src, dst) + w.vp;
+    const uint32_t avail = pg.raw_size - w.vp;
+    const uint32_t ns = avail / kSegBytes + 1;  // (the last one may be empty)
+    uint32_t at = 0, before = 0;
+    for (uint32_t s0 = 0; s0 < ns; s0 += 32) {
+      Segment mine{kSegNone, 0, kSegNone};
+      if (s0 + lane < ns) mine = segs[pg.seg0 + s0 + lane];
+      const uint32_t n = min(32u, ns - s0);
+      for (uint32_t k = 0; k < n; k++) {
+        const uint32_t q1 = min(avail, (s0 + k + 1) * kSegBytes);
+        Segment r{__shfl_sync(0xffffffffu, mine.start, k), __shfl_sync(0xffffffffu, mine.count, k),
+                  __shfl_sync(0xffffffffu, mine.exit, k)};
+        const uint32_t start = at, rank = before;
+        if (before < w.m && at < q1) {
+          if (r.start != at)
+            r = seg_walk(vp, avail, at, q1, [](uint32_t, uint32_t, uint32_t) {});
+          before = min(w.m, before + r.count);
+          at = r.exit == kSegStuck ? avail : r.exit;
+          if (r.exit == kSegStuck && before < w.m) {  // no more to be found
+            if (lane == 0) set_error(status, kErrPlain, p);
+            before = w.m;
+          }
+        }
+        if ((uint32_t)lane == k) mine = Segment{start, rank, 0};
+      }
+      if (s0 + lane < ns) segs[pg.seg0 + s0 + lane] = mine;
+    }
+    if (before < w.m && lane == 0) set_error(status, kErrPlain, p);
+  }
+}
+
+__global__ void __launch_bounds__(256)
+    k_seg_write(const PageInfo* __restrict__ pages, uint32_t np, uint32_t nseg,
+                const uint8_t* __restrict__ src, const uint8_t* __restrict__ dst,
+                const PageWalk* __restrict__ walks, const Segment* __restrict__ segs,
+                RowArrays ra) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nseg; i += nwarps) {
+    const uint32_t p = seg_page(pages, np, i);
+    const PageWalk w = walks[p];
+    if (w.m == 0) continue;
+    const PageInfo pg = pages[p];
+    const uint8_t* vp = page_bytes(pg, src, dst) + w.vp;
+    const uint32_t avail = pg.raw_size - w.vp, q0 = (i - pg.seg0) * kSegBytes;
+    if (q0 >= avail) continue;
+    const Segment g = segs[i];
+    const uint32_t q1 = min(avail, q0 + kSegBytes), left = w.m - g.count;
+    if (left == 0 || g.start >= q1) continue;
+    uint64_t* tptr = (w.nulls ? ra.tmp_ptr : ra.vptr) + pg.first_row + g.count;
+    uint32_t* tlen = (w.nulls ? ra.tmp_len : ra.vlen) + pg.first_row + g.count;
+    // lane j keeps the span of value j of each group of 32 and the warp stores
+    // a group at once
+    uint32_t my_q = 0, my_l = 0;
+    const Segment r = seg_walk(vp, avail, g.start, q1, [&](uint32_t k, uint32_t q, uint32_t l) {
+      const bool mine = (k & 31) == (uint32_t)lane;
+      my_q = mine ? q : my_q;
+      my_l = mine ? l : my_l;
+      if ((k & 31) == 31 && (k & ~31u) + lane < left) {
+        tptr[(k & ~31u) + lane] = reinterpret_cast<uint64_t>(vp + my_q);
+        tlen[(k & ~31u) + lane] = my_l;
+      }
+    });
+    const uint32_t k = (r.count & ~31u) + lane;
+    if (k < r.count && k < left) {
+      tptr[k] = reinterpret_cast<uint64_t>(vp + my_q);
+      tlen[k] = my_l;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(128)
+    k_seg_rows(const PageInfo* __restrict__ pages, uint32_t np, const PageWalk* __restrict__ walks,
+               RowArrays ra) {
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < np; p += nwarps) {
+    const PageWalk w = walks[p];
+    if (w.m && w.nulls) page_rows(pages[p], ra);
   }
 }
 
 // A warp takes 32 rows: lane k reads row k's span and output position, then
-// lane groups of 8 copy 4 values at a time (group_copy: whole destination
+// lane groups of 8 copy 4 values at a time (group_copy_once: whole destination
 // words, any alignment).
 __global__ void k_copy_values(const uint64_t* __restrict__ vptr,
                               const uint32_t* __restrict__ vlen,
@@ -626,7 +801,7 @@ __global__ void k_copy_values(const uint64_t* __restrict__ vptr,
       const uint64_t vs = __shfl_sync(0xffffffffu, sp, v + grp);
       const uint64_t vd = __shfl_sync(0xffffffffu, d, v + grp);
       const uint32_t vl = __shfl_sync(0xffffffffu, l, v + grp);
-      if (vl) group_copy<G>(reinterpret_cast<const uint8_t*>(vs), out + vd, vl, gl);
+      if (vl) group_copy_once<G, 7>(reinterpret_cast<const uint8_t*>(vs), out + vd, vl, gl);
     }
   }
 }
@@ -751,7 +926,7 @@ struct SpjParquet {
   uint64_t stage_h_cap = 0;
   DevBuf stage, pages, pagebuf, dict_base, dict_n, dict_ptr, dict_len, valid, tmp_ptr, tmp_len,
       vptr, vlen, pos, scan_tmp, out_off, out_data, out_valid, status, nulls, frag_base, frag_ip,
-      mode, work;
+      mode, work, walks, segs;
   double ms = 0, ms_phase[4] = {};  // H2D, decompress, decode, values
   uint64_t file_bytes = 0, page_bytes = 0, value_bytes = 0;
 
@@ -760,7 +935,7 @@ struct SpjParquet {
     for (DevBuf* b : {&stage, &pages, &pagebuf, &dict_base, &dict_n, &dict_ptr, &dict_len,
                       &valid, &tmp_ptr, &tmp_len, &vptr, &vlen, &pos, &scan_tmp, &out_off,
                       &out_data, &out_valid, &status, &nulls, &frag_base, &frag_ip, &mode,
-                      &work})
+                      &work, &walks, &segs})
       b->release();
     if (stream) {
       cudaStreamSynchronize(stream);
@@ -1026,11 +1201,14 @@ extern "C" int SpjParquetReadWkb(SpjParquet* p, const char* column, int32_t rg_b
                                         " values, the row groups " +
                                         std::to_string(rows_expected) + " rows");
     const uint64_t n = row;
-    uint64_t dst = 0, dict_total = 0, pbytes = 0;
+    uint64_t dst = 0, dict_total = 0, pbytes = 0, nseg = 0;
     std::vector<uint64_t> dict_base(ndict + 1, 0);
     std::vector<uint32_t> dict_n(ndict + 1, 0);
     for (auto& pg : pages) {
       pbytes += pg.raw_size;
+      pg.seg0 = (uint32_t)nseg;
+      if (pg.kind != 0 && pg.encoding == kPlain) nseg += pg.raw_size / kSegBytes + 1;
+      SPJ_CHECK(nseg < (1ull << 31), "more than 2^31 segments in one read");
       if (!pg.in_src) {
         pg.dst = dst;
         dst += (pg.raw_size + 15) & ~15ull;
@@ -1174,6 +1352,8 @@ extern "C" int SpjParquetReadWkb(SpjParquet* p, const char* column, int32_t rg_b
     p->vlen.reserve(4 * (n + 1), s);
     p->pos.reserve(8 * (n + 1), s);
     p->out_off.reserve(8 * (n + 1), s);
+    p->walks.reserve(sizeof(PageWalk) * (np + 1), s);
+    p->segs.reserve(sizeof(Segment) * (nseg + 1), s);
     p->status.reserve(8, s);
     p->nulls.reserve(8, s);
     SPJ_CUDA(cudaMemsetAsync(p->status.get(), 0, 8, s));
@@ -1200,8 +1380,6 @@ extern "C" int SpjParquetReadWkb(SpjParquet* p, const char* column, int32_t rg_b
     if (np) {
       SPJ_CUDA(cudaFuncSetAttribute(k_dict_pages, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     walk_smem));
-      SPJ_CUDA(cudaFuncSetAttribute(k_data_pages, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    walk_smem));
       if (ndict)
         k_dict_pages<<<g, kWalkThreads, walk_smem, s>>>(dpages, np, dsrc, dpb,
                                                p->dict_base.as<uint64_t>(),
@@ -1210,9 +1388,19 @@ extern "C" int SpjParquetReadWkb(SpjParquet* p, const char* column, int32_t rg_b
       RowArrays ra{p->valid.as<uint8_t>(),    p->tmp_ptr.as<uint64_t>(),
                    p->tmp_len.as<uint32_t>(), p->vptr.as<uint64_t>(),
                    p->vlen.as<uint32_t>(),    p->nulls.as<unsigned long long>()};
-      k_data_pages<<<g, kWalkThreads, walk_smem, s>>>(dpages, np, dsrc, dpb, p->dict_base.as<uint64_t>(),
-                                     p->dict_n.as<uint32_t>(), p->dict_ptr.as<uint64_t>(),
-                                     p->dict_len.as<uint32_t>(), ra, st);
+      PageWalk* walks = p->walks.as<PageWalk>();
+      k_data_pages<<<grid_for((int64_t)np * 32, 128, kNumSMs * 16), 128, 0, s>>>(
+          dpages, np, dsrc, dpb, p->dict_base.as<uint64_t>(), p->dict_n.as<uint32_t>(),
+          p->dict_ptr.as<uint64_t>(), p->dict_len.as<uint32_t>(), ra, walks, st);
+      if (nseg) {
+        Segment* segs = p->segs.as<Segment>();
+        const int gp = grid_for((int64_t)np * 32, 128, kNumSMs * 16);
+        const int gs = grid_for((int64_t)nseg * 32, 256, kNumSMs * 16);
+        k_seg_walk<<<gs, 256, 0, s>>>(dpages, np, (uint32_t)nseg, dsrc, dpb, walks, segs);
+        k_seg_chain<<<gp, 128, 0, s>>>(dpages, np, dsrc, dpb, walks, segs, st);
+        k_seg_write<<<gs, 256, 0, s>>>(dpages, np, (uint32_t)nseg, dsrc, dpb, walks, segs, ra);
+        k_seg_rows<<<gp, 128, 0, s>>>(dpages, np, walks, ra);
+      }
       SPJ_CUDA(cudaGetLastError());
     }
     SPJ_CUDA(cudaEventRecord(p->ev[3], s));

@@ -155,3 +155,40 @@ def test_device_matches_oracle(gp, oracle_lib, tmp_path, page_version):
     with gp.GeoParquetFile(path) as f:
         got = gp.device_to_host(f.read_wkb())
     _assert_column(got, off, data, valid)
+
+
+@pytest.mark.parametrize("compression", ["snappy", "none"])
+@pytest.mark.parametrize("kind", ["ragged", "decoys", "long", "mixed"])
+def test_plain_values_of_unequal_lengths(gp, tmp_path, compression, kind):
+    """The values' segments: starts that no guess finds (empty values, bytes
+    that are no WKB), values that hold what looks like other values, values
+    longer than a segment, pages of one value, nulls."""
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(len(kind))
+    real = wkb.wkb_polygon([np.array([(0, 0), (3, 1), (2, 5), (0, 0)], np.float64)])
+
+    def value(i):
+        k = kind if kind != "mixed" else ["ragged", "decoys", "long", "real"][int(rng.integers(4))]
+        if k == "ragged":
+            return rng.integers(0, 256, int(rng.integers(0, 40)), dtype=np.uint8).tobytes()
+        if k == "decoys":
+            piece = len(real).to_bytes(4, "little") + real
+            return rng.integers(0, 256, int(rng.integers(0, 9)), dtype=np.uint8).tobytes() + \
+                piece * int(rng.integers(0, 60))
+        if k == "long":
+            return b"\x01" * int(rng.choice([0, 1, 4092, 4096, 4100, 30000]))
+        return real
+    n = 3000 if kind != "long" else 400
+    vals = [value(i) for i in range(n)]
+    off = np.zeros(n + 1, np.int64)
+    off[1:] = np.cumsum([len(v) for v in vals])
+    data = np.frombuffer(b"".join(vals), np.uint8)
+    for nulls in (False, True):
+        valid = rng.random(n) > 0.2 if nulls else np.ones(n, bool)
+        c = wkb.WkbColumn(off, data, np.packbits(valid, bitorder="little") if nulls else None)
+        path = str(tmp_path / "seg.parquet")
+        gp.write_wkb(path, c, compression=compression, row_group_rows=n // 2 + 1,
+                     page_bytes=1 << 15)
+        with gp.GeoParquetFile(path) as f:
+            got = gp.device_to_host(f.read_wkb())
+        _assert_column(got, off, data[np.repeat(valid, np.diff(off))], valid)
