@@ -116,6 +116,7 @@ int rt_init(GpuSpatialRuntime* self, GpuSpatialRuntimeConfig* config) {
 void rt_release(GpuSpatialRuntime* self) {
   delete static_cast<RuntimeData*>(self->private_data);
   self->private_data = nullptr;
+  pinned_trim();
 }
 
 const char* rt_error(GpuSpatialRuntime* self) {
@@ -1544,6 +1545,75 @@ extern "C" const char* SpjVersion(void) { return "spj-gb300 0.1.0 (sm_103a)"; }
 
 namespace spj {
 std::atomic<uint64_t> g_allocations{0};
+
+namespace {
+struct PinnedPool {
+  struct Block {
+    void* p;
+    size_t n;
+  };
+  std::mutex mu;
+  std::vector<Block> free;  // in the order they were given
+  size_t held = 0;
+};
+PinnedPool& pinned_pool() {
+  static PinnedPool* pool = new PinnedPool;  // (the process's end unlocks what it holds)
+  return *pool;
+}
+}  // namespace
+
+void* pinned_take(size_t& bytes) {
+  PinnedPool& pool = pinned_pool();
+  {
+    std::lock_guard<std::mutex> lk(pool.mu);
+    auto best = pool.free.end();
+    for (auto it = pool.free.begin(); it != pool.free.end(); ++it)
+      if (it->n >= bytes && (best == pool.free.end() || it->n < best->n)) best = it;
+    if (best != pool.free.end()) {
+      void* p = best->p;
+      bytes = best->n;
+      pool.held -= best->n;
+      pool.free.erase(best);
+      return p;
+    }
+  }
+  void* p = nullptr;
+  if (cudaMallocHost(&p, bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    pinned_trim();
+    SPJ_CUDA(cudaMallocHost(&p, bytes));
+  }
+  g_allocations.fetch_add(1, std::memory_order_relaxed);
+  return p;
+}
+
+void pinned_give(void* p, size_t bytes) {
+  PinnedPool& pool = pinned_pool();
+  std::vector<void*> out;
+  {
+    std::lock_guard<std::mutex> lk(pool.mu);
+    pool.free.push_back({p, bytes});
+    pool.held += bytes;
+    while (pool.held > kPinnedHeld) {
+      out.push_back(pool.free.front().p);
+      pool.held -= pool.free.front().n;
+      pool.free.erase(pool.free.begin());
+    }
+  }
+  for (void* q : out) cudaFreeHost(q);
+}
+
+void pinned_trim() {
+  PinnedPool& pool = pinned_pool();
+  std::vector<PinnedPool::Block> out;
+  {
+    std::lock_guard<std::mutex> lk(pool.mu);
+    out.swap(pool.free);
+    pool.held = 0;
+  }
+  for (auto& b : out) cudaFreeHost(b.p);
+}
+
 }  // namespace spj
 
 extern "C" uint64_t SpjAllocationCount(void) {

@@ -922,8 +922,7 @@ struct SpjParquet {
   int device = -1;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[6] = {};  // start, after H2D, after Snappy, after decode, values start, end
-  PinnedBuf stage_h;
-  uint64_t stage_h_cap = 0;
+  PinnedBlock stage_h;  // (returned after release_device has waited for the stream)
   DevBuf stage, pages, pagebuf, dict_base, dict_n, dict_ptr, dict_len, valid, tmp_ptr, tmp_len,
       vptr, vlen, pos, scan_tmp, out_off, out_data, out_valid, status, nulls, frag_base, frag_ip,
       mode, work, walks, segs;
@@ -1153,9 +1152,9 @@ extern "C" int SpjParquetReadWkb(SpjParquet* p, const char* column, int32_t rg_b
       rows_expected += (uint64_t)m.row_groups[g].num_rows;
     }
     SPJ_CHECK(rows_expected < (1ull << 32), "more than 2^32 - 1 rows in one read");
-    if (total + 16 > p->stage_h_cap) {
+    if (total + 16 > p->stage_h.size()) {
+      SPJ_CUDA(cudaStreamSynchronize(s));  // (a read that failed may have left a copy in flight)
       p->stage_h.reserve(total + 16);
-      p->stage_h_cap = total + 16;
     }
     uint8_t* hb = p->stage_h.as<uint8_t>();
     p->file_bytes = total;

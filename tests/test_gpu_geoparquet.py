@@ -192,3 +192,37 @@ def test_plain_values_of_unequal_lengths(gp, tmp_path, compression, kind):
         with gp.GeoParquetFile(path) as f:
             got = gp.device_to_host(f.read_wkb())
         _assert_column(got, off, data[np.repeat(valid, np.diff(off))], valid)
+
+
+def test_files_share_page_locked_blocks(gp, tmp_path):
+    """Threads that open, read and close files of several sizes one after the
+    other: every read has its own bytes."""
+    import threading
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(11)
+    files = []
+    for k, n in enumerate((3, 1000, 40000)):
+        lens = rng.integers(0, 60, n)
+        off = np.zeros(n + 1, np.int64)
+        off[1:] = np.cumsum(lens)
+        data = rng.integers(0, 256, int(off[-1]), dtype=np.uint8)
+        path = str(tmp_path / f"{k}.parquet")
+        gp.write_wkb(path, wkb.WkbColumn(off, data, None))
+        files.append((path, off, data))
+    bad = []
+
+    def work(t):
+        try:
+            for i in range(12):
+                path, off, data = files[(t + i) % len(files)]
+                with gp.GeoParquetFile(path) as f:
+                    got = gp.device_to_host(f.read_wkb())
+                _assert_column(got, off, data, np.ones(len(off) - 1, bool))
+        except BaseException as e:  # noqa: BLE001
+            bad.append(e)
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad[0]
