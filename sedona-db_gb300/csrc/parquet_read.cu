@@ -206,6 +206,8 @@ constexpr uint32_t kFragBytes = 1u << 16;  // Snappy's compression block
 constexpr uint64_t kHeaderWindow = 4096;   // bytes read per page header from the file
 constexpr uint64_t kReadGroup = 4ull << 20;  // bytes of whole pages per reader-thread read
 constexpr uint32_t kFragWin = 2048;        // per warp, k_snappy_frags (headers, literals)
+constexpr uint32_t kFragRing = 8192;       // per warp, k_snappy_frags (output)
+constexpr uint32_t kFragSmem = kFragWin + 16 + kFragRing;
 constexpr uint32_t kWalkWin = 16384;       // per warp, PLAIN walks
 constexpr int kWalkThreads = 128;          // 4 walking warps per block
 enum PageMode : uint8_t { kModeStored = 0, kModeFragments = 1, kModeSequential = 2, kModeBad = 3 };
@@ -253,7 +255,10 @@ __device__ __forceinline__ bool snappy_header(Win& w, uint32_t ip, uint32_t& len
 // Warp per 64 KiB output block of a block-independent page: element
 // headers and literal bytes through a shared-memory window of the input
 // (restaged a window at a time, so an element does not wait on a global
-// load), copies from the block's own output, all by the 32 lanes.  A copy
+// load), copies from the block's own output, all by the 32 lanes.  The last
+// kFragRing output bytes are kept in shared memory, where most copies find
+// their source without waiting for its bytes to come back from L2.  Bound by the chain of element headers (400k polygons,
+// 700 blocks at once: 590 us, 466 with the ring).  A copy
 // that reaches before its block sends the page to k_snappy_pages.  Work item
 // (page, block 0) also copies a v2 page's level bytes.
 __global__ void __launch_bounds__(128) k_snappy_frags(
@@ -280,8 +285,8 @@ __global__ void __launch_bounds__(128) k_snappy_frags(
     const uint32_t fl = min(kFragBytes, out_n - f0);
     const uint8_t* in = in0 + pg.lvl_bytes;
     uint8_t* out = out0 + pg.lvl_bytes + f0;
-    win_init(w, in, pg.src_size - pg.lvl_bytes, smem + (threadIdx.x >> 5) * (kFragWin + 16),
-             kFragWin);
+    uint8_t* ring = smem + (threadIdx.x >> 5) * kFragSmem;
+    win_init(w, in, pg.src_size - pg.lvl_bytes, ring + kFragRing, kFragWin);
     uint32_t ip = frag_ip[frag_base[p] + k], op = 0;
     bool ok = true, local = true;
     while (op < fl) {
@@ -297,7 +302,11 @@ __global__ void __launch_bounds__(128) k_snappy_frags(
           const uint32_t piece = min(len - done, kFragWin - 16);
           win_need(w, ip + hdr + done, piece);
           const uint8_t* s = w.buf + (ip + hdr + done - w.p0);
-          for (uint32_t i = lane; i < piece; i += 32) out[op + done + i] = s[i];
+          for (uint32_t i = lane; i < piece; i += 32) {
+            const uint8_t v = s[i];
+            out[op + done + i] = v;
+            ring[(op + done + i) % kFragRing] = v;
+          }
           done += piece;
         }
       } else {
@@ -305,11 +314,17 @@ __global__ void __launch_bounds__(128) k_snappy_frags(
           local = false;
           break;
         }
-        const uint8_t* s = out + op - off;
-        if (off >= len) {
-          for (uint32_t i = lane; i < len; i += 32) out[op + i] = s[i];
-        } else {
-          for (uint32_t i = lane; i < len; i += 32) out[op + i] = s[i % off];
+        // a copy has at most 64 bytes: two per lane, whose sources lie before
+        // op and, in the ring, in other places than op .. op + len
+        const bool near = off + 64 <= kFragRing;
+#pragma unroll
+        for (uint32_t i = lane; i < 64; i += 32) {
+          if (i < len) {
+            const uint32_t from = op - off + (off >= len ? i : i % off);
+            const uint8_t v = near ? ring[from % kFragRing] : out[from];
+            out[op + i] = v;
+            ring[(op + i) % kFragRing] = v;
+          }
         }
       }
       __syncwarp();  // the bytes just written may be the next copy's source
@@ -1365,7 +1380,7 @@ extern "C" int SpjParquetReadWkb(SpjParquet* p, const char* column, int32_t rg_b
       // Snappy: block-parallel decode, then the pages that are not
       // block-independent
       k_snappy_frags<<<grid_for((int64_t)nwork * 32, 128, kNumSMs * 16), 128,
-                       4 * (kFragWin + 16), s>>>(
+                       4 * kFragSmem, s>>>(
           dpages, p->work.as<uint2>(), nwork, dsrc, dpb, p->frag_base.as<uint64_t>(),
           p->frag_ip.as<uint32_t>(), p->mode.as<uint8_t>(), st);
       k_snappy_pages<<<grid_for((int64_t)np * 32, 128, kNumSMs * 16), 128, 0, s>>>(
