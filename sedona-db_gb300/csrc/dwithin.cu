@@ -286,8 +286,8 @@ __global__ void __launch_bounds__(kTravThreads)
 // pairs in traversal order, so that nothing is traversed twice.  One
 // traversal per probe was bound by divergence and by its node loads, and the
 // probes with over 64 neighbours were traversed again: 4M x 400k clustered
-// points: 7.5 ms with its second traversal and copies, 2.3 ms this way (1.6
-// here, 0.1 the packets, 0.6 the pairs); FP32 operations bound it now.
+// points: 7.5 ms with its second traversal and copies, 2.2 ms this way (1.6
+// here, 0.1 the packets, 0.5 the pairs); FP32 operations bound it now.
 __global__ void __launch_bounds__(kTravThreads, 8)
     k_dwithin_packet(LbvhView t, const double2* __restrict__ bxy, const float4* __restrict__ bhl,
                      float bmag, int split_ok, const float4* __restrict__ probe_box,

@@ -23,9 +23,9 @@
 // the masks into pairs; records are in traversal order, so every probe row's
 // pairs come in the order of the candidate pairs' path.
 //
-// 2M buildings x 50k zones, ST_Intersects: 40.5 -> 19.1 ms a step (refine 28.5,
+// 2M buildings x 50k zones, ST_Intersects: 40.5 -> 18.2 ms a step (refine 28.5,
 // traversal 3.6, ordering and compaction of 132M pairs 4.9 before; k_packet
-// 9.5, k_packet_open 7.0, k_packet_scatter 0.5 now); 2M points x 50k zones:
+// 9.5, k_packet_open 7.0, k_packet_scatter 0.4 now); 2M points x 50k zones:
 // 15.7 -> 5.6 ms; 300k buildings in 20k holed zones: 17.4 -> 4.0 ms.  k_packet
 // is bound by its instructions (some 1,000 per packet and build row, from a
 // loop body larger than the instruction cache) and by the latency of the
@@ -980,13 +980,30 @@ __global__ void __launch_bounds__(kPacketThreads)
   flush_counters(st, esc, 0);
 }
 
-// A warp per packet: 32 records at a time, one per lane; for each probe the
-// lanes whose record holds its bit write its next pairs, side by side.
-__global__ void __launch_bounds__(256)
+// Lane l's bit i of the result: lane i's bit l of x (five exchanges of halves).
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
+  uint32_t m = 0x0000ffffu;
+#pragma unroll
+  for (int j = 16; j; j >>= 1, m ^= m << j) {
+    const uint32_t y = __shfl_xor_sync(kAll, x, j);
+    x = (lane & j) ? (x & ~m) | ((y & ~m) >> j) : (x & m) | ((y & m) << j);
+  }
+  return x;
+}
+
+// A warp per packet: 64 records at a time, two per lane, whose lane masks are
+// transposed into each probe's mask of records; then for each probe the lanes
+// whose record has it write its next pairs, side by side.  Bound by its
+// instructions (98M pairs of 4M points: 629 us with 32 records at a time, a
+// ballot for each probe and 64-bit positions, SCATTER_US this way; Pos: 32 bits
+// where the output has fewer places).  A block takes 4 packets and the next
+// block the next ones, as a dense packet has many times another's records.
+template <class Pos>
+__global__ void __launch_bounds__(128)
     k_packet_scatter(uint32_t n, const uint32_t* __restrict__ order,
                      const uint64_t* __restrict__ offs, uint32_t probe_base, PacketStore A,
                      uint32_t* __restrict__ out_build, uint32_t* __restrict__ out_probe,
-                     uint64_t cap) {
+                     Pos cap) {
   const int lane = threadIdx.x & 31;
   const uint32_t lower = (1u << lane) - 1u;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -994,24 +1011,36 @@ __global__ void __launch_bounds__(256)
   for (uint64_t g = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; g < npackets; g += nw) {
     const uint2 run = A.packets[g];
     const uint32_t pi = (uint32_t)lane < run.y ? order[run.x + lane] : n;
-    uint64_t pos = pi < n ? offs[pi] : 0;
+    // (past the output: at its end)
+    Pos pos = pi < n ? (Pos)min(offs[pi], (uint64_t)cap) : cap;
     const uint32_t nrec = A.nrec[g];
     uint32_t chunk = nrec ? A.head[g] : kNoChunk;
-    for (uint32_t r0 = 0; r0 < nrec && chunk < A.chunks; r0 += 32) {
-      uint2 rec = make_uint2(0u, 0u);
-      if (r0 + lane < nrec) rec = A.rec[(uint64_t)chunk * 32 + lane];
-      if (r0 + 32 < nrec) chunk = A.next[chunk];
-      for (int l = 0; l < 32; l++) {
-        const unsigned bits = __ballot_sync(kAll, (rec.y >> l) & 1u);
-        if (bits == 0) continue;
-        const uint64_t at = __shfl_sync(kAll, pos, l) + __popc(bits & lower);
-        const uint32_t row = __shfl_sync(kAll, pi, l);
-        if (((bits >> lane) & 1u) && at < cap) {
-          out_build[at] = rec.x;
-          out_probe[at] = row + probe_base;
-        }
-        if (lane == l) pos += __popc(bits);
+    for (uint32_t r0 = 0; r0 < nrec && chunk < A.chunks; r0 += 64) {
+      uint2 ra = make_uint2(0u, 0u), rb = ra;
+      if (r0 + lane < nrec) ra = A.rec[(uint64_t)chunk * 32 + lane];
+      if (r0 + 32 < nrec) {
+        chunk = A.next[chunk];
+        if (chunk >= A.chunks) break;
+        if (r0 + 32 + lane < nrec) rb = A.rec[(uint64_t)chunk * 32 + lane];
+        if (r0 + 64 < nrec) chunk = A.next[chunk];
       }
+      const uint32_t ma = transpose32(ra.y, lane), mb = transpose32(rb.y, lane);
+      for (unsigned rows = __ballot_sync(kAll, (ma | mb) != 0); rows; rows &= rows - 1) {
+        const int l = __ffs(rows) - 1;
+        const uint32_t ba = __shfl_sync(kAll, ma, l), bb = __shfl_sync(kAll, mb, l);
+        const Pos at = __shfl_sync(kAll, pos, l);
+        const uint32_t row = __shfl_sync(kAll, pi, l) + probe_base;
+        const Pos pa = at + __popc(ba & lower), pb = at + __popc(ba) + __popc(bb & lower);
+        if ((ra.y >> l) & 1u && pa < cap) {
+          out_build[pa] = ra.x;
+          out_probe[pa] = row;
+        }
+        if ((rb.y >> l) & 1u && pb < cap) {
+          out_build[pb] = rb.x;
+          out_probe[pb] = row;
+        }
+      }
+      pos = min(pos, cap) + (Pos)(__popc(ma) + __popc(mb));  // (never far past the output)
     }
   }
 }
@@ -1088,8 +1117,14 @@ void packet_scatter(uint32_t n, const uint32_t* order, const uint64_t* offs, uin
                     const PacketStore& a, uint32_t* out_build,
                     uint32_t* out_probe, uint64_t cap, cudaStream_t s) {
   if (n == 0) return;
-  k_packet_scatter<<<grid_for(n, 256, kNumSMs * 16), 256, 0, s>>>(
-      n, order, offs, probe_base, a, out_build, out_probe, cap);
+  const int g = grid_for(n, 128, 1 << 24);
+  // (32-bit positions: at most 64 past the output's end)
+  if (cap < 0xffffffffull - 0x01000000ull)
+    k_packet_scatter<uint32_t><<<g, 128, 0, s>>>(n, order, offs, probe_base, a, out_build,
+                                                 out_probe, (uint32_t)cap);
+  else
+    k_packet_scatter<uint64_t><<<g, 128, 0, s>>>(n, order, offs, probe_base, a, out_build,
+                                                 out_probe, cap);
   SPJ_CUDA(cudaGetLastError());
 }
 

@@ -257,9 +257,10 @@ __device__ __forceinline__ bool snappy_header(Win& w, uint32_t ip, uint32_t& len
 // (restaged a window at a time, so an element does not wait on a global
 // load), copies from the block's own output, all by the 32 lanes.  The last
 // kFragRing output bytes are kept in shared memory, where most copies find
-// their source without waiting for its bytes to come back from L2.  Bound by the chain of element headers (400k polygons,
-// 700 blocks at once: 590 us, 466 with the ring).  A copy
-// that reaches before its block sends the page to k_snappy_pages.  Work item
+// their source without waiting for its bytes to come back from L2.  Bound by
+// the chain of element headers (400k polygons, 700 blocks at once: 590 us, 466
+// with the ring).  A copy that reaches before its block sends the page to
+// k_snappy_pages.  Work item
 // (page, block 0) also copies a v2 page's level bytes.
 __global__ void __launch_bounds__(128) k_snappy_frags(
     const PageInfo* __restrict__ pages, const uint2* __restrict__ work, uint32_t nwork,
