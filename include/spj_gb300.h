@@ -90,7 +90,11 @@ int SpjJoinPushBuildArrow(SpjJoin* join, const struct ArrowSchema* schema,
                           const struct ArrowArray* array);
 int SpjJoinFinishBuild(SpjJoin* join);
 /* Execution options (they change speed, never the pairs or their order):
- *   "probe_order"       -1 row order, 0 Morton order from 65536 rows up, 1 always
+ *   "probe_order"       -1 row order, 0 Morton order from 65536 rows up (fewer
+ *                       where the packet kernels pay earlier), 1 always.  In
+ *                       Morton order, and with the options below at their
+ *                       defaults, 32 neighbouring probe rows are traversed and
+ *                       refined together, without candidate pairs
  *   "candidate_order"   3 (default) auto: 2 for relation predicates with 4M+
  *                       candidates over a build side that is not all points,
  *                       else 0; 2 by build row then probe Morton rank, 0 as
