@@ -339,15 +339,15 @@ def run_ours(args, world, rank, local, pg, light=False, workload=None, pred_over
                                          build_vbytes)
     ref_ms = st["ms_refine"] / steps
     achieved = ref_bytes / (ref_ms * 1e-3) / 1e9 if ref_ms > 0 else 0.0
-    kernel = "k_dwithin<fast>" if pred == "dwithin" else "k_refine<fast>"
-    if pred == "dwithin" and st["ms_compact"] == 0:
-        # point-point ST_DWithin is decided inside the traversal (count pass +
-        # scatter pass, no candidate pairs): per probe row its point and box
-        # (32 B) and a count (4 B), 8 B per result pair, the build points
-        # (FP64 + FP32 splits, 32 B) once
-        kernel = "k_dwithin_fused (count + scatter passes)"
+    kernel = "k_packet (+ k_packet_open)"
+    if pred == "dwithin":
+        # point-point ST_DWithin is decided inside the traversal (records of
+        # hits, then their pairs, no candidate pairs): per probe row its point
+        # and box (32 B) and a count (4 B), 8 B per result pair, the build
+        # points (FP64 + FP32 splits, 32 B) once
+        kernel = "k_dwithin_packet + k_packet_scatter"
         ref_bytes = n_rows * 36 + 8 * chosen["pairs"] + 32 * len(inp.build)
-        ref_ms = (st["ms_filter"] + st["ms_refine"]) / steps
+        ref_ms = (st["ms_refine"] + st["ms_compact"]) / steps
         achieved = ref_bytes / (ref_ms * 1e-3) / 1e9 if ref_ms > 0 else 0.0
     traffic = None
     traffic_note = None
@@ -355,8 +355,9 @@ def run_ours(args, world, rank, local, pg, light=False, workload=None, pred_over
     if os.path.exists(tf) and pred == "intersects":
         with open(tf) as f:
             tj = json.load(f)
-        traffic = tj.get("bytes_per_launch")
-        traffic_note = tj.get("scaled_from")
+        if tj.get("kernel", "").split("<")[0] in kernel:  # of the kernel that ran
+            traffic = tj.get("bytes_per_launch")
+            traffic_note = tj.get("scaled_from")
 
     pairs_total = chosen["pairs"] * world
     value = pairs_total / (chosen["ms"] * 1e-3)
@@ -713,7 +714,7 @@ def run_knn(inp, local, steps: int, warmup: int, parity: bool = False):
     ach = alg / (res["chosen"]["ms_per_step"] * 1e-3) / 1e9
     res["speedup_chosen_vs_plain"] = res["plain"]["ms_per_step"] / res["chosen"]["ms_per_step"]
     res["k"] = k
-    res["roofline"] = {"bound": "hbm", "kernel": "k_knn_split<8>", "achieved": ach,
+    res["roofline"] = {"bound": "hbm", "kernel": "k_knn_packet<8>", "achieved": ach,
                        "peak": hbm_peak, "unit": "GB/s", "frac": ach / hbm_peak,
                        "algorithmic_bytes_per_launch": alg}
     if parity:
@@ -949,7 +950,7 @@ def run_learned(args, world, rank, local, pg):
         "lbvh_fast_form": {"ms_per_step": fast_ms, "pairs_per_s": npairs / (fast_ms * 1e-3),
                            "form": "LBVH join, FP32-filtered refine, Morton-ordered probes",
                            "speedup_learned_vs_lbvh_fast": fast_ms / ms},
-        "roofline": {"bound": "hbm", "kernel": "k_learned_ranges + k_learned_eval (all passes)",
+        "roofline": {"bound": "hbm", "kernel": "k_learned_search + k_learned_write + k_learned_eval",
                      "achieved": achieved, "peak": hbm_peak, "peak_kind": peak_kind,
                      "unit": "GB/s", "frac": achieved / hbm_peak, "traffic": None,
                      "algorithmic_bytes_per_launch": alg},
@@ -1084,7 +1085,7 @@ def run_geoparquet(args, local):
                "decode": 41 * n,             # length word, validity, value spans (tmp + row)
                "values": 2 * vb + 28 * n}    # value bytes read + written, spans, offsets
         kernels = {"decompress": "k_snappy_frags (+ k_snappy_pages; host block index)",
-                   "decode": "k_data_pages",
+                   "decode": "k_data_pages + k_seg_walk / chain / write",
                    "values": "k_copy_values (+ k_offsets64)"}
         dom = max(alg, key=lambda k: ph_avg[k])
         hbm_peak, peak_kind = load_peaks()

@@ -27,7 +27,8 @@ struct EngineConfig {
   int refine_form = kFastF32;
   bool profile = false;  // time each phase with CUDA events on the engine stream
   // traversal order of the probe rows: 0 = Morton order from kOrderMinRows
-  // rows up, 1 = always Morton order, -1 = row order
+  // rows up (kPacketRows* where packets take them), 1 = always Morton order,
+  // -1 = row order
   int probe_order = 0;
   // point build and probe sides: decide ST_DWithin inside the traversal
   // (FAST_F32 form); otherwise filter, refine and compact
@@ -40,8 +41,13 @@ struct EngineConfig {
   // 80 % of the pairs).  0 off, 1 on, 2 auto: on when the probes are not in
   // Morton order.  20M x 1M GMM points: in row order 297 -> 139 ms per step;
   // in Morton order the counting pass slowed from 38 to 103 ms with it (the
-  // scatter pass fell from 33 to 9 ms), so auto leaves it off there
+  // scatter pass fell from 33 to 9 ms), so auto leaves it off there.  (Slots and
+  // arena are of the traversal per probe; ordered probes take packets unless
+  // one of them is set)
   int dwithin_arena = 2;
+  // (candidate_order, order_tiles, refine_min_blocks and refine_split are of the
+  // candidate pairs' path and their figures are its; ordered probe rows take the
+  // packet kernels unless one of them is set: 2M x 50k polygons 18.1 ms)
   // refine order of the candidates: 0 as listed (by probe row), 2 by build
   // row then probe Morton rank (a warp then tests one build geometry's edges
   // against neighbouring probes: shared loads and similar trip counts; 2M x
