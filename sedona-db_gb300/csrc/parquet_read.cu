@@ -655,7 +655,8 @@ __device__ __forceinline__ bool seg_value(const uint8_t* vp, uint32_t avail, uin
   if (order > 1) return false;
   const uint32_t t = ld_u32(vp + q + 5), type = order ? t : __byte_perm(t, 0, 0x0123);
   next = q + 4 + l;
-  return type >= 1 && type <= 7;
+  const uint32_t base = (type & 0x0fffffffu) % 1000u;  // (with or without Z, M, SRID flags)
+  return base >= 1 && base <= 17;
 }
 
 __device__ __forceinline__ uint32_t seg_page(const PageInfo* pages, uint32_t np, uint32_t seg) {
