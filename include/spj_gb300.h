@@ -112,6 +112,11 @@ int SpjJoinFinishBuild(SpjJoin* join);
  *                       all pairs queues the pairs it leaves open for a full
  *                       pass); 3 on, with the queue sorted back into the
  *                       candidate order before the full pass
+ *   "packet_bytes"      17179869184 (default), 0 and up: most device memory for
+ *                       the packet kernels' records, and as much again for the
+ *                       pairs that they leave open.  A call that needs more, or
+ *                       for which the memory is not there, takes the candidate
+ *                       pairs (ST_DWithin: a traversal per probe); 0: all calls
  *   "host_slices"       0 (default: auto, 2 from 524,288 rows), 1 (one
  *                       call), 2-64: row slices of SpjJoinProbeHost
  *   "cell_grid"         1 (default) / 0: per-ring cell grids on the build side

@@ -807,6 +807,9 @@ extern "C" int SpjJoinSetOption(SpjJoin* j, const char* key, int64_t value) {
     } else if (k == "refine_split") {
       SPJ_CHECK(value >= 0 && value <= 3, "refine_split must be 0, 1, 2 or 3");
       c.refine_split = (int)value;
+    } else if (k == "packet_bytes") {
+      SPJ_CHECK(value >= 0, "packet_bytes must be non-negative");
+      c.packet_bytes = (uint64_t)value;
     } else if (k == "host_slices") {
       SPJ_CHECK(value >= 0 && value <= 64, "host_slices must be in [0, 64]");
       c.host_slices = (int)value;

@@ -110,7 +110,7 @@ static uint32_t packet_min_rows(int predicate, bool points) {
 // unless the slots or the arena of the traversal per probe were asked for.
 bool JoinEngine::packet_dwithin() const {
   const EngineConfig auto_cfg;
-  return cfg_.dwithin_slots == auto_cfg.dwithin_slots &&
+  return cfg_.packet_bytes > 0 && cfg_.dwithin_slots == auto_cfg.dwithin_slots &&
          cfg_.dwithin_arena == auto_cfg.dwithin_arena;
 }
 
@@ -119,15 +119,15 @@ bool JoinEngine::packet_dwithin() const {
 // take the probe rows (which have to be in Morton order).
 bool JoinEngine::packet_path(int predicate, bool points) const {
   const EngineConfig auto_cfg;
-  return predicate != kPredDWithin && cfg_.refine_form == kFastF32 && !bg_.all_points &&
-         bg_.nrings > 0 && bvh_.nprims > 0 && cfg_.candidate_order == auto_cfg.candidate_order &&
+  return cfg_.packet_bytes > 0 && predicate != kPredDWithin && cfg_.refine_form == kFastF32 &&
+         !bg_.all_points && bg_.nrings > 0 && bvh_.nprims > 0 && cfg_.candidate_order == auto_cfg.candidate_order &&
          cfg_.order_tiles == auto_cfg.order_tiles && cfg_.refine_split == auto_cfg.refine_split &&
          cfg_.refine_min_blocks == auto_cfg.refine_min_blocks && !cfg_.grid_rings &&
          packet_takes(predicate, points);
 }
 
 // The pairs by the packet kernels; false where their records would pass the
-// limits (the candidate pairs' path then answers).
+// limits or find no memory (the candidate pairs' path then answers).
 bool JoinEngine::packet_probe(Workspace& ws, int predicate, double distance, const double* d_row,
                               const float4* boxes, uint32_t probe_base, const uint32_t* order,
                               DeviceStatus& hst, uint64_t& launches, uint64_t& total) {
@@ -141,10 +141,11 @@ bool JoinEngine::packet_probe(Workspace& ws, int predicate, double distance, con
   ws.psc.offsets.reserve(((size_t)n + 1) * 8, s);
   // first guesses (2M buildings x 50k zones: 2.4 records and 6 open pairs per
   // probe row); a column that needs more tells how much and runs again
-  uint64_t chunks = std::min<uint64_t>(n / 8 + 1024, kPacketMaxChunks);
-  uint64_t queued = points ? 0 : std::min<uint64_t>((uint64_t)n * 8 + 1024, kPacketMaxQueue);
+  const PacketLimits most(cfg_.packet_bytes);
+  uint64_t chunks = std::min<uint64_t>(n / 8 + 1024, most.chunks);
+  uint64_t queued = points ? 0 : std::min<uint64_t>((uint64_t)n * 8 + 1024, most.queue);
   for (int attempt = 0;; attempt++) {
-    ws.packet.reserve(n, chunks, queued, s);
+    if (!ws.packet.reserve(n, chunks, queued, s)) return false;
     const PacketStore a = ws.packet.store(n);
     reset_status(ws.status, s);
     if (dwithin)
@@ -164,12 +165,12 @@ bool JoinEngine::packet_probe(Workspace& ws, int predicate, double distance, con
     check_traversal_word(rb->fault);
     if (rb->ctrl[0] <= a.chunks && rb->ctrl[1] <= a.queue_cap) break;
     SPJ_CHECK(attempt < 2, "packet refine: record capacities did not settle");
-    if (rb->ctrl[0] > kPacketMaxChunks || rb->ctrl[1] > kPacketMaxQueue) {
+    if (rb->ctrl[0] > most.chunks || rb->ctrl[1] > most.queue) {
       ws.packet.release();
       return false;
     }
-    chunks = std::min(rb->ctrl[0] + rb->ctrl[0] / 8, kPacketMaxChunks);
-    queued = std::min(rb->ctrl[1] + rb->ctrl[1] / 8, kPacketMaxQueue);
+    chunks = std::min(rb->ctrl[0] + rb->ctrl[0] / 8, most.chunks);
+    queued = std::min(rb->ctrl[1] + rb->ctrl[1] / 8, most.queue);
   }
   hst = rb->st;
   total = rb->total;

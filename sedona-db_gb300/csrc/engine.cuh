@@ -89,6 +89,10 @@ struct EngineConfig {
   // host probes (SpjJoinProbeHost): 0 auto (2 slices from 524,288 rows up),
   // 1 one call, n > 1 that many slices
   int host_slices = 0;
+  // most memory of the packet kernels' records, and as much again of the pairs
+  // that they leave open; joins that need more, or whose memory is not there,
+  // take the candidate pairs (ST_DWithin: a traversal per probe).  0: none
+  uint64_t packet_bytes = 1ull << 34;
 };
 constexpr uint32_t kOrderMinRows = 1u << 16;
 // Rows from which the packet kernels are taken, by what a candidate costs

@@ -1049,17 +1049,26 @@ __global__ void __launch_bounds__(128)
 
 static uint64_t most_packets(uint32_t n) { return ((uint64_t)n + 31) / 32 * 32; }
 
-void PacketBufs::reserve(uint32_t n, uint64_t chunks, uint64_t queued, cudaStream_t s) {
+bool PacketBufs::reserve(uint32_t n, uint64_t chunks, uint64_t queued, cudaStream_t s) {
   const uint64_t most = most_packets(n);
-  chunk_cap = std::max(chunk_cap, chunks);
-  queue_cap = std::max(queue_cap, queued);
-  SPJ_CHECK(chunk_cap <= kPacketMaxChunks && queue_cap <= kPacketMaxQueue,
+  chunks = std::max(chunk_cap, chunks);
+  queued = std::max(queue_cap, queued);
+  SPJ_CHECK(chunks <= kPacketMaxChunks && queued <= kPacketMaxQueue,
             "packet records exceed their limit");
-  rec.reserve(chunk_cap * 32 * sizeof(uint2), s);
-  next.reserve(chunk_cap * 4, s);
-  queue.reserve((queue_cap + 1) * sizeof(uint4), s);
-  heads.reserve((most + 1) * 16, s);
-  ctrl.reserve(kPacketCtrlBytes, s);
+  try {
+    rec.reserve(chunks * 32 * sizeof(uint2), s);
+    next.reserve(chunks * 4, s);
+    queue.reserve((queued + 1) * sizeof(uint4), s);
+    heads.reserve((most + 1) * 16, s);
+    ctrl.reserve(kPacketCtrlBytes, s);
+  } catch (const Error&) {
+    (void)cudaGetLastError();  // (the next launch's check is not to find it)
+    release();
+    return false;
+  }
+  chunk_cap = chunks;
+  queue_cap = queued;
+  return true;
 }
 
 PacketStore PacketBufs::store(uint32_t n) const {

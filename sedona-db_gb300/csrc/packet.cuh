@@ -58,15 +58,25 @@ __device__ __forceinline__ uint32_t packet_append(const PacketStore& A, uint32_t
 }
 #endif
 
-// Most chunks and queued pairs a join keeps (16 GB each); one that needs more
-// takes the candidate pairs' path, which has no records.
+// Most chunks and queued pairs a join keeps (at most 16 GB each); one that needs
+// more, or whose memory is not there, takes the candidate pairs' path, which has
+// no records.
 constexpr uint64_t kPacketMaxChunks = 1ull << 26, kPacketMaxQueue = 1ull << 30;
+struct PacketLimits {
+  uint64_t chunks, queue;
+  // as many as `bytes` of records and `bytes` of queued pairs hold
+  explicit PacketLimits(uint64_t bytes)
+      : chunks(bytes / (32 * sizeof(uint2)) < kPacketMaxChunks ? bytes / (32 * sizeof(uint2))
+                                                               : kPacketMaxChunks),
+        queue(bytes / sizeof(uint4) < kPacketMaxQueue ? bytes / sizeof(uint4) : kPacketMaxQueue) {}
+};
 
 struct PacketBufs {
   DevBuf rec, next, heads, queue, ctrl;
-  uint64_t chunk_cap = 0, queue_cap = 0;
-  // reserves room for n probe rows and at least the given chunks / pairs
-  void reserve(uint32_t n, uint64_t chunks, uint64_t queued, cudaStream_t s);
+  uint64_t chunk_cap = 0, queue_cap = 0;  // what the buffers hold
+  // Makes room for n probe rows and at least the given chunks / pairs.  False
+  // when the memory is not there: nothing is kept then.
+  bool reserve(uint32_t n, uint64_t chunks, uint64_t queued, cudaStream_t s);
   PacketStore store(uint32_t n) const;
   void release();
 };

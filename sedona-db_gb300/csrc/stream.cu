@@ -175,7 +175,9 @@ void StreamJoin::set_batches(const std::vector<WkbDeviceColumn>& cols) {
     ccap_ = (uint64_t)nrows_ * 8 + 1024;
     ocap_ = (uint64_t)nrows_ * 4 + 1024;
   }
-  chunks_cap_ = std::max(chunks_cap_, std::min<uint64_t>(nrows_ / 8 + 1024, kPacketMaxChunks));
+  const PacketLimits most(eng_.config().packet_bytes);
+  chunks_cap_ =
+      std::max(packet_.chunk_cap, std::min<uint64_t>(nrows_ / 8 + 1024, most.chunks));
   packet_off_ = false;
   SPJ_CUDA(cudaStreamSynchronize(s_));
   std::ostringstream sig;
@@ -201,11 +203,13 @@ void StreamJoin::build_graph(int predicate) {
   // here, so the capture allocates nothing
   const bool want = cfg.probe_order > 0 || (cfg.probe_order == 0 && nrows_ >= kOrderMinRows);
   graph_packet_ = want && nrows_ >= 2 && !packet_off_ && eng_.packet_path(predicate, true);
+  if (graph_packet_ && !packet_.reserve(nrows_, chunks_cap_, 0, s_)) {
+    graph_packet_ = false;  // no memory for the records: the candidate pairs
+    packet_off_ = true;
+  }
   const bool ordered = want && (graph_packet_ || ccap_ < 0xFFFFFFFFull);
   // capacity-sized buffers
-  if (graph_packet_) {
-    packet_.reserve(nrows_, chunks_cap_, 0, s_);
-  } else {
+  if (!graph_packet_) {
     cand_b_.reserve((ccap_ + 1) * 4, s_);
     cand_p_.reserve((ccap_ + 1) * 4, s_);
     flags_.reserve(ccap_ + 1, s_);
@@ -306,11 +310,12 @@ uint64_t StreamJoin::run(int predicate, const uint32_t** d_build, const uint32_t
     if (graph_packet_ && h_tot_[4] > chunks_cap_) {
       // the packets' records did not fit: grow, re-capture, replay (past the
       // limit: with the candidate pairs)
-      if (h_tot_[4] > kPacketMaxChunks) {
+      const PacketLimits most(eng_.config().packet_bytes);
+      if (h_tot_[4] > most.chunks) {
         packet_off_ = true;
         packet_.release();
       } else {
-        chunks_cap_ = std::min(h_tot_[4] + h_tot_[4] / 8, kPacketMaxChunks);
+        chunks_cap_ = std::min(h_tot_[4] + h_tot_[4] / 8, most.chunks);
       }
       destroy_graph();
       continue;

@@ -3,7 +3,7 @@ candidate pairs' path and the oracle."""
 import numpy as np
 import pytest
 
-from gpu_util import pairs
+from gpu_util import device_column, device_pairs, pairs
 
 pytestmark = pytest.mark.gpu
 
@@ -135,6 +135,73 @@ def test_packet_capacities_grow(capi):
                               [_star(rng, rng.uniform(-40, 40, 2), 5, 3.0)]]) for _ in range(40)])
     for _ in _both(capi, build, multi, ["intersects", "contains"]):
         pass
+
+
+@pytest.mark.parametrize("size", [256, 256 * 300, 0])
+def test_packet_memory_limit(capi, size):
+    """Records and open pairs past packet_bytes: the candidate pairs (ST_DWithin:
+    the traversal per probe) answer, and the packets again with more room."""
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(11)
+    zones = _zones(rng, 400, holes=True)
+    build = wkb.column_from_values(zones)
+    for kind in ("points", "mixed"):
+        probe = wkb.column_from_values(_probes(rng, 600, kind, zones))
+        j = capi.SpatialJoin(probe_order=1)
+        j.build(build)
+        for pred in ("intersects", "contains"):
+            exp = j.probe(probe, pred)
+            for limit in (size, 1 << 34):
+                j.set_option("packet_bytes", limit)
+                k = capi.SpatialJoin(probe_order=1)
+                k.set_option("packet_bytes", limit)
+                k.build(build)
+                for got in (j.probe(probe, pred), k.probe(probe, pred)):
+                    np.testing.assert_array_equal(exp[0], got[0])
+                    np.testing.assert_array_equal(exp[1], got[1])
+    bp, pp = (wkb.points_column(*rng.uniform(0, 50, (2, m))) for m in (2000, 500))
+    got = []
+    for limit in (1 << 34, size):
+        j = capi.SpatialJoin(probe_order=1)
+        j.set_option("packet_bytes", limit)
+        j.build(bp)
+        got.append(j.probe(pp, "dwithin", distance=4.0))
+    np.testing.assert_array_equal(got[0][0], got[1][0])
+    np.testing.assert_array_equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("limit", [1 << 34, 256 * 1500])
+def test_packet_stream_grows(capi, limit):
+    """A stream whose records and pairs both outgrow their first room (the graph
+    is captured again; only the pairs are written again), or pass the limit (the
+    candidate pairs): the arrays of the unordered graph, run after run and for
+    smaller batches afterwards."""
+    import torch
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(12)
+    build = wkb.column_from_values([wkb.wkb_polygon([_star(rng, np.zeros(2), 12, 50.0)])
+                                    for _ in range(2000)])
+    sizes = (900, 1, 1600, 0, 499)
+    cols = [wkb.points_column(*rng.uniform(-45, 45, (2, m))) for m in sizes]
+    out = []
+    for order in (-1, 1):
+        j = capi.SpatialJoin(probe_order=order)
+        j.set_option("packet_bytes", limit)
+        j.build(build)
+        st = capi.StreamProbe(j)
+        res = []
+        for some in (cols, cols[:2], cols):
+            dev = [device_column(capi, c) for c in some]
+            torch.cuda.synchronize()
+            st.set_batches([d for d, _ in dev])
+            for pred in ("intersects", "contains", "contains"):
+                db, dp, n = st.run(pred)
+                res.append(device_pairs(db, dp, n))
+        out.append(res)
+    assert len(out[0][0][0]) > 4 * sum(sizes) + 1024
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a[0], b[0])
+        np.testing.assert_array_equal(a[1], b[1])
 
 
 @pytest.mark.parametrize("n,leaf", [(2, 16), (31, 1), (32, 16), (33, 64), (127, 33), (2500, 16)])
