@@ -288,10 +288,13 @@ void StreamJoin::build_graph(int predicate) {
   cudaGraphDestroy(g);
   SPJ_CUDA(e);
   graph_pred_ = predicate;
-  // memsets 2, decode 1, count 1, scan 3, scatter 1, refine 1, flag counts 2, compact 1;
-  // ordered: keys 1 + 4 radix passes of 5, candidate order 5, flags memset 1
-  // (packets: memsets 3, decode 1, order 21, packets 1, join 1, scan 3, scatter 1)
-  stats_.launches_per_replay = graph_packet_ ? 31 : 12 + (cperm ? 27 : (order ? 21 : 0));
+  // memsets 2, decode 1, scan; ordered: keys 1 and the sort
+  const uint64_t scan = scan_launches(nrows_);
+  stats_.launches_per_replay = 3 + scan + (order ? 1 + radix_sort_launches(nrows_, 32) : 0);
+  if (graph_packet_)
+    stats_.launches_per_replay += 4;  // memset, packets, join, scatter
+  else  // count, scatter, refine, flag counts 2, compact; counts in order, scan, permutation, memset
+    stats_.launches_per_replay += 6 + (cperm ? 3 + scan : 0);
 }
 
 uint64_t StreamJoin::run(int predicate, const uint32_t** d_build, const uint32_t** d_probe) {

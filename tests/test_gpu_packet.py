@@ -204,6 +204,27 @@ def test_packet_stream_grows(capi, limit):
         np.testing.assert_array_equal(a[1], b[1])
 
 
+@pytest.mark.parametrize("n,order,packets,launches", [
+    (3000, -1, True, 10), (3000, 1, True, 10), (3000, 1, False, 16),
+    (70000, -1, True, 12), (70000, 0, True, 23), (70000, 0, False, 31)])
+def test_stream_launches(capi, n, order, packets, launches):
+    """Launches per replay: scans and sorts of up to 16,384 elements are one each
+    (the scans within the sort of 70,000 rows are of 35 tiles' 256 counts)."""
+    import torch
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(13)
+    j = capi.SpatialJoin(probe_order=order)
+    if not packets:
+        j.set_option("packet_bytes", 0)
+    j.build(wkb.column_from_values(_zones(rng, 20, holes=False)))
+    dev = device_column(capi, wkb.points_column(*rng.uniform(0, 200, (2, n))))
+    torch.cuda.synchronize()
+    st = capi.StreamProbe(j)
+    st.set_batches([dev[0]])
+    st.run("contains")
+    assert st.stats()["launches_per_replay"] == launches
+
+
 @pytest.mark.parametrize("n,leaf", [(2, 16), (31, 1), (32, 16), (33, 64), (127, 33), (2500, 16)])
 def test_packet_dwithin_same_pairs_and_positions(capi, n, leaf):
     """ST_DWithin of points by the packet traversal against the traversal per
