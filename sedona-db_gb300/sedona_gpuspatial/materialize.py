@@ -199,7 +199,8 @@ class VisitedBitmap:
         left anti and full joins), ascending, as int32."""
         count = C.c_uint64(0)
         s = _stream(self.words)
-        # room for all rows where that is little memory, else their count first
+        # room for all rows where that is little memory, else their count first;
+        # the result keeps only the memory of its own rows
         cap = self.n_rows if self.n_rows <= (1 << 22) else 0
         out = torch.empty((cap,), dtype=torch.int32, device=self.words.device)
         rc = lib().SpjVisitedCollect(_ptr(self.words), self.n_rows, int(visited), _ptr(out), cap,
@@ -211,7 +212,8 @@ class VisitedBitmap:
             _check(lib().SpjVisitedCollect(_ptr(self.words), self.n_rows, int(visited),
                                            _ptr(out), out.numel(), C.byref(count), s),
                    "visited collect")
-        return out[:int(count.value)]
+        n = int(count.value)
+        return out if n == out.numel() else out[:n].clone()
 
     def bitmap(self) -> torch.Tensor:
         """The mark column of a mark join: Arrow LSB bits, one per row."""

@@ -168,6 +168,17 @@ def test_visited_collect_too_small(mat):
     assert out.cpu().tolist() == [-5, -5]
 
 
+@pytest.mark.parametrize("n_rows", [1, 5000, (1 << 22) + 5])
+def test_visited_collect_keeps_its_rows_only(mat, n_rows):
+    """The memory behind a result is that of its rows, not of the whole side."""
+    vb = mat.VisitedBitmap(n_rows)
+    ids = np.unique(np.linspace(0, n_rows - 1, 7).astype(np.int32))
+    vb.mark(_t(ids))
+    got = vb.collect(True)
+    assert np.array_equal(got.cpu().numpy(), ids)
+    assert got.untyped_storage().nbytes() == 4 * len(ids)
+
+
 def test_joined_batch_and_left_outer_join(mat, oracle_lib):
     """One probe of the fused join, its pairs left on the device, then the
     joined batch (build WKB + build id column + probe WKB) and the unmatched
