@@ -94,7 +94,9 @@ int SpjJoinFinishBuild(SpjJoin* join);
  *                       where the packet kernels pay earlier), 1 always.  In
  *                       Morton order, and with the options below at their
  *                       defaults, 32 neighbouring probe rows are traversed and
- *                       refined together, without candidate pairs
+ *                       refined together, without candidate pairs: always with
+ *                       1, with 0 where the build rows are estimated to be
+ *                       large and the probe rows dense enough for it to pay
  *   "candidate_order"   3 (default) auto: 2 for relation predicates with 4M+
  *                       candidates over a build side that is not all points,
  *                       else 0; 2 by build row then probe Morton rank, 0 as
@@ -192,6 +194,9 @@ int SpjJoinSetProbeDistances(SpjJoin* join, const double* distances, uint64_t n,
 /* The CUDA stream (cudaStream_t) the join launches its kernels on. */
 void* SpjJoinStream(SpjJoin* join);
 int SpjJoinGetStats(SpjJoin* join, struct SpjJoinStats* out);
+/* Probe calls of this join that the packet kernels answered (32 neighbouring
+ * probe rows at a time; the others took candidate pairs). */
+uint64_t SpjJoinPacketCalls(SpjJoin* join);
 int SpjJoinResetStats(SpjJoin* join);
 
 /* ------------------------------------------------------------------------ */

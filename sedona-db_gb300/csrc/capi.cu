@@ -1093,6 +1093,8 @@ extern "C" int SpjJoinGetStats(SpjJoin* j, SpjJoinStats* out) {
   });
 }
 
+extern "C" uint64_t SpjJoinPacketCalls(SpjJoin* j) { return j->engine->packet_calls(); }
+
 extern "C" int SpjJoinResetStats(SpjJoin* j) {
   return guarded(j->last_error, [&] { j->engine->reset_stats(); });
 }

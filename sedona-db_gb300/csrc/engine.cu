@@ -98,12 +98,37 @@ static inline float ev_ms(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
-// (ST_Intersects and ST_Disjoint stop at the first edge that decides, and
-// points visit few edges: their pairs are cheap.)
-static uint32_t packet_min_rows(int predicate, bool points) {
-  if (predicate == kPredDWithin) return kPacketRowsDWithin;
-  return points || predicate == kIntersects || predicate == kDisjoint ? kOrderMinRows
-                                                                      : kPacketRowsFull;
+bool packet_pays(int predicate, bool points, uint64_t rows, const PacketTree& t) {
+  if (predicate == kPredDWithin)
+    return rows >= kPacketRowsDWithin &&
+           (t.nprims <= 100000 || rows * 12 >= t.nprims || t.crowd >= 1.0);
+  const bool first = predicate == kIntersects || predicate == kDisjoint;
+  if (rows < (points || first ? kOrderMinRows : kPacketRowsFull)) return false;
+  const double covers = t.share * t.nprims, held = t.share * rows;
+  if (points)
+    return held >= 90.0 + 1.3 * covers ||
+           (covers <= 2.0 && rows >= 6ull * t.nprims && (t.nprims <= 8192 || covers >= 0.1));
+  if (first) return held >= 48.0 || (covers >= 0.04 && covers <= 0.3);
+  switch (predicate) {
+    case kContains:
+    case kCovers:
+      return held >= (t.holes ? 14.0 : 28.0) || (covers >= 0.5 && rows >= 10ull * t.nprims);
+    case kTouches:
+      return covers >= 0.04;
+    default:
+      return covers >= (rows >= kOrderMinRows ? 0.04 : 6.0);
+  }
+}
+
+PacketTree JoinEngine::packet_tree(double distance) const {
+  PacketTree t;
+  t.nprims = bvh_.nprims;
+  t.share = bvh_.extent_area > 0.0f
+                ? std::min(1.0, (double)bvh_.mean_w * bvh_.mean_h / bvh_.extent_area)
+                : 1.0;
+  t.holes = bg_.nrings > bg_.nparts;
+  t.crowd = 4.0 * distance * distance * bvh_.leaf_density;
+  return t;
 }
 
 // Fused ST_DWithin of probes in Morton order: one traversal per 32 of them,
@@ -120,7 +145,8 @@ bool JoinEngine::packet_dwithin() const {
 bool JoinEngine::packet_path(int predicate, bool points) const {
   const EngineConfig auto_cfg;
   return cfg_.packet_bytes > 0 && predicate != kPredDWithin && cfg_.refine_form == kFastF32 &&
-         !bg_.all_points && bg_.nrings > 0 && bvh_.nprims > 0 && cfg_.candidate_order == auto_cfg.candidate_order &&
+         !bg_.all_points && bg_.nrings > 0 && bvh_.nprims > 0 &&
+         cfg_.candidate_order == auto_cfg.candidate_order &&
          cfg_.order_tiles == auto_cfg.order_tiles && cfg_.refine_split == auto_cfg.refine_split &&
          cfg_.refine_min_blocks == auto_cfg.refine_min_blocks && !cfg_.grid_rings &&
          packet_takes(predicate, points);
@@ -226,12 +252,14 @@ uint64_t JoinEngine::probe(Workspace& ws, const WkbDeviceColumn& col, int predic
   const bool fused = predicate == kPredDWithin && cfg_.fuse_dwithin &&
                      cfg_.refine_form == kFastF32 && ws.probe.all_points &&
                      bsplit_.n == bvh_.nprims && bvh_.nprims > 0;
+  // (a probe_order that is set decides by itself; distances per row are not
+  // known here)
   const bool packet =
-      fused ? packet_dwithin() : packet_path(predicate, ws.probe.all_points);
+      (fused ? packet_dwithin() : packet_path(predicate, ws.probe.all_points)) &&
+      (cfg_.probe_order > 0 || packet_pays(predicate, ws.probe.all_points, n,
+                                           packet_tree(d_row ? 0.0 : distance)));
   const uint32_t* order = nullptr;
-  if (cfg_.probe_order > 0 ||
-      (cfg_.probe_order == 0 &&
-       n >= (packet ? packet_min_rows(predicate, ws.probe.all_points) : kOrderMinRows))) {
+  if (cfg_.probe_order > 0 || (cfg_.probe_order == 0 && (packet || n >= kOrderMinRows))) {
     order = probe_order(tv, boxes, n, ws.psc, s);
     if (order) launches += 1 + radix_sort_launches(n, 32);
   }
@@ -261,6 +289,7 @@ uint64_t JoinEngine::probe(Workspace& ws, const WkbDeviceColumn& col, int predic
     uint64_t total = 0;
     if (packet_probe(ws, predicate, distance, d_row, boxes, probe_base, order, hst, launches,
                      total)) {
+      packet_calls_++;
       if (prof) SPJ_CUDA(cudaEventRecord(ws.ev[4], s));
       SPJ_CUDA(cudaStreamSynchronize(s));
       count(hst, total);

@@ -8,6 +8,7 @@
 // runs RTSpatialIndex::Probe and RTSpatialRefiner::Refine back to back with
 // host round trips in between.
 #pragma once
+#include <atomic>
 #include <mutex>
 
 #include "geoms.cuh"
@@ -27,8 +28,8 @@ struct EngineConfig {
   int refine_form = kFastF32;
   bool profile = false;  // time each phase with CUDA events on the engine stream
   // traversal order of the probe rows: 0 = Morton order from kOrderMinRows
-  // rows up (kPacketRows* where packets take them), 1 = always Morton order,
-  // -1 = row order
+  // rows up, and of fewer where packets take them (packet_pays), 1 = always
+  // Morton order, -1 = row order
   int probe_order = 0;
   // point build and probe sides: decide ST_DWithin inside the traversal
   // (FAST_F32 form); otherwise filter, refine and compact
@@ -95,17 +96,40 @@ struct EngineConfig {
   uint64_t packet_bytes = 1ull << 34;
 };
 constexpr uint32_t kOrderMinRows = 1u << 16;
-// Rows from which the packet kernels are taken, by what a candidate costs
-// (packet_min_rows).  A packet's warp goes through its build rows one after
-// the other, so below some size the longest packet takes longer than the
-// candidate pairs spread over all threads.  Packets against pairs, us per
-// call: ST_DWithin with 400k points 720 / 857 at 2,000 rows; buildings
-// touching 50k zones 1,940 / 2,488 at 8,000 rows, in 20k holed zones
-// 1,242 / 1,228 at 8,000 and 1,298 / 1,497 at 12,000; intersecting 50k zones
-// 2,227 / 2,157 at 48,000 and 2,377 / 2,888 at 66,000; points in 50k zones
-// 1,298 / 1,100 at 66,000 and 1,341 / 1,600 at 100,000 (kOrderMinRows).
+// When the packet kernels are taken (packet_pays).  A packet's warp goes
+// through its build rows one after the other, so with few packets the longest
+// takes longer than the candidate pairs spread over all threads; and where 32
+// neighbouring rows lie far apart against the build rows, their packet walks
+// the tree for each of them in turn.  Both show in how many probe rows a build
+// row's box holds (share * rows, the rows spread as the build rows are; a probe
+// row meets share * nprims build rows).  Packets against pairs, us per call:
+//  - points in 50k zones: 66k rows (84 held) 1,460 / 1,097, 140k (180)
+//    1,649 / 1,674, 200k 1,962 / 2,008; in 10k zones 100k (128) 515 / 510, 140k
+//    558 / 629: from 90 held, and 1.3 for each build row that one meets;
+//  - points in small build rows, where the packets save launches and no more:
+//    10k stars 1M rows 490 / 537; 50k stars 130k rows 360 / 335, 500k 558 / 587;
+//    5k clustered buildings 250k rows 277 / 301, 50k of them 610 / 354;
+//  - buildings intersecting 50k zones: 49k rows (63) 2,315 / 2,150, 66k (84)
+//    2,289 / 2,498; 50k stars, 1M rows (31) 2,180 / 1,847, 10k 130k rows 467 / 496;
+//  - containment (dearer pairs): 50k zones 16k rows (21) 2,063 / 1,662, 24k (31)
+//    1,895 / 2,275; with holes 8k (10) 2,301 / 2,245, 12k (15) 2,500 / 2,987;
+//    20k stars 250k rows 652 / 650, 1M 1,301 / 1,431;
+//  - touches (the dearest): 50k zones 8k rows 1,987 / 2,575, 5k stars 452 / 524,
+//    50k clustered buildings (0.02 met) 647 / 568;
+//  - within, covered by, equals: 5k zones (6.4 met) 16k rows 246 / 239, 50k 472 / 586;
+//  - ST_DWithin, by how many points of a middling leaf's density the square of
+//    twice the distance holds (crowd): 400k points, 4k rows: 2 m 400 / 315, 10 m
+//    (0.8) 624 / 427, 30 m (6.9) 740 / 1,066; 32k rows: 339 / 334, 461 / 469,
+//    693 / 1,121; 100k points, 2k rows: 269 / 250, 283 / 288, 329 / 484.
 constexpr uint32_t kPacketRowsDWithin = 1u << 11;
 constexpr uint32_t kPacketRowsFull = 1u << 13;
+struct PacketTree {
+  uint64_t nprims = 0;
+  double share = 0;    // of the build rows' extent that the mean box covers
+  bool holes = false;  // some build polygon has holes
+  double crowd = 0;
+};
+bool packet_pays(int predicate, bool points, uint64_t rows, const PacketTree& t);
 constexpr uint64_t kBuildMajorMin = 1ull << 22;  // candidates before build-major order pays
 constexpr uint64_t kOrderTileCandidates = 1ull << 19;  // auto order_tiles: candidates per tile
 
@@ -201,6 +225,9 @@ class JoinEngine {
   // Whether probes in Morton order take the packet kernels (packet.cuh).
   bool packet_path(int predicate, bool points) const;
   bool packet_dwithin() const;
+  // What packet_pays goes by.
+  PacketTree packet_tree(double distance) const;
+  uint64_t packet_calls() const { return packet_calls_; }
 
   JoinStats stats();
   void reset_stats();
@@ -211,6 +238,7 @@ class JoinEngine {
                     const float4* boxes, uint32_t probe_base, const uint32_t* order,
                     DeviceStatus& hst, uint64_t& launches, uint64_t& total);
   int device_;
+  std::atomic<uint64_t> packet_calls_{0};
   EngineConfig cfg_;
   DeviceGeoms bg_;
   DecodeScratch bsc_;

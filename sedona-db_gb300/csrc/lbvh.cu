@@ -182,14 +182,19 @@ __global__ void k_refit(const float4* __restrict__ sbox, uint32_t m, uint32_t L,
   }
 }
 
+// *log_area += log2 of the leaves' areas
 __global__ void k_leaf_boxes(const float4* __restrict__ sbox, uint32_t m, uint32_t L, uint32_t ls,
-                             float4* __restrict__ out) {
+                             float4* __restrict__ out, float* __restrict__ log_area) {
+  float a = 0.0f;
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < L; c += gridDim.x * blockDim.x) {
     const uint32_t b0 = c * ls, b1 = min(b0 + ls, m);
     float4 bb = sbox[b0];
     for (uint32_t k = b0 + 1; k < b1; k++) bb = box_union(bb, sbox[k]);
     out[c] = bb;
+    a += log2f(fminf(fmaxf((bb.z - bb.x) * (bb.w - bb.y), 1e-30f), 1e30f));
   }
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  if ((threadIdx.x & 31) == 0 && a != 0.0f) atomicAdd(log_area, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -661,12 +666,13 @@ void build_lbvh(const float4* boxes, uint32_t n, uint32_t leaf_size, Lbvh& out, 
   out.fault.reserve(8, s);
   SPJ_CUDA(cudaMemsetAsync(out.fault.get(), 0, 8, s));
   out.mean_w = out.mean_h = out.extent_area = 0.0f;
+  out.leaf_density = 0.0;
   if (m == 0) return;
   uint32_t* ids = out.sorted_id.as<uint32_t>();
   k_compact_ids<<<g, 256, 0, s>>>(flag.as<uint8_t>(), pos.as<uint64_t>(), n, ids);
-  DevBuf ext(24, s);
-  uint32_t init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u};
-  SPJ_CUDA(cudaMemcpyAsync(ext.get(), init, 24, cudaMemcpyHostToDevice, s));
+  DevBuf ext(28, s);
+  uint32_t init[7] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u};
+  SPJ_CUDA(cudaMemcpyAsync(ext.get(), init, 28, cudaMemcpyHostToDevice, s));
   const int gm = grid_for(m, 256);
   k_bounds<<<gm, 256, 0, s>>>(boxes, ids, m, ext.as<uint32_t>(), ext.as<float>() + 4);
   DevBuf keys((size_t)m * 4, s), akeys((size_t)m * 4, s), avals((size_t)m * 4, s);
@@ -675,7 +681,7 @@ void build_lbvh(const float4* boxes, uint32_t n, uint32_t leaf_size, Lbvh& out, 
                    tmp, s);
   k_gather_boxes<<<gm, 256, 0, s>>>(boxes, ids, m, out.sorted_box.as<float4>());
   k_leaf_boxes<<<grid_for(L, 256), 256, 0, s>>>(out.sorted_box.as<float4>(), m, L, leaf_size,
-                                                out.leaf_box.as<float4>());
+                                                out.leaf_box.as<float4>(), ext.as<float>() + 6);
   if (L > 1) {
     DevBuf parent_int((size_t)L * 4, s), parent_leaf((size_t)L * 4, s), visits((size_t)L * 4, s);
     SPJ_CUDA(cudaMemsetAsync(visits.get(), 0, (size_t)L * 4, s));
@@ -687,16 +693,17 @@ void build_lbvh(const float4* boxes, uint32_t n, uint32_t leaf_size, Lbvh& out, 
                                              out.node_box.as<float4>(), visits.as<unsigned>());
   }
   SPJ_CUDA(cudaGetLastError());
-  uint32_t e[6];
-  SPJ_CUDA(cudaMemcpyAsync(e, ext.get(), 24, cudaMemcpyDeviceToHost, s));
+  uint32_t e[7];
+  SPJ_CUDA(cudaMemcpyAsync(e, ext.get(), 28, cudaMemcpyDeviceToHost, s));
   SPJ_CUDA(cudaStreamSynchronize(s));
-  float sums[2];
-  memcpy(sums, e + 4, 8);
+  float sums[3];
+  memcpy(sums, e + 4, 12);
   const float area = (o2f(e[2]) - o2f(e[0])) * (o2f(e[3]) - o2f(e[1]));
   const bool ok = std::isfinite(sums[0]) && std::isfinite(sums[1]) && std::isfinite(area);
   out.mean_w = ok ? sums[0] / (float)m : 0.0f;
   out.mean_h = ok ? sums[1] / (float)m : 0.0f;
   out.extent_area = ok ? area : 0.0f;
+  out.leaf_density = std::isfinite(sums[2]) ? leaf_size * std::exp2(-(double)sums[2] / L) : 0.0;
 }
 
 void check_traversal(const LbvhView& t, cudaStream_t s) {

@@ -37,6 +37,9 @@ struct LbvhView {
 struct Lbvh {
   uint32_t nprims = 0, nleaves = 0, leaf_size = 4;
   float mean_w = 0.0f, mean_h = 0.0f, extent_area = 0.0f;
+  // primitives per area in a middling leaf (the geometric mean of the leaves'
+  // areas: of clustered points most lie far denser than over the extent)
+  double leaf_density = 0.0;
   DevBuf sorted_box, sorted_id, node_box, node_child, leaf_box, fault;
   LbvhView view() const {
     LbvhView v;

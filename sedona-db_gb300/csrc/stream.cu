@@ -202,7 +202,9 @@ void StreamJoin::build_graph(int predicate) {
   // neighbouring probes together); everything the ordering uses is reserved
   // here, so the capture allocates nothing
   const bool want = cfg.probe_order > 0 || (cfg.probe_order == 0 && nrows_ >= kOrderMinRows);
-  graph_packet_ = want && nrows_ >= 2 && !packet_off_ && eng_.packet_path(predicate, true);
+  graph_packet_ =
+      want && nrows_ >= 2 && !packet_off_ && eng_.packet_path(predicate, true) &&
+      (cfg.probe_order > 0 || packet_pays(predicate, true, nrows_, eng_.packet_tree(0.0)));
   if (graph_packet_ && !packet_.reserve(nrows_, chunks_cap_, 0, s_)) {
     graph_packet_ = false;  // no memory for the records: the candidate pairs
     packet_off_ = true;

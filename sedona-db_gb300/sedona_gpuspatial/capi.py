@@ -189,6 +189,7 @@ EXPORTS = [
     "SpjJoinPushBuildArrow",
     "SpjJoinFinishBuild", "SpjJoinBuildDevice", "SpjJoinProbeArrow", "SpjJoinProbeDevice",
     "SpjJoinProbeHost", "SpjJoinStream", "SpjJoinGetStats", "SpjJoinResetStats",
+    "SpjJoinPacketCalls",
     "SpjKnnCreate", "SpjKnnRelease", "SpjKnnLastError", "SpjKnnBuild", "SpjKnnQuery",
     "SpjKnnQueryTies", "SpjKnnQueryArrow", "SpjJoinSetProbeDistances",
     "SpjKnnStream", "SpjKnnGetStats", "SpjHostRegister", "SpjHostUnregister", "SpjVersion",
@@ -267,6 +268,8 @@ def lib() -> C.CDLL:
             L.SpjJoinStream.restype = C.c_void_p
             L.SpjJoinGetStats.argtypes = [C.c_void_p, C.POINTER(SpjJoinStats)]
             L.SpjJoinResetStats.argtypes = [C.c_void_p]
+            L.SpjJoinPacketCalls.argtypes = [C.c_void_p]
+            L.SpjJoinPacketCalls.restype = C.c_uint64
             L.SpjKnnCreate.argtypes = [C.POINTER(SpjKnnConfig), C.POINTER(C.c_void_p)]
             L.SpjKnnRelease.argtypes = [C.c_void_p]
             L.SpjKnnRelease.restype = None
@@ -679,6 +682,10 @@ class SpatialJoin:
 
     def reset_stats(self):
         _check(lib().SpjJoinResetStats(self.h), "reset_stats", self._err)
+
+    def packet_calls(self) -> int:
+        """Probe calls that the packet kernels answered."""
+        return int(lib().SpjJoinPacketCalls(self.h))
 
     def __del__(self):
         if getattr(self, "h", None):

@@ -199,8 +199,8 @@ class VisitedBitmap:
         left anti and full joins), ascending, as int32."""
         count = C.c_uint64(0)
         s = _stream(self.words)
-        # room for all rows where that is little memory, else their count first;
-        # the result keeps only the memory of its own rows
+        # room for all rows where that is little memory, else their count first
+        # (a result that leaves over 1 MB of it unused is copied: 15 us)
         cap = self.n_rows if self.n_rows <= (1 << 22) else 0
         out = torch.empty((cap,), dtype=torch.int32, device=self.words.device)
         rc = lib().SpjVisitedCollect(_ptr(self.words), self.n_rows, int(visited), _ptr(out), cap,
@@ -213,7 +213,7 @@ class VisitedBitmap:
                                            _ptr(out), out.numel(), C.byref(count), s),
                    "visited collect")
         n = int(count.value)
-        return out if n == out.numel() else out[:n].clone()
+        return out[:n].clone() if out.numel() - n > (1 << 18) else out[:n]
 
     def bitmap(self) -> torch.Tensor:
         """The mark column of a mark join: Arrow LSB bits, one per row."""

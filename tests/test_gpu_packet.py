@@ -305,3 +305,34 @@ def test_packet_from_the_first_row_counts(capi, pred, n):
         np.testing.assert_array_equal(got[0][0], other[0])
         np.testing.assert_array_equal(got[0][1], other[1])
     assert len(got[0][0]) > 0 or pred == "touches"
+
+
+@pytest.mark.parametrize("build_rows,radius,n,pred,distance,packets", [
+    (2000, 20.0, 70000, "intersects", 0.0, 1),   # many probes in each build row's box
+    (2000, 20.0, 65535, "intersects", 0.0, 0),
+    (20000, 0.02, 70000, "contains", 0.0, 0),    # build rows that hardly any probe meets
+    (130000, 0.0, 2400, "dwithin", 0.01, 0),     # few probes, far apart
+    (130000, 0.0, 2400, "dwithin", 1.0, 1),      # many neighbours each
+    (130000, 0.0, 11000, "dwithin", 0.01, 1)])
+def test_packets_by_density(capi, build_rows, radius, n, pred, distance, packets):
+    """The path that the sizes choose, with the pairs of the other one."""
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(build_rows + n)
+    if radius:
+        turn = np.linspace(0, 2 * np.pi, 9)
+        ring = radius * np.stack([np.cos(turn), np.sin(turn)], 1)
+        ring[-1] = ring[0]
+        build = wkb.column_from_values([wkb.wkb_polygon([ring + c])
+                                        for c in rng.uniform(0, 200, (build_rows, 2))])
+    else:
+        build = wkb.points_column(*rng.uniform(0, 200, (2, build_rows)))
+    probe = wkb.points_column(*rng.uniform(0, 200, (2, n)))
+    got = []
+    for limit in (1 << 34, 0):
+        j = capi.SpatialJoin()
+        j.set_option("packet_bytes", limit)
+        j.build(build)
+        got.append(j.probe(probe, pred, distance=distance))
+        assert j.packet_calls() == (packets if limit else 0)
+    np.testing.assert_array_equal(got[0][0], got[1][0])
+    np.testing.assert_array_equal(got[0][1], got[1][1])
