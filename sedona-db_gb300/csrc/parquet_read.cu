@@ -941,7 +941,7 @@ struct SpjParquet {
   cudaEvent_t ev[6] = {};  // start, after H2D, after Snappy, after decode, values start, end
   PinnedBlock stage_h;  // (returned after release_device has waited for the stream)
   DevBuf stage, pages, pagebuf, dict_base, dict_n, dict_ptr, dict_len, valid, tmp_ptr, tmp_len,
-      vptr, vlen, pos, scan_tmp, out_off, out_data, out_valid, status, nulls, frag_base, frag_ip,
+      vptr, vlen, pos, scan_tmp, out_off, out_data, out_valid, status, frag_base, frag_ip,
       mode, work, walks, segs;
   double ms = 0, ms_phase[4] = {};  // H2D, decompress, decode, values
   uint64_t file_bytes = 0, page_bytes = 0, value_bytes = 0;
@@ -950,7 +950,7 @@ struct SpjParquet {
   void release_device() {
     for (DevBuf* b : {&stage, &pages, &pagebuf, &dict_base, &dict_n, &dict_ptr, &dict_len,
                       &valid, &tmp_ptr, &tmp_len, &vptr, &vlen, &pos, &scan_tmp, &out_off,
-                      &out_data, &out_valid, &status, &nulls, &frag_base, &frag_ip, &mode,
+                      &out_data, &out_valid, &status, &frag_base, &frag_ip, &mode,
                       &work, &walks, &segs})
       b->release();
     if (stream) {
@@ -1370,10 +1370,15 @@ extern "C" int SpjParquetReadWkb(SpjParquet* p, const char* column, int32_t rg_b
     p->out_off.reserve(8 * (n + 1), s);
     p->walks.reserve(sizeof(PageWalk) * (np + 1), s);
     p->segs.reserve(sizeof(Segment) * (nseg + 1), s);
-    p->status.reserve(8, s);
-    p->nulls.reserve(8, s);
-    SPJ_CUDA(cudaMemsetAsync(p->status.get(), 0, 8, s));
-    SPJ_CUDA(cudaMemsetAsync(p->nulls.get(), 0, 8, s));
+    // the error (code, page), the null rows and the value bytes, read back by one copy
+    struct ReadResult {
+      uint32_t err[2];
+      unsigned long long nulls;
+      uint64_t bytes;
+    } res{};
+    p->status.reserve(sizeof res, s);
+    SPJ_CUDA(cudaMemsetAsync(p->status.get(), 0, sizeof res, s));
+    ReadResult* dres = p->status.as<ReadResult>();
     const PageInfo* dpages = p->pages.as<PageInfo>();
     const uint8_t* dsrc = p->stage.as<uint8_t>();
     uint8_t* dpb = p->pagebuf.as<uint8_t>();
@@ -1403,7 +1408,7 @@ extern "C" int SpjParquetReadWkb(SpjParquet* p, const char* column, int32_t rg_b
                                                p->dict_len.as<uint32_t>(), st);
       RowArrays ra{p->valid.as<uint8_t>(),    p->tmp_ptr.as<uint64_t>(),
                    p->tmp_len.as<uint32_t>(), p->vptr.as<uint64_t>(),
-                   p->vlen.as<uint32_t>(),    p->nulls.as<unsigned long long>()};
+                   p->vlen.as<uint32_t>(),    &dres->nulls};
       PageWalk* walks = p->walks.as<PageWalk>();
       k_data_pages<<<grid_for((int64_t)np * 32, 128, kNumSMs * 16), 128, 0, s>>>(
           dpages, np, dsrc, dpb, p->dict_base.as<uint64_t>(), p->dict_n.as<uint32_t>(),
@@ -1420,17 +1425,14 @@ extern "C" int SpjParquetReadWkb(SpjParquet* p, const char* column, int32_t rg_b
       SPJ_CUDA(cudaGetLastError());
     }
     SPJ_CUDA(cudaEventRecord(p->ev[3], s));
-    uint32_t hst[2] = {0, 0};
-    SPJ_CUDA(cudaMemcpyAsync(hst, st, 8, cudaMemcpyDeviceToHost, s));
-    unsigned long long hnulls = 0;
-    SPJ_CUDA(cudaMemcpyAsync(&hnulls, p->nulls.get(), 8, cudaMemcpyDeviceToHost, s));
-    scan_u32_u64(p->vlen.as<uint32_t>(), p->pos.as<uint64_t>(), (int64_t)n, p->scan_tmp, s);
-    uint64_t vbytes = 0;
-    SPJ_CUDA(cudaMemcpyAsync(&vbytes, p->pos.as<uint64_t>() + n, 8, cudaMemcpyDeviceToHost, s));
+    scan_u32_u64_many(p->vlen.as<uint32_t>(), 0, p->pos.as<uint64_t>(), 0, (int64_t)n, 1,
+                      &dres->bytes, p->scan_tmp, s);
+    SPJ_CUDA(cudaMemcpyAsync(&res, dres, sizeof res, cudaMemcpyDeviceToHost, s));
     SPJ_CUDA(cudaStreamSynchronize(s));
-    if (hst[0]) {
-      const uint32_t bad = hst[1] < np ? hst[1] : 0;
-      throw Error(std::string("parquet: ") + pq::error_name(hst[0]) + " in page " +
+    const uint64_t vbytes = res.bytes;
+    if (res.err[0]) {
+      const uint32_t bad = res.err[1] < np ? res.err[1] : 0;
+      throw Error(std::string("parquet: ") + pq::error_name(res.err[0]) + " in page " +
                   std::to_string(bad) + " of the read (" + std::to_string(np) + " pages)");
     }
     p->value_bytes = vbytes;
@@ -1443,7 +1445,7 @@ extern "C" int SpjParquetReadWkb(SpjParquet* p, const char* column, int32_t rg_b
           p->vptr.as<uint64_t>(), p->vlen.as<uint32_t>(), p->pos.as<uint64_t>(), n,
           p->out_data.as<uint8_t>());
     const uint8_t* validity = nullptr;
-    if (hnulls) {
+    if (res.nulls) {
       p->out_valid.reserve(((n + 31) / 32) * 4 + 16, s);
       k_pack_valid<<<grid_for((int64_t)(n + 31) / 32, 256), 256, 0, s>>>(
           p->valid.as<uint8_t>(), n, p->out_valid.as<uint32_t>());
