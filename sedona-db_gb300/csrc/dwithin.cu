@@ -279,6 +279,13 @@ __global__ void __launch_bounds__(kTravThreads)
   }
 }
 
+// What a lane of k_dwithin_packet needs of its probe off the main loop.
+struct DwithinLane {
+  double2 p;
+  double d;
+  float cerr, d_lo, d_hi;
+};
+
 // The same for probes in Morton order, 32 neighbours to a traversal (a packet,
 // packet.cuh): a node is opened when any of their expanded boxes overlaps it,
 // and each build point of a leaf is loaded once and tested by all lanes.  Hits
@@ -287,7 +294,11 @@ __global__ void __launch_bounds__(kTravThreads)
 // traversal per probe was bound by divergence and by its node loads, and the
 // probes with over 64 neighbours were traversed again: 4M x 400k clustered
 // points: 7.5 ms with its second traversal and copies, 2.2 ms this way (1.6
-// here, 0.1 the packets, 0.5 the pairs); FP32 operations bound it now.
+// here, 0.1 the packets, 0.5 the pairs); FP32 operations and registers bound it
+// now.  Points are taken two at a time and what only the undecided ones need
+// (DwithinLane) lies in shared memory: together they pay for the count of
+// overlapping boxes (one point at a time in registers, the call took 3.20 ms
+// with that count and 3.02 without it; 3.05 this way).
 __global__ void __launch_bounds__(kTravThreads, 8)
     k_dwithin_packet(LbvhView t, const double2* __restrict__ bxy, const float4* __restrict__ bhl,
                      float bmag, int split_ok, const float4* __restrict__ probe_box,
@@ -296,6 +307,8 @@ __global__ void __launch_bounds__(kTravThreads, 8)
                      const uint32_t* __restrict__ order, uint32_t* __restrict__ counts,
                      PacketStore A, DeviceStatus* st) {
   __shared__ int stacks[kTravThreads / 32][kTravStack];
+  __shared__ DwithinLane lanes[kTravThreads];
+  DwithinLane& own = lanes[threadIdx.x];
   const unsigned all = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   int* stack = stacks[threadIdx.x >> 5];
@@ -319,10 +332,10 @@ __global__ void __launch_bounds__(kTravThreads, 8)
     if (have) q = probe_box[pi];
     const bool live = q.x <= q.z && q.y <= q.w && t.nprims > 0;
     double2 p = make_double2(0.0, 0.0);
-    double d = d0;
     float d_lo = d_lo0, d_hi = d_hi0;
     if (live) {
       p = probe_pt[pi];
+      double d = d0;
       if (d_row) {
         d = d_row[pi];
         d_lo = __double2float_rn(d);
@@ -330,10 +343,12 @@ __global__ void __launch_bounds__(kTravThreads, 8)
         if ((double)d_lo > d) d_lo = next_downf(d_lo);
         if ((double)d_hi < d) d_hi = next_upf(d_hi);
       }
+      own.p = p;
+      own.d = d;
     }
     const bool split =
         live && split_ok && fabs(p.x) <= kSplitMaxCoord && fabs(p.y) <= kSplitMaxCoord;
-    float hx = 0, hy = 0, lx = 0, ly = 0, cerr = 0;
+    float hx = 0, hy = 0, lx = 0, ly = 0;
     // d2 below in2: within d; above out2: farther (the point test of
     // k_dwithin_fused solved for d2, with slack for the rounding of the bounds);
     // between them that test decides
@@ -343,13 +358,30 @@ __global__ void __launch_bounds__(kTravThreads, 8)
       hy = __double2float_rn(p.y);
       lx = __double2float_rn(__dsub_rn(p.x, (double)hx));
       ly = __double2float_rn(__dsub_rn(p.y, (double)hy));
-      cerr = __fadd_ru(__fmul_ru(__fadd_ru(bmag, __fadd_ru(fabsf(hx), fabsf(hy))), kTwoM44),
-                       kTwoM120);
+      const float cerr =
+          __fadd_ru(__fmul_ru(__fadd_ru(bmag, __fadd_ru(fabsf(hx), fabsf(hy))), kTwoM44), kTwoM120);
+      own.cerr = cerr;
+      own.d_lo = d_lo;
+      own.d_hi = d_hi;
       const float a = __fmul_rd(__fsub_rd(d_lo, cerr), 0.999998f);
       if (a > 0.0f) in2 = __fmul_rd(a, a);
       const float b = __fmul_ru(__fadd_ru(d_hi, cerr), 1.000002f);
       out2 = __fmul_ru(b, b);
     }
+    auto dist2 = [&](const float4 h) {
+      const float dx = __fadd_rn(__fsub_rn(h.x, hx), __fsub_rn(h.z, lx));
+      const float dy = __fadd_rn(__fsub_rn(h.y, hy), __fsub_rn(h.w, ly));
+      return __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+    };
+    // point k, whose split distance squared lies between in2 and out2
+    auto decide = [&](uint32_t k, float d2) {
+      if (split) {
+        if (__fadd_ru(__fmul_ru(__fsqrt_ru(d2), kSplitUp), own.cerr) < own.d_lo) return true;
+        if (__fsub_rd(__fmul_rd(__fsqrt_rd(d2), kSplitDown), own.cerr) > own.d_hi) return false;
+      }
+      esc++;
+      return exact::dwithin_exact(bxy[k], own.p, own.d);
+    };
     uint32_t cnt = 0, nrec = 0, chunk = kNoChunk;
     int sp = 0;
     int node = t.nleaves > 1 ? 0 : ~0;
@@ -367,36 +399,34 @@ __global__ void __launch_bounds__(kTravThreads, 8)
           break;
         }
         const uint32_t b0 = c * t.leaf_size, b1 = min(b0 + t.leaf_size, t.nprims);
-        const bool near = live && box_overlap(t.leaf_box[c], q);
-        tested += near ? b1 - b0 : 0u;
+        bool near = live && box_overlap(t.leaf_box[c], q);
+        // the candidates are those of k_dwithin_fused: overlapping boxes, none
+        // in a leaf that lies farther than d as a whole (a point's box is its
+        // RN32 copy)
+        if (near && split && leaf_class(t.leaf_box[c], hx, hy, lx, ly, own.cerr, own.d_lo, own.d_hi) < 0)
+          near = false;
+        const float inn = near ? in2 : -1.0f;
         for (uint32_t k0 = b0; k0 < b1; k0 += 32) {
           uint32_t mask = 0;  // of point k0 + lane
           const uint32_t k1 = min(k0 + 32, b1);
-          for (uint32_t k = k0; k < k1; k++) {
-            const float4 h = bhl[k];
-            const float dx = __fadd_rn(__fsub_rn(h.x, hx), __fsub_rn(h.z, lx));
-            const float dy = __fadd_rn(__fsub_rn(h.y, hy), __fsub_rn(h.w, ly));
-            const float d2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-            bool hit = near && split && d2 < in2;
-            const bool open = near && (!split || (!hit && !(d2 > out2)));
-            if (__any_sync(all, open)) {
-              if (open) {
-                int r = -1;
-                if (split) {
-                  if (__fadd_ru(__fmul_ru(__fsqrt_ru(d2), kSplitUp), cerr) < d_lo) r = 1;
-                  else if (__fsub_rd(__fmul_rd(__fsqrt_rd(d2), kSplitDown), cerr) > d_hi) r = 0;
-                }
-                if (r < 0) {
-                  esc++;
-                  r = box_overlap(t.sorted_box[k], q) && exact::dwithin_exact(bxy[k], p, d) ? 1 : 0;
-                }
-                hit = r != 0;
-              }
+          for (uint32_t k = k0; k < k1; k += 2) {
+            const bool two = k + 1 < k1;
+            const float4 a = bhl[k], b = bhl[two ? k + 1 : k];
+            const float da = dist2(a), db = two ? dist2(b) : qnan;
+            const bool ina = near && a.x >= q.x && a.x <= q.z && a.y >= q.y && a.y <= q.w;
+            const bool inb = near && two && b.x >= q.x && b.x <= q.z && b.y >= q.y && b.y <= q.w;
+            tested += (ina ? 1u : 0u) + (inb ? 1u : 0u);
+            bool hita = da < inn, hitb = db < inn;
+            const bool opena = ina && !hita && !(da > out2), openb = inb && !hitb && !(db > out2);
+            if (__any_sync(all, opena || openb)) {
+              if (opena) hita = decide(k, da);
+              if (openb) hitb = decide(k + 1, db);
               __syncwarp();
             }
-            const unsigned hits = __ballot_sync(all, hit);
-            cnt += hit ? 1u : 0u;
-            if (lane == (int)(k - k0)) mask = hits;
+            const unsigned ma = __ballot_sync(all, hita), mb = __ballot_sync(all, hitb);
+            cnt += (hita ? 1u : 0u) + (hitb ? 1u : 0u);
+            if (lane == (int)(k - k0)) mask = ma;
+            if (lane == (int)(k + 1 - k0)) mask = mb;
           }
           const uint32_t id = mask ? t.sorted_id[k0 + lane] : 0u;
           packet_append(A, g, lane, mask != 0, make_uint2(id, mask), nrec, chunk);

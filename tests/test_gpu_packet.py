@@ -261,6 +261,30 @@ def test_packet_dwithin_same_pairs_and_positions(capi, n, leaf):
             np.testing.assert_array_equal(got[0][1], got[1][1])
 
 
+@pytest.mark.parametrize("leaf", [1, 16, 33, 64])
+def test_packet_dwithin_counts_the_same_candidates(capi, leaf):
+    """The statistics of the packet traversal are those of the traversal per probe:
+    boxes that overlap, of leaves that are not farther as a whole."""
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(leaf)
+    build = wkb.points_column(*np.concatenate([rng.normal(50, 3, (2, 3000)),
+                                               rng.uniform(0, 100, (2, 2000))], 1))
+    probe = wkb.points_column(*rng.uniform(0, 100, (2, 700)))
+    far = wkb.column_from_values([wkb.wkb_point(1e30, 1.0), wkb.wkb_point(50.0, 50.0)] * 40)
+    for pts in (probe, far):
+        for d in (0.0, 0.7, 6.0, 90.0):
+            got = []
+            for limit in (1 << 34, 0):
+                j = capi.SpatialJoin(probe_order=1, leaf_size=leaf)
+                j.set_option("packet_bytes", limit)
+                j.build(build)
+                b, _ = j.probe(pts, "dwithin", distance=d)
+                st = j.stats()
+                got.append((len(b), st["candidates"], st["pairs_evaluated"]))
+                assert j.packet_calls() == (1 if limit else 0)
+            assert got[0] == got[1]
+
+
 @pytest.mark.parametrize("n", [1, 31, 4096, 4097, 8193, 16384, 16385, 20001])
 @pytest.mark.parametrize("order", [-1, 1])
 def test_scans_and_sorts_at_the_sizes_of_one_block(capi, n, order):
