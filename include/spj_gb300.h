@@ -626,6 +626,10 @@ uint64_t SpjAllocationCount(void);
 
 int SpjHostRegister(void* ptr, uint64_t bytes);
 int SpjHostUnregister(void* ptr);
+/* Gives back the page-locked host memory that GeoParquet reads keep for the next
+ * file (at most 256 MB a process); returns the bytes.  Releasing a runtime does
+ * the same.  Blocks of reads under way are not touched; any thread may call. */
+uint64_t SpjHostTrim(void);
 /* Library version string. */
 const char* SpjVersion(void);
 

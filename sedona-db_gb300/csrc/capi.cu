@@ -1546,6 +1546,8 @@ extern "C" int SpjHostUnregister(void* ptr) {
   return e == cudaSuccess ? 0 : EINVAL;
 }
 
+extern "C" uint64_t SpjHostTrim(void) { return pinned_trim(); }
+
 extern "C" const char* SpjVersion(void) { return "spj-gb300 0.1.0 (sm_103a)"; }
 
 namespace spj {
@@ -1593,6 +1595,10 @@ void* pinned_take(size_t& bytes) {
 }
 
 void pinned_give(void* p, size_t bytes) {
+  if (bytes > kPinnedHeld) {
+    cudaFreeHost(p);
+    return;
+  }
   PinnedPool& pool = pinned_pool();
   std::vector<void*> out;
   {
@@ -1608,15 +1614,17 @@ void pinned_give(void* p, size_t bytes) {
   for (void* q : out) cudaFreeHost(q);
 }
 
-void pinned_trim() {
+size_t pinned_trim() {
   PinnedPool& pool = pinned_pool();
   std::vector<PinnedPool::Block> out;
+  size_t bytes = 0;
   {
     std::lock_guard<std::mutex> lk(pool.mu);
     out.swap(pool.free);
-    pool.held = 0;
+    std::swap(bytes, pool.held);
   }
   for (auto& b : out) cudaFreeHost(b.p);
+  return bytes;
 }
 
 }  // namespace spj

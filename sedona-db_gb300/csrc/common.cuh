@@ -202,12 +202,13 @@ class PinnedBuf {
 // their decode.  pinned_take returns a free block of at least `bytes` (and sets
 // bytes to its size) or locks a new one; pinned_give returns it, with no copy
 // to or from it in flight.  At most kPinnedHeld bytes stay locked (the longest
-// unused are unlocked first); pinned_trim unlocks all that are free, which
-// releasing a runtime does.  Safe from any thread; defined in capi.cu.
+// unused are unlocked first, a block over that at once); pinned_trim unlocks all
+// that are free and returns their bytes, which SpjHostTrim and releasing a
+// runtime do.  Safe from any thread; defined in capi.cu.
 constexpr size_t kPinnedHeld = 256u << 20;
 void* pinned_take(size_t& bytes);
 void pinned_give(void* p, size_t bytes);
-void pinned_trim();
+size_t pinned_trim();
 
 // A grow-only buffer of such a block (contents not preserved).  Its owner
 // waits for its copies before it grows or goes.

@@ -192,7 +192,8 @@ EXPORTS = [
     "SpjJoinPacketCalls",
     "SpjKnnCreate", "SpjKnnRelease", "SpjKnnLastError", "SpjKnnBuild", "SpjKnnQuery",
     "SpjKnnQueryTies", "SpjKnnQueryArrow", "SpjJoinSetProbeDistances",
-    "SpjKnnStream", "SpjKnnGetStats", "SpjHostRegister", "SpjHostUnregister", "SpjVersion",
+    "SpjKnnStream", "SpjKnnGetStats", "SpjHostRegister", "SpjHostUnregister", "SpjHostTrim",
+    "SpjVersion",
     "SpjIndexProbeNoAlloc", "SpjAllocationCount",
     "SpjMaterializeLastError", "SpjGatherFixed", "SpjGatherValidity", "SpjGatherBinary",
     "SpjGatherColumns", "SpjGatherColumnsData", "SpjVisitedMark", "SpjVisitedCollect",
@@ -332,6 +333,8 @@ def lib() -> C.CDLL:
             L.SpjAllocationCount.restype = C.c_uint64
             L.SpjHostRegister.argtypes = [C.c_void_p, C.c_uint64]
             L.SpjHostUnregister.argtypes = [C.c_void_p]
+            L.SpjHostTrim.argtypes = []
+            L.SpjHostTrim.restype = C.c_uint64
             L.SpjVersion.restype = C.c_char_p
             L.SpjStreamCreate.argtypes = [C.c_void_p, C.POINTER(C.c_void_p)]
             L.SpjStreamRelease.argtypes = [C.c_void_p]

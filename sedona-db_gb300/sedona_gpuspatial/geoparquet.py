@@ -104,6 +104,12 @@ class GeoParquetFile:
         self.close()
 
 
+def trim() -> int:
+    """Gives back the page-locked memory that reads keep for the next file; returns
+    its bytes."""
+    return int(lib().SpjHostTrim())
+
+
 def write_wkb(path: str, col: WkbColumn, column: str = "geometry", compression: str = "snappy",
               page_version: int = 1, row_group_rows: int = 0, page_bytes: int = 0):
     """Writes ``col`` as a GeoParquet file with one WKB column."""

@@ -226,3 +226,21 @@ def test_files_share_page_locked_blocks(gp, tmp_path):
     for t in threads:
         t.join()
     assert not bad, bad[0]
+
+
+def test_trim_gives_back_page_locked_blocks(gp, tmp_path):
+    """What closed files leave can be given back, what an open one uses cannot."""
+    from sedona_gpuspatial import wkb
+    path = str(tmp_path / "t.parquet")
+    off = np.arange(0, 21 * 501, 21, dtype=np.int64)
+    data = np.arange(off[-1]).astype(np.uint8)
+    gp.write_wkb(path, wkb.WkbColumn(off, data, None))
+    gp.trim()
+    with gp.GeoParquetFile(path) as f:
+        f.read_wkb()
+        assert gp.trim() == 0
+        _assert_column(gp.device_to_host(f.read_wkb()), off, data, np.ones(500, bool))
+    assert os.path.getsize(path) // 2 < gp.trim() <= 256 << 20
+    assert gp.trim() == 0
+    with gp.GeoParquetFile(path) as f:
+        _assert_column(gp.device_to_host(f.read_wkb()), off, data, np.ones(500, bool))
