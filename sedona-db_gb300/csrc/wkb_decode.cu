@@ -235,28 +235,6 @@ __global__ void k_wkb_struct(WkbDeviceColumn col, bool al, const uint8_t* __rest
 
 __device__ __forceinline__ bool feq(double x, double y) { return !((x < y) | (x > y)); }
 
-// Integers that order like doubles (NaN left out): one signed comparison.
-__device__ __forceinline__ long long f64_key(double x) {
-  const long long b = __double_as_longlong(x);
-  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
-}
-__device__ __forceinline__ double f64_of_key(long long k) {
-  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
-}
-
-// x rounded to the nearest float, ties to even, on the integer units for
-// values in the float's normal range.
-__device__ __forceinline__ float f64_to_f32(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const uint32_t e = (uint32_t)(b >> 52) & 0x7ffu;
-  if (e < 897u || e > 1150u) return __double2float_rn(x);
-  const uint32_t low = (uint32_t)b & 0x1fffffffu;  // the 29 bits that are dropped
-  uint32_t f = (uint32_t)(b >> 32) & 0x80000000u;
-  f |= (e - 896u) << 23 | ((uint32_t)(b >> 29) & 0x7fffffu);
-  f += (low > 0x10000000u || (low == 0x10000000u && (f & 1u))) ? 1u : 0u;
-  return __uint_as_float(f);
-}
-
 // kG lanes per ring (8 for columns of small rings such as building
 // footprints, 32 otherwise); consecutive groups take consecutive rings.
 // Each ring is a chain of dependent loads (its source offset, then its

@@ -121,6 +121,38 @@ def test_packet_far_offset_and_huge_probes(capi):
         pass
 
 
+@pytest.mark.parametrize("sizes", [(1023, 1024), (1024, 1025), (5000, 300), (65535, 65536, 70000, 40)])
+def test_packet_large_rings(capi, oracle_lib, sizes):
+    """Rings of both sides of what one block indexes (1,024 edges) and of what has
+    an index at all (65,535), beside small ones; one whose edges crowd in a cell
+    (over 255, so the grid does not answer there); with and without holes."""
+    from sedona_gpuspatial import wkb
+    rng = np.random.default_rng(len(sizes) + sizes[0])
+    zones = []
+    for k, n in enumerate(sizes):
+        c = rng.uniform(60, 140, 2)
+        shell = _star(rng, c, n, 60.0)
+        zones.append(wkb.wkb_polygon([shell] + ([(c + (shell - c) / 3.0)[::-1]] if k % 2 else [])))
+    ang = np.sort(rng.uniform(0, 2 * np.pi, 900))
+    rad = np.where(np.arange(900) % 2, 40.0, 1e-3)
+    spikes = 100.0 + np.stack([rad * np.cos(ang), rad * np.sin(ang)], 1)
+    zones.append(wkb.wkb_polygon([np.vstack([spikes, spikes[:1]])]))
+    zones += _zones(rng, 20, holes=True)
+    build = wkb.column_from_values(zones)
+    assert max(len(z) for z in zones) > 16 * max(sizes)
+    for kind, n in (("points", 400), ("polygons", 120)):
+        rows = _probes(rng, n, kind, zones)
+        rows += [wkb.wkb_point(*(100.0 + rng.uniform(-0.1, 0.1, 2))) if kind == "points" else
+                 wkb.wkb_polygon([_star(rng, 100.0 + rng.uniform(-2, 2, 2), 5, 1.0)])
+                 for _ in range(40)]
+        probe = wkb.column_from_values(rows)
+        for pred, b, p in _both(capi, build, probe, PREDS):
+            if pred in ("intersects", "contains"):
+                ob, op = oracle_lib.join(oracle_lib.Geoms(build), oracle_lib.Geoms(probe), pred,
+                                         nthreads=8)
+                assert pairs(b, p) == sorted(zip(op.tolist(), ob.tolist())), pred
+
+
 def test_packet_capacities_grow(capi):
     """More records and more open pairs than the first guess has room for."""
     from sedona_gpuspatial import wkb
