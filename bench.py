@@ -238,6 +238,7 @@ def run_ours(args, world, rank, local, pg, light=False, workload=None, pred_over
         ms = barrier_max(pg, ms, dev)
         st = j.stats()
         results[name] = {"ms": ms, "pairs": npairs, "stats": st,
+                         "packets": j.packet_calls() > 0,
                          "clocks": sampler.summary() if sampler else None, "join": j}
     chosen = results["chosen"]
     st = chosen["stats"]
@@ -331,31 +332,39 @@ def run_ours(args, world, rank, local, pg, light=False, workload=None, pred_over
         del jv
 
 
-    # roofline of the dominant kernel (refine) over the timed steps
+    # roofline of the dominant kernels over the timed steps, by the path that ran
     hbm_peak, peak_kind = load_peaks()
     probe_vpr = probe_vertices_per_row(inp.probe)
     build_vbytes = int(st["build_vertices"]) * 16
-    ref_bytes = algorithmic_refine_bytes({"candidates": st["candidates"] / steps}, probe_vpr,
-                                         build_vbytes)
-    ref_ms = st["ms_refine"] / steps
-    achieved = ref_bytes / (ref_ms * 1e-3) / 1e9 if ref_ms > 0 else 0.0
-    kernel = "k_packet (+ k_packet_open)"
+    bound = "hbm"
     if pred == "dwithin":
-        # point-point ST_DWithin is decided inside the traversal (records of
-        # hits, then their pairs, no candidate pairs): per probe row its point
-        # and box (32 B) and a count (4 B), 8 B per result pair, the build
-        # points (FP64 + FP32 splits, 32 B) once
-        kernel = "k_dwithin_packet + k_packet_scatter"
+        # point-point ST_DWithin is decided inside the traversal (no candidate
+        # pairs): per probe row its point and box (32 B) and a count (4 B), 8 B
+        # per result pair, the build points (FP64 + FP32 splits, 32 B) once
+        kernel = "k_dwithin_packet + k_packet_scatter" if chosen["packets"] else "k_dwithin_fused"
         ref_bytes = n_rows * 36 + 8 * chosen["pairs"] + 32 * len(inp.build)
         ref_ms = (st["ms_refine"] + st["ms_compact"]) / steps
-        achieved = ref_bytes / (ref_ms * 1e-3) / 1e9 if ref_ms > 0 else 0.0
+    elif chosen["packets"]:
+        # neither candidate pairs nor flags: per probe row its vertices (16 B
+        # each), box and count (20 B), the build vertices once, 8 B per result
+        # pair.  These kernels are bound by their instructions
+        bound = "instructions"
+        kernel = "k_packet + k_packet_open + k_packet_scatter"
+        ref_bytes = n_rows * (16 * probe_vpr + 20) + build_vbytes + 8 * chosen["pairs"]
+        ref_ms = (st["ms_refine"] + st["ms_compact"]) / steps
+    else:
+        kernel = "k_refine"
+        ref_bytes = algorithmic_refine_bytes({"candidates": st["candidates"] / steps}, probe_vpr,
+                                             build_vbytes)
+        ref_ms = st["ms_refine"] / steps
+    achieved = ref_bytes / (ref_ms * 1e-3) / 1e9 if ref_ms > 0 else 0.0
     traffic = None
     traffic_note = None
     tf = os.path.join(ROOT, "profiles", f"refine_traffic_workload{workload}.json")
     if os.path.exists(tf) and pred == "intersects":
         with open(tf) as f:
             tj = json.load(f)
-        if tj.get("kernel", "").split("<")[0] in kernel:  # of the kernel that ran
+        if tj.get("kernel", "").split("<")[0] == kernel:  # of the kernel that ran
             traffic = tj.get("bytes_per_launch")
             traffic_note = tj.get("scaled_from")
 
@@ -396,7 +405,7 @@ def run_ours(args, world, rank, local, pg, light=False, workload=None, pred_over
                 "ms_per_step": e2e_ms,
                 "h2d_bytes_per_step": int(off.nbytes + data.nbytes),
                 "d2h_bytes_per_step": int(8 * n_e2e)},
-        "roofline": {"bound": "hbm", "kernel": kernel, "achieved": achieved,
+        "roofline": {"bound": bound, "kernel": kernel, "achieved": achieved,
                      "peak": hbm_peak, "peak_kind": peak_kind, "unit": "GB/s",
                      "frac": achieved / hbm_peak, "traffic": traffic,
                      "algorithmic_bytes_per_launch": ref_bytes},
@@ -660,7 +669,7 @@ def run_stream(args, world, rank, local, pg):
                 "d2h_bytes_per_step": int(8 * npairs)},
         "gpu_launches": int(sstats["launches_per_replay"] * args.steps),
         "fp64_escalations_per_replay": sstats["escalations"] / max(1, args.steps + args.warmup + 2),
-        "roofline": {"bound": "hbm", "kernel": "stream replay (decode, traversal, refine, compact)",
+        "roofline": {"bound": "hbm", "kernel": "stream replay (decode, order, packets, pairs)",
                      "achieved": achieved, "peak": hbm_peak, "peak_kind": peak_kind,
                      "unit": "GB/s", "frac": achieved / hbm_peak, "traffic": None,
                      "algorithmic_bytes_per_launch": alg},
@@ -1199,7 +1208,7 @@ def run_materialize(args, local):
                  for i in sample)
     seen = torch.bincount(bi.long(), minlength=nb) > 0
     ok_vis = bool(torch.equal(un.long(), torch.nonzero(~seen).flatten()))
-    # roofline of the binary gather (k_bin_lengths + scan + k_bin_copy, run
+    # roofline of the binary gather (k_gather_columns + scan + k_bin_copy, run
     # twice by take_binary: a sizing call, then the copy): value bytes read
     # and written, per pair its index and the source offsets (12 B) and the
     # output offset (8 B), twice for the sizing pass
@@ -1220,11 +1229,12 @@ def run_materialize(args, local):
         "value": npairs / (ms * 1e-3), "unit": "pairs/s", "ms_per_step": ms, "steps": steps,
         "warmup": warmup,
         "phases_ms_per_step": {"probe_wkb_take_binary": bin_ms},
-        "roofline": {"bound": "hbm", "kernel": "k_bin_copy (+ k_bin_lengths, scan)",
+        "roofline": {"bound": "hbm", "kernel": "k_bin_copy (+ k_gather_columns, scan)",
                      "achieved": achieved, "peak": hbm_peak, "peak_kind": peak_kind,
                      "unit": "GB/s", "frac": achieved / hbm_peak, "traffic": None,
                      "algorithmic_bytes_per_launch": alg},
-        "gpu_launches": 26 * steps,
+        # values and lengths 1, scan 3, copy 1, mark 1, collect 3
+        "gpu_launches": 9 * steps,
         "parity": {"id_columns_equal": ok_ids, "wkb_lengths_equal": ok_len,
                    "wkb_sampled_values_equal": bool(ok_val), "unmatched_rows_equal": ok_vis,
                    "pairs": npairs},
