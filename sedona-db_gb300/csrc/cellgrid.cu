@@ -13,11 +13,10 @@
 // with an edge whose side of the centre is not decided is not answered).
 //
 // Every edge visits the cells of its bbox (6 or 7 for the zones' rings of 145
-// vertices and 26 x 26 cells), twice: to count and to fill.  (When each cell
-// scanned the bands it spans instead, some 50 edges a cell, 50k zones took
-// 4.47 ms; counting and filling take 0.46 + 1.97.)  A point in a mixed cell reads the 2 or 3 edges of its cell where the
-// y-band scan reads some 10, and a box those of the cells it lies in where that
-// reads 20.
+// vertices and 26 x 26 cells), twice: to count and to fill, 0.46 + 1.97 ms for
+// 50k zones.  (4.47 when each cell scanned the some 50 edges of the bands that
+// it spans.)  A packet (packet.cu) reads the 2 or 3 edges of a mixed cell where
+// the y-band scan of a point reads some 10, and of a box some 20.
 #include "geoms.cuh"
 #include "predicates.cuh"
 #include "prims.cuh"

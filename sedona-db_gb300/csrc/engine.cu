@@ -99,9 +99,12 @@ static inline float ev_ms(cudaEvent_t a, cudaEvent_t b) {
 }
 
 bool packet_pays(int predicate, bool points, uint64_t rows, const PacketTree& t) {
-  if (predicate == kPredDWithin)
-    return rows >= kPacketRowsDWithin &&
-           (t.nprims <= 100000 || rows * 12 >= t.nprims || t.crowd >= 1.0);
+  if (predicate == kPredDWithin) {
+    if (rows < kPacketRowsDWithin) return false;
+    // (the sort of the rows, by tiles but not otherwise needed)
+    if (t.nprims <= 8192 && rows > 16384 && rows < kOrderMinRows) return t.crowd >= 8.0;
+    return t.nprims <= 250000 || rows <= 4096 || rows * 12 >= t.nprims || t.crowd >= 1.0;
+  }
   const bool first = predicate == kIntersects || predicate == kDisjoint;
   if (rows < (points || first ? kOrderMinRows : kPacketRowsFull)) return false;
   const double covers = t.share * t.nprims, held = t.share * rows;
@@ -123,11 +126,11 @@ bool packet_pays(int predicate, bool points, uint64_t rows, const PacketTree& t)
 PacketTree JoinEngine::packet_tree(double distance) const {
   PacketTree t;
   t.nprims = bvh_.nprims;
-  t.share = bvh_.extent_area > 0.0f
-                ? std::min(1.0, (double)bvh_.mean_w * bvh_.mean_h / bvh_.extent_area)
+  t.share = bvh_.spread_area > 0.0f
+                ? std::min(1.0, (double)bvh_.mean_w * bvh_.mean_h / bvh_.spread_area)
                 : 1.0;
   t.holes = bg_.nrings > bg_.nparts;
-  t.crowd = 4.0 * distance * distance * bvh_.leaf_density;
+  t.crowd = std::isfinite(distance) ? 4.0 * distance * distance * bvh_.leaf_density : 1e30;
   return t;
 }
 

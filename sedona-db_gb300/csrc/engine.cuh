@@ -48,7 +48,8 @@ struct EngineConfig {
   int dwithin_arena = 2;
   // (candidate_order, order_tiles, refine_min_blocks and refine_split are of the
   // candidate pairs' path and their figures are its; ordered probe rows take the
-  // packet kernels unless one of them is set: 2M x 50k polygons 18.1 ms)
+  // packet kernels where these pay unless one of them is set: 2M x 50k polygons
+  // 18.1 ms)
   // refine order of the candidates: 0 as listed (by probe row), 2 by build
   // row then probe Morton rank (a warp then tests one build geometry's edges
   // against neighbouring probes: shared loads and similar trip counts; 2M x
@@ -118,9 +119,9 @@ constexpr uint32_t kOrderMinRows = 1u << 16;
 //    50k clustered buildings (0.02 met) 647 / 568;
 //  - within, covered by, equals: 5k zones (6.4 met) 16k rows 246 / 239, 50k 472 / 586;
 //  - ST_DWithin, by how many points of a middling leaf's density the square of
-//    twice the distance holds (crowd): 400k points, 4k rows: 2 m 400 / 315, 10 m
-//    (0.8) 624 / 427, 30 m (6.9) 740 / 1,066; 32k rows: 339 / 334, 461 / 469,
-//    693 / 1,121; 100k points, 2k rows: 269 / 250, 283 / 288, 329 / 484.
+//    twice the distance holds (crowd): 400k points, 16k rows: 5 m 510 / 456, 10 m
+//    (0.8) 582 / 528, 20 m (3) 690 / 821; 4k rows at 10 m 490 / 523; 200k points,
+//    16k rows: 5 m 411 / 427; 5k points, 20k rows 200 / 172.
 constexpr uint32_t kPacketRowsDWithin = 1u << 11;
 constexpr uint32_t kPacketRowsFull = 1u << 13;
 struct PacketTree {

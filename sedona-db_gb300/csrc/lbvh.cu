@@ -49,11 +49,18 @@ __global__ void k_compact_ids(const uint8_t* __restrict__ flag, const uint64_t* 
 }
 
 // ext[0..3]: extent of the box centres (order-preserving integers); sums[0..1]:
-// total box width and height
+// total box width and height, sums[2..3]: total x and y distance between the
+// centres of kSpreadPairs (or m) pairs of rows drawn by a hash
+constexpr uint32_t kSpreadPairs = 1u << 16;
+__device__ __forceinline__ uint32_t hashed_row(uint64_t i, uint32_t m) {
+  uint64_t z = i * 0x9E3779B97F4A7C15ull;
+  z = (z ^ (z >> 32)) * 0xD6E8FEB86659FD93ull;
+  return (uint32_t)(((z ^ (z >> 32)) >> 32) * m >> 32);
+}
 __global__ void k_bounds(const float4* __restrict__ boxes, const uint32_t* __restrict__ ids,
                          uint32_t m, uint32_t* __restrict__ ext, float* __restrict__ sums) {
   float mnx = INFINITY, mny = INFINITY, mxx = -INFINITY, mxy = -INFINITY;
-  float w = 0.0f, h = 0.0f;
+  float w = 0.0f, h = 0.0f, dx = 0.0f, dy = 0.0f;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m;
        i += (int64_t)gridDim.x * blockDim.x) {
     float4 b = boxes[ids[i]];
@@ -64,6 +71,11 @@ __global__ void k_bounds(const float4* __restrict__ boxes, const uint32_t* __res
     mxy = fmaxf(mxy, cy);
     w += b.z - b.x;
     h += b.w - b.y;
+    if (i < kSpreadPairs) {
+      const float4 p = boxes[ids[hashed_row(2 * i + 1, m)]], q = boxes[ids[hashed_row(2 * i + 2, m)]];
+      dx += fabsf(0.5f * (p.x + p.z) - 0.5f * (q.x + q.z));
+      dy += fabsf(0.5f * (p.y + p.w) - 0.5f * (q.y + q.w));
+    }
   }
   for (int o = 16; o > 0; o >>= 1) {
     mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
@@ -72,6 +84,8 @@ __global__ void k_bounds(const float4* __restrict__ boxes, const uint32_t* __res
     mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
     w += __shfl_xor_sync(0xffffffffu, w, o);
     h += __shfl_xor_sync(0xffffffffu, h, o);
+    dx += __shfl_xor_sync(0xffffffffu, dx, o);
+    dy += __shfl_xor_sync(0xffffffffu, dy, o);
   }
   if ((threadIdx.x & 31) == 0) {
     atomicMin(&ext[0], f2o(mnx));
@@ -80,6 +94,8 @@ __global__ void k_bounds(const float4* __restrict__ boxes, const uint32_t* __res
     atomicMax(&ext[3], f2o(mxy));
     if (w != 0.0f) atomicAdd(&sums[0], w);
     if (h != 0.0f) atomicAdd(&sums[1], h);
+    if (dx != 0.0f) atomicAdd(&sums[2], dx);
+    if (dy != 0.0f) atomicAdd(&sums[3], dy);
   }
 }
 
@@ -665,14 +681,14 @@ void build_lbvh(const float4* boxes, uint32_t n, uint32_t leaf_size, Lbvh& out, 
   out.leaf_box.reserve((size_t)(L > 0 ? L : 1) * sizeof(float4), s);
   out.fault.reserve(8, s);
   SPJ_CUDA(cudaMemsetAsync(out.fault.get(), 0, 8, s));
-  out.mean_w = out.mean_h = out.extent_area = 0.0f;
-  out.leaf_density = 0.0;
+  out.mean_w = out.mean_h = out.extent_area = out.spread_area = out.leaf_density = 0.0f;
   if (m == 0) return;
   uint32_t* ids = out.sorted_id.as<uint32_t>();
   k_compact_ids<<<g, 256, 0, s>>>(flag.as<uint8_t>(), pos.as<uint64_t>(), n, ids);
-  DevBuf ext(28, s);
-  uint32_t init[7] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u};
-  SPJ_CUDA(cudaMemcpyAsync(ext.get(), init, 28, cudaMemcpyHostToDevice, s));
+  constexpr size_t kExt = 36;  // the extent, then five sums
+  DevBuf ext(kExt, s);
+  uint32_t init[9] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+  SPJ_CUDA(cudaMemcpyAsync(ext.get(), init, kExt, cudaMemcpyHostToDevice, s));
   const int gm = grid_for(m, 256);
   k_bounds<<<gm, 256, 0, s>>>(boxes, ids, m, ext.as<uint32_t>(), ext.as<float>() + 4);
   DevBuf keys((size_t)m * 4, s), akeys((size_t)m * 4, s), avals((size_t)m * 4, s);
@@ -681,7 +697,7 @@ void build_lbvh(const float4* boxes, uint32_t n, uint32_t leaf_size, Lbvh& out, 
                    tmp, s);
   k_gather_boxes<<<gm, 256, 0, s>>>(boxes, ids, m, out.sorted_box.as<float4>());
   k_leaf_boxes<<<grid_for(L, 256), 256, 0, s>>>(out.sorted_box.as<float4>(), m, L, leaf_size,
-                                                out.leaf_box.as<float4>(), ext.as<float>() + 6);
+                                                out.leaf_box.as<float4>(), ext.as<float>() + 8);
   if (L > 1) {
     DevBuf parent_int((size_t)L * 4, s), parent_leaf((size_t)L * 4, s), visits((size_t)L * 4, s);
     SPJ_CUDA(cudaMemsetAsync(visits.get(), 0, (size_t)L * 4, s));
@@ -693,17 +709,22 @@ void build_lbvh(const float4* boxes, uint32_t n, uint32_t leaf_size, Lbvh& out, 
                                              out.node_box.as<float4>(), visits.as<unsigned>());
   }
   SPJ_CUDA(cudaGetLastError());
-  uint32_t e[7];
-  SPJ_CUDA(cudaMemcpyAsync(e, ext.get(), 28, cudaMemcpyDeviceToHost, s));
+  uint32_t e[9];
+  SPJ_CUDA(cudaMemcpyAsync(e, ext.get(), kExt, cudaMemcpyDeviceToHost, s));
   SPJ_CUDA(cudaStreamSynchronize(s));
-  float sums[3];
-  memcpy(sums, e + 4, 12);
+  float sums[5];
+  memcpy(sums, e + 4, 20);
   const float area = (o2f(e[2]) - o2f(e[0])) * (o2f(e[3]) - o2f(e[1]));
+  // two places spread over a width lie a third of it apart on average
+  const float pairs = (float)std::min(m, kSpreadPairs);
+  const float spread = (3.0f * sums[2] / pairs) * (3.0f * sums[3] / pairs);
   const bool ok = std::isfinite(sums[0]) && std::isfinite(sums[1]) && std::isfinite(area);
   out.mean_w = ok ? sums[0] / (float)m : 0.0f;
   out.mean_h = ok ? sums[1] / (float)m : 0.0f;
   out.extent_area = ok ? area : 0.0f;
-  out.leaf_density = std::isfinite(sums[2]) ? leaf_size * std::exp2(-(double)sums[2] / L) : 0.0;
+  out.spread_area = ok && std::isfinite(spread) ? spread : 0.0f;
+  const double density = leaf_size * std::exp2(-(double)sums[4] / L);
+  out.leaf_density = std::isfinite(sums[4]) && density < 1e30 ? (float)density : 0.0f;
 }
 
 void check_traversal(const LbvhView& t, cudaStream_t s) {

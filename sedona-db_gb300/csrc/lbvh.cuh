@@ -32,14 +32,17 @@ struct LbvhView {
   // mean primitive box and the area of the boxes' centres' extent (estimates
   // of how many primitives a box meets; 0 when not finite)
   float mean_w = 0.0f, mean_h = 0.0f, extent_area = 0.0f;
+  // primitives per area in a middling leaf (the geometric mean of the leaves'
+  // areas: of clustered points most lie far denser than over the extent)
+  float leaf_density = 0.0f;
 };
 
 struct Lbvh {
   uint32_t nprims = 0, nleaves = 0, leaf_size = 4;
-  float mean_w = 0.0f, mean_h = 0.0f, extent_area = 0.0f;
-  // primitives per area in a middling leaf (the geometric mean of the leaves'
-  // areas: of clustered points most lie far denser than over the extent)
-  double leaf_density = 0.0;
+  float mean_w = 0.0f, mean_h = 0.0f, extent_area = 0.0f, leaf_density = 0.0f;
+  // the area that the centres spread over, by the mean distance of two of them
+  // (the extent is at the mercy of one row far off)
+  float spread_area = 0.0f;
   DevBuf sorted_box, sorted_id, node_box, node_child, leaf_box, fault;
   LbvhView view() const {
     LbvhView v;
@@ -55,6 +58,7 @@ struct Lbvh {
     v.mean_w = mean_w;
     v.mean_h = mean_h;
     v.extent_area = extent_area;
+    v.leaf_density = leaf_density;
     return v;
   }
   size_t device_bytes() const {

@@ -23,14 +23,15 @@
 // the masks into pairs; records are in traversal order, so every probe row's
 // pairs come in the order of the candidate pairs' path.
 //
-// 2M buildings x 50k zones, ST_Intersects: 40.5 -> 18.2 ms a step (refine 28.5,
+// 2M buildings x 50k zones, ST_Intersects: 40.5 -> 18.1 ms a step (refine 28.5,
 // traversal 3.6, ordering and compaction of 132M pairs 4.9 before; k_packet
-// 9.5, k_packet_open 7.0, k_packet_scatter 0.4 now); 2M points x 50k zones:
-// 15.7 -> 5.6 ms; 300k buildings in 20k holed zones: 17.4 -> 4.0 ms.  k_packet
-// is bound by its instructions (some 1,000 per packet and build row, from a
-// loop body larger than the instruction cache) and by the latency of the
-// loads at 24 warps per SM; 64 / 80 registers measured 10 % better than
-// 80 / 96 and 128.
+// 9.1, k_packet_open 6.9, k_packet_scatter 0.4 now); 2M points x 50k zones:
+// 15.7 -> 5.6 ms; 300k buildings in 20k holed zones: 17.4 -> 3.8 ms.  k_packet
+// is bound by its instructions (some 1,000 per packet and build row): for
+// polygons from a loop body larger than the instruction cache (a quarter of a
+// warp's cycles wait for instructions, as many for loads, at 24 warps per SM;
+// half of the issue slots are used), for points 70 % of the slots are used.
+// 64 / 80 registers measured 10 % better than 80 / 96 and 128.
 #include "packet.cuh"
 
 #include <algorithm>
@@ -995,7 +996,7 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
 // transposed into each probe's mask of records; then for each probe the lanes
 // whose record has it write its next pairs, side by side.  Bound by its
 // instructions (98M pairs of 4M points: 629 us with 32 records at a time, a
-// ballot for each probe and 64-bit positions, SCATTER_US this way; Pos: 32 bits
+// ballot for each probe and 64-bit positions, 532 this way; Pos: 32 bits
 // where the output has fewer places).  A block takes 4 packets and the next
 // block the next ones, as a dense packet has many times another's records.
 template <class Pos>
@@ -1096,20 +1097,23 @@ bool packet_takes(int predicate, bool points) {
          predicate == kDisjoint;
 }
 
+float mean_density(const LbvhView& t) {
+  return t.extent_area > 0.0f ? (float)t.nprims / t.extent_area : 0.0f;
+}
+
 void packet_runs(const LbvhView& t, const float4* box, const uint32_t* order, uint32_t n,
-                 const PacketStore& a, cudaStream_t s) {
+                 float density, const PacketStore& a, cudaStream_t s) {
   SPJ_CUDA(cudaMemsetAsync(a.ctrl, 0, kPacketCtrlBytes, s));
   if (n == 0) return;
-  const float per_area = t.extent_area > 0.0f ? (float)t.nprims / t.extent_area : 0.0f;
   k_packets<<<grid_for(n, 256, kNumSMs * 8), 256, 0, s>>>(t, box, order, n, t.mean_w, t.mean_h,
-                                                          per_area, a.packets, a.ctrl);
+                                                          density, a.packets, a.ctrl);
   SPJ_CUDA(cudaGetLastError());
 }
 
 void packet_join(const LbvhView& t, const GeomsView& build, const GeomsView& probe, bool points,
                  const uint32_t* order, int predicate, uint32_t* counts, const PacketStore& a,
                  DeviceStatus* st, cudaStream_t s) {
-  packet_runs(t, probe.box, order, probe.n, a, s);
+  packet_runs(t, probe.box, order, probe.n, mean_density(t), a, s);
   if (probe.n == 0) return;
   // (a warp per packet, and a packet may hold one row)
   const int g = grid_for((int64_t)probe.n * 32, kPacketThreads, kNumSMs * 8);

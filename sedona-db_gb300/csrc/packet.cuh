@@ -93,9 +93,11 @@ void packet_join(const LbvhView& t, const GeomsView& build, const GeomsView& pro
                  DeviceStatus* st, cudaStream_t s);
 
 // Cuts the n probe rows' Morton order into packets (a.packets, a.ctrl[3]) and
-// clears a's counts.
+// clears a's counts.  density: build rows per area, by which it judges how many
+// a packet may meet (mean_density: over the whole extent).
 void packet_runs(const LbvhView& t, const float4* box, const uint32_t* order, uint32_t n,
-                 const PacketStore& a, cudaStream_t s);
+                 float density, const PacketStore& a, cudaStream_t s);
+float mean_density(const LbvhView& t);
 
 // The pairs of the n probe rows, grouped by probe row in ascending order (offs:
 // exclusive scan of counts), writes bounded by cap.

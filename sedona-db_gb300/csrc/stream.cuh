@@ -8,14 +8,16 @@
 // runs:
 //   1. a persistent decode kernel pulling chunks from a work queue (one atomic
 //      per chunk) and decoding every row's point into one stream-wide column;
-//   2. from 65,536 rows, the rows' Morton order (keys + radix sort), then the
-//      LBVH count pass, a scan, and the scatter pass over that column in that
-//      order (candidate pairs, bounded by the candidate capacity), and the
-//      candidates' permutation into the same order;
+//   2. from 65,536 rows, the rows' Morton order (keys + radix sort); then,
+//      where the packet kernels take the rows (packet_pays), these and the
+//      scatter of their records into pairs, and 4;
+//      else the LBVH count pass, a scan, and the scatter pass over that column
+//      in that order (candidate pairs, bounded by the candidate capacity), and
+//      the candidates' permutation into the same order;
 //   3. the refine kernel over the candidates in that order (the pair count is
 //      read on the device), a scan of its flags, and the compaction (bounded
 //      by the output capacity);
-//   4. the copy-out of the two totals.
+//   4. the copy-out of the totals.
 // The host checks the totals after the replay; when a capacity was too small
 // it grows the buffers, re-captures and replays (the buffers then stay large
 // enough for later replays of the same stream).  Pairs come out grouped by

@@ -367,9 +367,11 @@ def test_packet_from_the_first_row_counts(capi, pred, n):
     (2000, 20.0, 70000, "intersects", 0.0, 1),   # many probes in each build row's box
     (2000, 20.0, 65535, "intersects", 0.0, 0),
     (20000, 0.02, 70000, "contains", 0.0, 0),    # build rows that hardly any probe meets
-    (130000, 0.0, 2400, "dwithin", 0.01, 0),     # few probes, far apart
-    (130000, 0.0, 2400, "dwithin", 1.0, 1),      # many neighbours each
-    (130000, 0.0, 11000, "dwithin", 0.01, 1)])
+    (300000, 0.0, 5000, "dwithin", 0.01, 0),     # few probes, far apart
+    (300000, 0.0, 5000, "dwithin", 1.0, 1),      # many neighbours each
+    (300000, 0.0, 4000, "dwithin", 0.01, 1),
+    (300000, 0.0, 26000, "dwithin", 0.01, 1),
+    (5000, 0.0, 20000, "dwithin", 0.01, 0)])
 def test_packets_by_density(capi, build_rows, radius, n, pred, distance, packets):
     """The path that the sizes choose, with the pairs of the other one."""
     from sedona_gpuspatial import wkb

@@ -69,7 +69,8 @@ CALLS = [
     ("kTouches", 0, 8192, 5000, STARS, 0, 0, 1), ("kTouches", 0, 250000, 50000, TINY, 0, 0, 0),
     ("kWithin", 0, 8192, 50000, ZONES, 0, 0, 1), ("kEquals", 0, 32000, 1000, ZONES, 0, 0, 0),
     ("kCoveredBy", 0, 65000, 50000, TINY, 0, 0, 0),
-    ("kPredDWithin", 1, 4000, 400000, 0, 0, 0.8, 0), ("kPredDWithin", 1, 4000, 400000, 0, 0, 6.9, 1),
+    ("kPredDWithin", 1, 16000, 400000, 0, 0, 0.8, 0), ("kPredDWithin", 1, 16000, 400000, 0, 0, 3.0, 1),
+    ("kPredDWithin", 1, 4000, 400000, 0, 0, 0.8, 1), ("kPredDWithin", 1, 20000, 5000, 0, 0, 0.1, 0),
     ("kPredDWithin", 1, 64000, 400000, 0, 0, 0.03, 1), ("kPredDWithin", 1, 2047, 5000, 0, 0, 50, 0),
     ("kPredDWithin", 1, 2048, 20000, 0, 0, 0.03, 1),
 ]
