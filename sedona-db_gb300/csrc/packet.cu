@@ -370,7 +370,7 @@ __device__ __forceinline__ bool isolated_result(int predicate, bool in) {
 // others are done, so it is cut in halves, down to one row: an aligned group of
 // rows is split where its box, widened by the mean build box, is over
 // kPacketGrowth times one row's and may meet over kPacketRows build rows (by
-// their mean density over the tree; with fewer, splitting costs more than it
+// the density that the caller gives; with fewer, splitting costs more than it
 // saves).  (8,000 buildings, whose neighbours lie far apart: 1,667 us with
 // packets of 4 rows and up, 1,242 with single rows; 2M alike.)
 constexpr float kPacketRows = 64.0f, kPacketGrowth = 4.0f;
