@@ -299,8 +299,8 @@ __device__ __forceinline__ float list_at(const float (&ld)[K + 1], uint32_t i) {
   return v;
 }
 
-// A probe's place in the queue of the exact kernel: its row, and an upper
-// bound of its k-th distance.
+// A probe's place in the queue of another kernel: its row and, for the exact one
+// (else null), an upper bound of its k-th distance.
 struct KnnQueue {
   uint32_t* rows;
   float* bound;
@@ -308,7 +308,7 @@ struct KnnQueue {
   __device__ __forceinline__ void push(uint64_t qi, float b) const {
     const uint32_t at = atomicAdd(count, 1u);
     rows[at] = (uint32_t)qi;
-    bound[at] = b;
+    if (bound) bound[at] = b;
   }
 };
 
@@ -1115,14 +1115,12 @@ void KnnIndex::query(const double* probe_xy, uint64_t n, uint32_t k, uint32_t* o
     if (form_ == 1 && k <= 16 && split_ok_) {
       // queues: near ties, probes past the split range, probes of warps whose
       // 32 searches lie apart
-      redo_.reserve((n + 1) * 24, s);
-      uint32_t* rows = redo_.as<uint32_t>();
-      auto queue_at = [&](int i) {
-        return KnnQueue{rows + 2 * i * (n + 1), reinterpret_cast<float*>(rows + (2 * i + 1) * (n + 1)),
-                        nredo + i};
-      };
-      const KnnQueue queue = queue_at(0), big = queue_at(1), wide = queue_at(2);
       const bool packet = order != nullptr && n >= bvh_.nprims;
+      redo_.reserve((n + 1) * (packet ? 16 : 12), s);
+      uint32_t* rows = redo_.as<uint32_t>();
+      const KnnQueue queue{rows, reinterpret_cast<float*>(rows + (n + 1)), nredo};
+      const KnnQueue big{rows + 2 * (n + 1), nullptr, nredo + 1};
+      const KnnQueue wide{packet ? rows + 3 * (n + 1) : nullptr, nullptr, nredo + 2};
       const int gr = grid_for((int64_t)n, kKnnThreads, kNumSMs * 4);
 #define SPJ_KNN_SPLIT(KK)                                                                        \
   if (packet)                                                                                    \
