@@ -701,12 +701,16 @@ __global__ void __launch_bounds__(256)
 
 // Proves a page's segments in order: the first starts with the first value,
 // every other one with the value behind the one before it.  Where the guess
-// was another value the segment is walked again from there.  Leaves each
+// was another value the segment is walked from there, as far as the guess if that
+// lies on the way (page decode of 200k polygons among as many empty values: 1,520
+// us walked to the end, 1,055 with one walk per page, 290 this way; of 400k values
+// that are no WKB 5,670, 3,050, and with the window 3,120).  Leaves each
 // segment's start and, as its count, the values before it (m: past the last).
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kWalkThreads)
     k_seg_chain(const PageInfo* __restrict__ pages, uint32_t np, const uint8_t* __restrict__ src,
                 const uint8_t* __restrict__ dst, const PageWalk* __restrict__ walks,
                 Segment* __restrict__ segs, uint32_t* status) {
+  extern __shared__ __align__(16) uint8_t smem[];
   const int lane = threadIdx.x & 31;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < np; p += nwarps) {
@@ -716,6 +720,8 @@ __global__ void __launch_bounds__(128)
     const uint8_t* vp = page_bytes(pg, src, dst) + w.vp;
     const uint32_t avail = pg.raw_size - w.vp;
     const uint32_t ns = avail / kSegBytes + 1;  // (the last one may be empty)
+    Win win;
+    win_init(win, vp, avail, smem + (threadIdx.x >> 5) * (kWalkWin + 16), kWalkWin);
     uint32_t at = 0, before = 0;
     for (uint32_t s0 = 0; s0 < ns; s0 += 32) {
       Segment mine{kSegNone, 0, kSegNone};
@@ -727,8 +733,26 @@ __global__ void __launch_bounds__(128)
                   __shfl_sync(0xffffffffu, mine.exit, k)};
         const uint32_t start = at, rank = before;
         if (before < w.m && at < q1) {
-          if (r.start != at)
-            r = seg_walk(vp, avail, at, q1, [](uint32_t, uint32_t, uint32_t) {});
+          if (r.start != at) {
+            // (up to the guess, where that is a later value: an empty value is
+            // never guessed; a longer walk goes through the warp's window)
+            uint32_t q = at, c = 0;
+            while (q < q1 && q != r.start) {
+              if (avail - q < 4) break;
+              uint32_t l;
+              if (c < 8) {
+                l = ld_u32(vp + q);
+              } else {
+                win_need(win, q, 4);
+                l = win_u32(win, q);
+              }
+              if (avail - q - 4 < l) break;
+              c++;
+              q += 4 + l;
+            }
+            if (q == r.start && q < q1) r.count += c;
+            else r = Segment{at, c, q < q1 ? kSegStuck : q};
+          }
           before = min(w.m, before + r.count);
           at = r.exit == kSegStuck ? avail : r.exit;
           if (r.exit == kSegStuck && before < w.m) {  // no more to be found
@@ -1418,7 +1442,9 @@ extern "C" int SpjParquetReadWkb(SpjParquet* p, const char* column, int32_t rg_b
         const int gp = grid_for((int64_t)np * 32, 128, kNumSMs * 16);
         const int gs = grid_for((int64_t)nseg * 32, 256, kNumSMs * 16);
         k_seg_walk<<<gs, 256, 0, s>>>(dpages, np, (uint32_t)nseg, dsrc, dpb, walks, segs);
-        k_seg_chain<<<gp, 128, 0, s>>>(dpages, np, dsrc, dpb, walks, segs, st);
+        SPJ_CUDA(cudaFuncSetAttribute(k_seg_chain, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      walk_smem));
+        k_seg_chain<<<g, kWalkThreads, walk_smem, s>>>(dpages, np, dsrc, dpb, walks, segs, st);
         k_seg_write<<<gs, 256, 0, s>>>(dpages, np, (uint32_t)nseg, dsrc, dpb, walks, segs, ra);
         k_seg_rows<<<gp, 128, 0, s>>>(dpages, np, walks, ra);
       }

@@ -194,6 +194,36 @@ def test_plain_values_of_unequal_lengths(gp, tmp_path, compression, kind):
         _assert_column(got, off, data[np.repeat(valid, np.diff(off))], valid)
 
 
+@pytest.mark.parametrize("share", [0.02, 0.5, 0.98])
+@pytest.mark.parametrize("compression", ["snappy", "none"])
+def test_empty_values_before_a_guessed_one(gp, tmp_path, compression, share):
+    """Segments that start with empty values, whose guess is the polygon behind
+    them; runs of empty values over whole segments; a damaged length behind one."""
+    from sedona_gpuspatial import capi, wkb
+    rng = np.random.default_rng(int(share * 100))
+    n = 20000
+    lens = np.where(rng.random(n) < share, 0, 13 + 16 * rng.integers(4, 14, n))
+    lens[5000:9000] = 0
+    off = np.zeros(n + 1, np.int64)
+    off[1:] = np.cumsum(lens)
+    data = rng.integers(0, 256, int(off[-1]), dtype=np.uint8)
+    at = off[:-1][lens > 0]
+    data[at] = 1
+    data[at[:, None] + np.arange(1, 5)] = (3, 0, 0, 0)
+    path = str(tmp_path / "e.parquet")
+    gp.write_wkb(path, wkb.WkbColumn(off, data, None), compression=compression, page_bytes=1 << 16)
+    with gp.GeoParquetFile(path) as f:
+        _assert_column(gp.device_to_host(f.read_wkb()), off, data, np.ones(n, bool))
+    if compression == "none":
+        raw = bytearray(open(path, "rb").read())
+        k = raw.rfind(data[at[-1]:].tobytes()) - 4  # the last polygon's length word
+        assert k > 0 and int.from_bytes(raw[k:k + 4], "little") == lens[lens > 0][-1]
+        raw[k:k + 4] = (1 << 30).to_bytes(4, "little")
+        open(path, "wb").write(raw)
+        with gp.GeoParquetFile(path) as f, pytest.raises(capi.GpuSpatialError):
+            f.read_wkb()
+
+
 def test_files_share_page_locked_blocks(gp, tmp_path):
     """Threads that open, read and close files of several sizes one after the
     other: every read has its own bytes."""
