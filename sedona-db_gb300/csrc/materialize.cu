@@ -53,8 +53,9 @@ struct GatherCol {
   unsigned long long* nulls = nullptr;
 };
 constexpr uint32_t kGatherCols = 8;
+template <uint32_t kCols>
 struct GatherCols {
-  GatherCol c[kGatherCols];
+  GatherCol c[kCols];
 };
 constexpr int kGatherRows = 4;  // rows of a lane in flight
 
@@ -103,7 +104,9 @@ __device__ __forceinline__ void gather_lengths(const GatherCol& c, const uint32_
 // are coalesced and 4 gathered values are in flight.  Bound by L2 and HBM: 4M
 // rows, 5 columns with validity, 171 us in passes of their own (32 rows per
 // thread for the validity words), 63 this way.
-__global__ void __launch_bounds__(256) k_gather_columns(const __grid_constant__ GatherCols cols) {
+template <uint32_t kCols>
+__global__ void __launch_bounds__(256)
+    k_gather_columns(const __grid_constant__ GatherCols<kCols> cols) {
   const GatherCol& c = cols.c[blockIdx.y];
   const int lane = threadIdx.x & 31;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -148,20 +151,26 @@ __global__ void __launch_bounds__(256) k_gather_columns(const __grid_constant__ 
   }
 }
 
-void gather_columns(const GatherCol* c, size_t count, cudaStream_t s) {
-  for (size_t k = 0; k < count; k += kGatherCols) {
-    GatherCols a;
-    uint64_t most = 0;
-    const unsigned m = (unsigned)std::min<size_t>(kGatherCols, count - k);
-    for (unsigned q = 0; q < m; q++) {
-      a.c[q] = c[k + q];
-      most = std::max(most, c[k + q].n);
-    }
-    if (most == 0) continue;
-    const int g = grid_for((int64_t)(most + kGatherRows - 1) / kGatherRows, 256, kNumSMs * 8);
-    k_gather_columns<<<dim3((unsigned)g, m), 256, 0, s>>>(a);
-    SPJ_CUDA(cudaGetLastError());
+template <uint32_t kCols>
+void launch_gather(const GatherCol* c, unsigned m, cudaStream_t s) {
+  GatherCols<kCols> a;
+  uint64_t most = 0;
+  for (unsigned q = 0; q < m; q++) {
+    a.c[q] = c[q];
+    most = std::max(most, c[q].n);
   }
+  if (most == 0) return;
+  const int g = grid_for((int64_t)(most + kGatherRows - 1) / kGatherRows, 256, kNumSMs * 8);
+  k_gather_columns<kCols><<<dim3((unsigned)g, m), 256, 0, s>>>(a);
+  SPJ_CUDA(cudaGetLastError());
+}
+
+// (a column alone is launched without the parameters of eight, which cost a
+// short call 2 of 30 us)
+void gather_columns(const GatherCol* c, size_t count, cudaStream_t s) {
+  if (count == 1) return launch_gather<1>(c, 1, s);
+  for (size_t k = 0; k < count; k += kGatherCols)
+    launch_gather<kGatherCols>(c + k, (unsigned)std::min<size_t>(kGatherCols, count - k), s);
 }
 
 // A warp takes 32 values: lane k reads value k's index, source range and
