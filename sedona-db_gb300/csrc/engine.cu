@@ -111,7 +111,8 @@ bool packet_pays(int predicate, bool points, uint64_t rows, const PacketTree& t)
   if (points)
     return held >= 90.0 + 1.3 * covers ||
            (covers <= 2.0 && rows >= 6ull * t.nprims && (t.nprims <= 8192 || covers >= 0.1));
-  if (first) return held >= 48.0 || (covers >= 0.04 && covers <= 0.3);
+  if (first)
+    return held >= 48.0 || (covers <= 0.3 && (covers >= 0.04 || t.nprims <= 2048));
   switch (predicate) {
     case kContains:
     case kCovers:

@@ -111,7 +111,8 @@ constexpr uint32_t kOrderMinRows = 1u << 16;
 //    10k stars 1M rows 490 / 537; 50k stars 130k rows 360 / 335, 500k 558 / 587;
 //    5k clustered buildings 250k rows 277 / 301, 50k of them 610 / 354;
 //  - buildings intersecting 50k zones: 49k rows (63) 2,315 / 2,150, 66k (84)
-//    2,289 / 2,498; 50k stars, 1M rows (31) 2,180 / 1,847, 10k 130k rows 467 / 496;
+//    2,289 / 2,498; 50k stars, 1M rows (31) 2,180 / 1,847, 10k 130k rows 467 / 496,
+//    500 131k rows (with the copies of a host batch) 549 / 589;
 //  - containment (dearer pairs): 50k zones 16k rows (21) 2,063 / 1,662, 24k (31)
 //    1,895 / 2,275; with holes 8k (10) 2,301 / 2,245, 12k (15) 2,500 / 2,987;
 //    20k stars 250k rows 652 / 650, 1M 1,301 / 1,431;

@@ -61,6 +61,7 @@ CALLS = [
     ("kIntersects", 1, 250000, 5000, TINY, 0, 0, 1), ("kDisjoint", 1, 80000, 50000, ZONES, 0, 0, 0),
     ("kIntersects", 0, 65537, 50000, ZONES, 0, 0, 1), ("kIntersects", 0, 2000000, 50000, ZONES, 0, 0, 1),
     ("kIntersects", 0, 1000000, 50000, STARS, 0, 0, 0), ("kIntersects", 0, 250000, 50000, TINY, 0, 0, 0),
+    ("kIntersects", 0, 131072, 500, STARS, 0, 0, 1), ("kIntersects", 0, 131072, 10000, STARS, 0, 0, 1),
     ("kContains", 0, 8192, 50000, ZONES, 0, 0, 0), ("kContains", 0, 16000, 50000, ZONES, 0, 0, 0),
     ("kCovers", 0, 32000, 50000, ZONES, 0, 0, 1), ("kCovers", 0, 32000, 50000, STARS, 0, 0, 0),
     ("kContains", 0, 1000000, 50000, STARS, 0, 0, 1), ("kContains", 0, 300007, 20000, ZONES, 1, 0, 1),
