@@ -403,7 +403,8 @@ __global__ void __launch_bounds__(kTravThreads, 8)
         // the candidates are those of k_dwithin_fused: overlapping boxes, none
         // in a leaf that lies farther than d as a whole (a point's box is its
         // RN32 copy)
-        if (near && split && leaf_class(t.leaf_box[c], hx, hy, lx, ly, own.cerr, own.d_lo, own.d_hi) < 0)
+        if (near && split &&
+            leaf_class(t.leaf_box[c], hx, hy, lx, ly, own.cerr, own.d_lo, own.d_hi) < 0)
           near = false;
         const float inn = near ? in2 : -1.0f;
         for (uint32_t k0 = b0; k0 < b1; k0 += 32) {

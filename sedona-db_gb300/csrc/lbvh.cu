@@ -72,7 +72,8 @@ __global__ void k_bounds(const float4* __restrict__ boxes, const uint32_t* __res
     w += b.z - b.x;
     h += b.w - b.y;
     if (i < kSpreadPairs) {
-      const float4 p = boxes[ids[hashed_row(2 * i + 1, m)]], q = boxes[ids[hashed_row(2 * i + 2, m)]];
+      const float4 p = boxes[ids[hashed_row(2 * i + 1, m)]];
+      const float4 q = boxes[ids[hashed_row(2 * i + 2, m)]];
       dx += fabsf(0.5f * (p.x + p.z) - 0.5f * (q.x + q.z));
       dy += fabsf(0.5f * (p.y + p.w) - 0.5f * (q.y + q.w));
     }
